@@ -3,23 +3,25 @@
 //
 // Tensor cores cannot evaluate (min,+), so the math runs on the CUDA cores:
 //   int32 : one DPX __viaddmin_s32 (add + min fused) per (i,j,k) pair;
-//   fp32  : FADD per pair and a three-input min.f32 per two pairs.
-// Data movement is TMA: each k-tile of A (128 rows x 32 k, 128-byte swizzle)
-// and B (32 k x 128 cols) lands in shared memory through
-// cp.async.bulk.tensor with an mbarrier transaction count, three stages deep,
-// issued by one thread; 256 threads each own an 8 x 8 block of C and read
-// their A fragments as float4 along k (swizzle makes the two row groups of a
-// warp hit different banks) and B fragments as float4 along n.
+//   fp32  : two additions (or one packed addition) and a three-input min.f32
+//           per two pairs.
+// Two kernels share that arithmetic and 8 x 8 outputs per thread:
+//   k_minplus_tma : 128 x 128 tiles, each k tile of A (128 rows x 32 k, 128-byte
+//                   swizzle) and B (32 k x 128 cols) brought in by TMA
+//                   (cp.async.bulk.tensor, mbarrier transaction counts, three
+//                   stages, one issuing thread);
+//   k_minplus_cp  : 128 x 128 or 64 x 64 tiles filled by cp.async, which takes
+//                   any leading dimension and base, with k split over the blocks
+//                   of a cluster where the tiles alone would leave SMs idle.
+// pick_shape() chooses between them by size and alignment.
 //
 // Semantics follow minplus_kernel_f32 (HIP_kernel/minplus_mm/src/minplus_hip.cpp:13-118):
 // accumulators start at +inf and a NaN candidate never replaces the
 // accumulator.  The int32 twin (no reference counterpart) starts at
 // INT32_MAX/2 = 1073741823 (the "missing" sentinel), so results are clamped to
 // it; inputs must lie in [-2^30, 2^30-1] so no sum overflows.
-// Partial k-tiles are bounded by a uniform loop limit, so TMA's out-of-range
-// fill value never enters a minimum.  Operands that TMA cannot describe
-// (unaligned base or leading dimension) take a plain-load kernel with the same
-// tiling.
+// Fill values never enter a minimum: k_minplus_tma bounds the loop of a partial
+// k tile, k_minplus_cp pads it with A = +inf (missing) and B = 0.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -38,6 +40,8 @@ constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3, NT = 256;
 constexpr int A_TILE = BM * BK;   // elements
 constexpr int B_TILE = BK * BN;
 constexpr int kMissing = 1073741823;
+constexpr int kMaxSplit = 8;      // portable cluster size
+typedef unsigned long long Pair;   // two k-adjacent 32-bit operands
 
 // Set by a bounded mbarrier wait that gave up.  One word per device: every
 // product clears it in stream order before its launch (clear_mp_error), APSP
@@ -59,6 +63,16 @@ struct MP<float> {
     return r;
   }
   __device__ __forceinline__ static float step1(float acc, float a, float b) { return fminf(acc, a + b); }
+  __device__ __forceinline__ static float vmin(float x, float y) { return fminf(x, y); }
+  // acc = min(acc, a.lo + b.lo, a.hi + b.hi): both sums in one packed addition
+  __device__ __forceinline__ static float pair(float acc, Pair a, Pair b) {
+    Pair s;
+    float x, y, r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(s) : "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s));
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(acc), "f"(x), "f"(y));
+    return r;
+  }
   static constexpr bool kTwoPerMin = true;   // one 3-input min per two pairs
 };
 template <>
@@ -68,6 +82,10 @@ struct MP<int> {
     return __viaddmin_s32(a1, b1, __viaddmin_s32(a0, b0, acc));
   }
   __device__ __forceinline__ static int step1(int acc, int a, int b) { return __viaddmin_s32(a, b, acc); }
+  __device__ __forceinline__ static int vmin(int x, int y) { return min(x, y); }
+  __device__ __forceinline__ static int pair(int acc, Pair a, Pair b) {
+    return step2(acc, (int)(uint32_t)a, (int)(uint32_t)b, (int)(a >> 32), (int)(b >> 32));
+  }
   static constexpr bool kTwoPerMin = false;  // one fused add+min per pair
 };
 
@@ -248,41 +266,262 @@ __global__ void __launch_bounds__(NT, 2)
   store_tile<T>(C, M, N, ldc, m0, n0, tx, ty, acc, Aold, lda, changed);
 }
 
-// Plain-load twin for operands TMA cannot address (same tiling, same math).
+// ---- cp.async kernel --------------------------------------------------------
+// Bound by instruction issue and register reads, like k_minplus_tma; what it is
+// for is everything that keeps that kernel from its rate: operands TMA cannot
+// describe (each B word is copied by itself, A 16 bytes at a time where its rows
+// allow it), and products with too few 128 x 128 tiles for the GPU.  B's tile is
+// stored with each pair of k rows interleaved, [k/2][n][2] (free, since every
+// word is placed by its own copy), so that both operands come as k-adjacent
+// register pairs and two additions are one add.f32x2.  A cluster of up to 8
+// blocks splits k and takes the minimum of its partial tiles through
+// distributed shared memory (minima are exact in any order).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(NT, 2)
-    k_minplus_plain(const T* __restrict__ A, const T* __restrict__ B, T* C, int M, int N, int K, int lda, int ldb,
-                    int ldc, const T* Aold, uint32_t* changed) {
-  __shared__ __align__(16) T As[A_TILE];
-  __shared__ __align__(16) T Bs[B_TILE];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int tm, tn;
-  tile_coords((M + BM - 1) / BM, (N + BN - 1) / BN, tm, tn);
-  const int m0 = tm * BM, n0 = tn * BN;
+struct Operands {
+  const T* A;
+  const T* B;
+  T* C;
+  int M, N, K, lda, ldb, ldc;
+  const T* Aold;             // APSP: the result is compared with it ...
+  uint32_t* changed;         // ... and any difference sets this word
+  int a_vec;                 // A rows start on 16 bytes
+  int c_vec;                 // 4: C rows start on 16 bytes, 2: on 8, 1: neither
+};
+
+template <int NTX, int NTY, int BK_>
+struct Tile {
+  static constexpr int NT = NTX * NTY, BM = 8 * NTY, BN = 8 * NTX, BK = BK_;
+  static constexpr int kA = BM * BK, kB = BK * BN;   // elements per stage
+  static constexpr size_t kSmem = (size_t)STAGES * (kA + kB) * 4;
+  static_assert(kSmem >= (size_t)BM * BN * 4, "a partial tile reuses the pipeline's memory");
+  // Thread column tx owns columns 4 tx .. 4 tx + 3 of each half of the tile
+  // (16-byte stores).  B's columns are permuted in shared memory so that its q-th
+  // pair of columns sits at 2 NTX q + 2 tx: the 16-byte reads of 8 neighbouring
+  // threads are contiguous.
+  __device__ __forceinline__ static int column(int tx, int q) { return 4 * NTX * (q >> 1) + 4 * tx + 2 * (q & 1); }
+  __device__ __forceinline__ static int b_position(int n) {
+    const int r = n % (4 * NTX);
+    return 2 * NTX * (2 * (n / (4 * NTX)) + ((r >> 1) & 1)) + 2 * (r >> 2) + (r & 1);
+  }
+  // 16-byte chunk of A row r that holds k .. k+3 (chunk c = k / 4): rows read
+  // by one warp at the same k fall into different banks
+  __device__ __forceinline__ static int a_index(int r, int c) {
+    const int f = BK == 32 ? (r & 7) : ((r >> 1) & 3);
+    return r * BK + ((c ^ f) << 2);
+  }
+};
+
+// Start the copies of k tile `kt` into one stage.
+template <typename T, class TL>
+__device__ __forceinline__ void load_stage(const Operands<T>& P, T* As, T* Bs, int m0, int n0, int kt) {
+  const int tid = threadIdx.x;
+  const int k0 = kt * TL::BK;
+  if (P.a_vec) {
+    constexpr int CH = TL::BK / 4, RP = TL::NT / CH;
+    const int c = tid % CH, r0 = tid / CH;
+    const int k = k0 + 4 * c;
+    const T* src = P.A + (size_t)(m0 + r0) * P.lda + k;
+    if (k + 4 <= P.K) {
+#pragma unroll
+      for (int p = 0; p < TL::BM / RP; ++p, src += (size_t)RP * P.lda)
+        if (m0 + r0 + p * RP < P.M) cp_async16(smem_u32(As + TL::a_index(r0 + p * RP, c)), src);
+    } else {   // the chunk crosses K: pad it
+      for (int p = 0; p < TL::BM / RP; ++p, src += (size_t)RP * P.lda)
+        for (int q = 0; q < 4; ++q)
+          As[TL::a_index(r0 + p * RP, c) + q] =
+              (k + q < P.K && m0 + r0 + p * RP < P.M) ? src[q] : MP<T>::init();
+    }
+  } else {
+    constexpr int RP = TL::NT / TL::BK;
+    const int k = tid % TL::BK, r0 = tid / TL::BK;
+    const T* src = P.A + (size_t)(m0 + r0) * P.lda + k0 + k;
+    if (k0 + k < P.K) {
+#pragma unroll
+      for (int p = 0; p < TL::BM / RP; ++p, src += (size_t)RP * P.lda)
+        if (m0 + r0 + p * RP < P.M) cp_async4(smem_u32(As + TL::a_index(r0 + p * RP, k >> 2) + (k & 3)), src);
+    } else {
+      for (int p = 0; p < TL::BM / RP; ++p) As[TL::a_index(r0 + p * RP, k >> 2) + (k & 3)] = MP<T>::init();
+    }
+  }
+  {
+    constexpr int KP = TL::NT / TL::BN;   // k rows per pass
+    const int n = tid % TL::BN, kk = tid / TL::BN;
+    const T* src = P.B + (size_t)(k0 + kk) * P.ldb + n0 + n;
+    const int pos = TL::b_position(n);
+    if (k0 + TL::BK <= P.K) {
+      if (n0 + n < P.N) {
+#pragma unroll
+        for (int p = 0; p < TL::BK / KP; ++p, src += (size_t)KP * P.ldb) {
+          const int k = kk + p * KP;
+          cp_async4(smem_u32(Bs + ((k >> 1) * TL::BN + pos) * 2 + (k & 1)), src);
+        }
+      }
+    } else {
+      for (int p = 0; p < TL::BK / KP; ++p, src += (size_t)KP * P.ldb) {
+        const int k = kk + p * KP;
+        T* dst = Bs + ((k >> 1) * TL::BN + pos) * 2 + (k & 1);
+        if (k0 + k < P.K && n0 + n < P.N) cp_async4(smem_u32(dst), src);
+        else *dst = T(0);
+      }
+    }
+  }
+}
+
+// Two k steps: A as one pair per row (8-byte loads, a warp reads four rows), B
+// as 16-byte vectors (two columns' pairs).  Loading A 16 bytes at a time would
+// halve its loads but needs 16 more registers than two blocks per SM leave.
+template <typename T, class TL>
+__device__ __forceinline__ void two_k(const T* As, const T* Bs, int k2, int tx, int ty, T (&acc)[8][8]) {
+  constexpr int NTY = TL::BM / 8, NTX = TL::BN / 8;
+  Pair a[8], b[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    a[i] = *reinterpret_cast<const Pair*>(As + TL::a_index(ty + NTY * i, k2 >> 1) + 2 * (k2 & 1));
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const ulonglong2 v =
+        *reinterpret_cast<const ulonglong2*>(Bs + ((size_t)k2 * TL::BN + 2 * tx + 2 * NTX * q) * 2);
+    b[2 * q] = v.x;
+    b[2 * q + 1] = v.y;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = MP<T>::pair(acc[i][j], a[i], b[j]);
+}
+
+template <typename T, class TL>
+__global__ void __launch_bounds__(TL::NT, TL::NT == 256 ? 2 : 8)
+    k_minplus_cp(const Operands<T> P, int splits) {
+  extern __shared__ __align__(16) unsigned char cp_smem[];
+  T* As = reinterpret_cast<T*>(cp_smem);
+  T* Bs = As + STAGES * TL::kA;
+  constexpr int NTX = TL::BN / 8, NTY = TL::BM / 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = (lane & 7) + 8 * (warp % (NTX / 8)), ty = (lane >> 3) + 4 * (warp / (NTX / 8));
+  // tile order: groups of 8 tile rows share B panels in L2
+  const int tiles_m = (P.M + TL::BM - 1) / TL::BM, tiles_n = (P.N + TL::BN - 1) / TL::BN;
+  const int tile = blockIdx.x / splits, part = blockIdx.x - tile * splits;   // the cluster's blocks are the k parts
+  const int g = tile / (8 * tiles_n), first_m = g * 8;
+  const int gsz = min(tiles_m - first_m, 8), in = tile - g * 8 * tiles_n;
+  const int m0 = (first_m + in % gsz) * TL::BM, n0 = (in / gsz) * TL::BN;
+  const int KT = (P.K + TL::BK - 1) / TL::BK;
+  const int kt0 = (int)((int64_t)KT * part / splits), kt1 = (int)((int64_t)KT * (part + 1) / splits);
+
   T acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = MP<T>::init();
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int idx = tid; idx < A_TILE; idx += NT) {
-      const int r = idx / BK, k = idx % BK;
-      const int gr = m0 + r, gk = k0 + k;
-      const T v = (gr < M && gk < K) ? A[(size_t)gr * lda + gk] : MP<T>::init();
-      As[r * BK + (((k >> 2) ^ (r & 7)) << 2) + (k & 3)] = v;   // same swizzle as TMA
-    }
-    for (int idx = tid; idx < B_TILE; idx += NT) {
-      const int k = idx / BN, c = idx % BN;
-      const int gk = k0 + k, gc = n0 + c;
-      Bs[idx] = (gk < K && gc < N) ? B[(size_t)gk * ldb + gc] : MP<T>::init();
-    }
-    __syncthreads();
-    const int kvalid = min(BK, K - k0);
-    if (kvalid == BK) mma_tile<T, true>(As, Bs, BK, tx, ty, acc);
-    else mma_tile<T, false>(As, Bs, kvalid, tx, ty, acc);
-    __syncthreads();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (kt0 + s < kt1) load_stage<T, TL>(P, As + s * TL::kA, Bs + s * TL::kB, m0, n0, kt0 + s);
+    cp_async_commit();
   }
-  store_tile<T>(C, M, N, ldc, m0, n0, tx, ty, acc, Aold, lda, changed);
+  int s = 0;
+  for (int kt = kt0; kt < kt1; ++kt) {
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();   // stage s has landed for everyone; everyone is done with the stage refilled next
+    {
+      const int nx = s == 0 ? STAGES - 1 : s - 1;
+      if (kt + STAGES - 1 < kt1) load_stage<T, TL>(P, As + nx * TL::kA, Bs + nx * TL::kB, m0, n0, kt + STAGES - 1);
+      cp_async_commit();
+    }
+    const T* as = As + s * TL::kA;
+    const T* bs = Bs + s * TL::kB;
+    if (kt * TL::BK + TL::BK <= P.K) {
+#pragma unroll
+      for (int k2 = 0; k2 < TL::BK / 2; ++k2) two_k<T, TL>(as, bs, k2, tx, ty, acc);
+    } else {
+      const int n2 = (P.K - kt * TL::BK + 1) / 2;
+      for (int k2 = 0; k2 < n2; ++k2) two_k<T, TL>(as, bs, k2, tx, ty, acc);
+    }
+    s = s == STAGES - 1 ? 0 : s + 1;
+  }
+
+  bool diff = false;
+  if (splits == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = m0 + ty + NTY * i;
+      if (r >= P.M) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = n0 + TL::column(tx, 2 * h);
+        int* dst = reinterpret_cast<int*>(P.C) + (size_t)r * P.ldc + c;
+        int v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const int*>(&acc[i][4 * h + e]);
+        if (P.c_vec == 4 && c + 3 < P.N) {
+          *reinterpret_cast<int4*>(dst) = make_int4(v[0], v[1], v[2], v[3]);
+        } else if (P.c_vec == 2 && c + 3 < P.N) {
+          reinterpret_cast<int2*>(dst)[0] = make_int2(v[0], v[1]);
+          reinterpret_cast<int2*>(dst)[1] = make_int2(v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (c + e < P.N) dst[e] = v[e];
+        }
+        if (P.Aold) {
+          const int* old = reinterpret_cast<const int*>(P.Aold) + (size_t)r * P.lda + c;
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (c + e < P.N) diff |= old[e] != v[e];
+        }
+      }
+    }
+  } else {
+    // partial tile -> own shared memory; then part p reduces rows
+    // [p BM / splits, (p + 1) BM / splits) over all the cluster's blocks
+    cp_async_wait<0>();
+    __syncthreads();
+    T* mine = reinterpret_cast<T*>(cp_smem);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        mine[(ty + NTY * i) * TL::BN + TL::column(tx, j >> 1) + (j & 1)] = acc[i][j];
+    cluster_sync();
+    const int rows = TL::BM / splits;
+    const uint32_t base = smem_u32(mine);
+    for (int idx = tid; idx < rows * TL::BN; idx += TL::NT) {
+      const int lr = part * rows + idx / TL::BN, lc = idx % TL::BN;
+      const int r = m0 + lr, c = n0 + lc;
+      if (r >= P.M || c >= P.N) continue;
+      const uint32_t at = base + (uint32_t)(lr * TL::BN + lc) * 4u;
+      T v = MP<T>::init();
+      for (int p = 0; p < splits; ++p) {
+        int w;
+        asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(w) : "r"(cluster_map(at, (uint32_t)p)) : "memory");
+        v = MP<T>::vmin(v, *reinterpret_cast<const T*>(&w));
+      }
+      P.C[(size_t)r * P.ldc + c] = v;
+      if (P.Aold) {
+        const T o = P.Aold[(size_t)r * P.lda + c];
+        diff |= *reinterpret_cast<const int*>(&o) != *reinterpret_cast<const int*>(&v);
+      }
+    }
+    cluster_sync();   // nobody leaves while a peer may still read its tile
+  }
+  if (P.Aold && __any_sync(0xffffffffu, diff) && lane == 0) *(volatile uint32_t*)P.changed = 1u;
 }
 
 // ---- host ----------------------------------------------------------------
@@ -322,10 +561,14 @@ constexpr size_t kTmaSmem = (size_t)STAGES * (A_TILE + B_TILE) * 4 + STAGES * 8 
 // attribute is a per-device setting, and the error word's device address is
 // looked up with that device current.
 constexpr int kMaxDevices = 64;
+struct Capacity {
+  int sms = 0;
+  int big[4] = {}, small[4] = {};   // blocks, then clusters of 2, 4, 8, that fit the device at once
+};
 struct DeviceState {
-  bool attr_f32 = false;
-  bool attr_i32 = false;
+  Capacity f32, i32;
   uint32_t* err = nullptr;
+  bool tma_used = false;   // a kernel that can set the error word has run on this device
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[kMaxDevices];
@@ -339,19 +582,111 @@ cudaError_t current_state(DeviceState** out) {
   return cudaSuccess;
 }
 
+using Big = Tile<16, 16, 32>;
+using Small = Tile<8, 8, 16>;
+
+template <class TL>
+cudaLaunchConfig_t cp_config(int64_t tiles, int splits, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * splits));
+  cfg.blockDim = dim3(TL::NT);
+  cfg.dynamicSmemBytes = TL::kSmem;
+  cfg.stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)splits;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  return cfg;
+}
+
+// Per-device facts of one k_minplus_cp instance: its shared-memory attribute
+// is made and the clusters that fit the device at once are counted.
+template <typename T, class TL>
+cudaError_t prepare_cp(int sms, int (&fit)[4]) {
+  cudaError_t e =
+      cudaFuncSetAttribute(k_minplus_cp<T, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TL::kSmem);
+  int per = 0;
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_minplus_cp<T, TL>, TL::NT, TL::kSmem);
+  fit[0] = per * sms;
+  for (int i = 1; i < 4 && e == cudaSuccess; ++i) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cp_config<TL>(1, 1 << i, nullptr, &attr);
+    e = cudaOccupancyMaxActiveClusters(&fit[i], k_minplus_cp<T, TL>, &cfg);
+  }
+  return e;
+}
+
 template <typename T>
-cudaError_t ensure_smem_attr() {
+cudaError_t ensure_kernels(const Capacity** cap) {
   DeviceState* d = nullptr;
   cudaError_t e = current_state(&d);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(g_dev_mu);
-  bool& done = std::is_same<T, float>::value ? d->attr_f32 : d->attr_i32;
-  if (!done) {
-    e = cudaFuncSetAttribute(k_minplus_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem);
+  Capacity& c = std::is_same<T, float>::value ? d->f32 : d->i32;
+  if (!c.sms) {
+    int dev = 0, sms = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess && std::is_same<T, int>::value)
+      e = cudaFuncSetAttribute(k_minplus_tma<int>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem);
+    if (e == cudaSuccess) e = prepare_cp<T, Big>(sms, c.big);
+    if (e == cudaSuccess) e = prepare_cp<T, Small>(sms, c.small);
     if (e != cudaSuccess) return e;
-    done = true;
+    c.sms = sms;
   }
+  *cap = &c;
   return cudaSuccess;
+}
+
+enum Kernel { kTma, kBig, kSmall };
+struct Shape {
+  Kernel kernel;
+  int splits;
+};
+
+// The kernel, tile and k split with the least estimated time.  Blocks run in
+// rounds of as many as fit the device; a round lasts as long as its fullest SM
+// needs for its pairs, at about 115 G pairs/s with 8 resident warps or more (a
+// 128 x 128 tile's block brings 8, a 64 x 64 tile's 2) and proportionally
+// longer with fewer.  Every round adds the fill of the pipeline, a split the
+// exchange of partial tiles (both in pairs at the full rate).
+// Relative cost of a pair, measured at 4736 x 4096 x 4736: int32 17.0 T pairs/s
+// by TMA, 16.4 by the 128-tile cp.async kernel; fp32 16.6 and 17.0, so that
+// fp32 has no TMA instance.  The 64-tile kernel reaches 13.7 (2048^3): it
+// reads and copies twice the operand bytes per pair.
+Shape pick_shape(int M, int N, int K, const Capacity& cap, bool tma, bool is_int) {
+  Shape best{kBig, 1};
+  double least = 1e300;
+  for (int kern = tma && is_int ? kTma : kBig; kern <= kSmall; ++kern) {
+    const int bm = kern == kSmall ? Small::BM : Big::BM, bk = kern == kSmall ? Small::BK : Big::BK;
+    const int warps = kern == kSmall ? 2 : 8;
+    const double cost = kern == kTma ? 1.0 : kern == kBig ? (is_int ? 1.037 : 1.0) : 1.25;
+    const int64_t tiles = (int64_t)((M + bm - 1) / bm) * ((N + bm - 1) / bm);
+    const int kt = (K + bk - 1) / bk;
+    const int most = kern == kTma ? 1 : kMaxSplit;
+    for (int i = 0; (1 << i) <= most && (1 << i) <= kt; ++i) {
+      const int s = 1 << i;
+      const int64_t fit = kern == kSmall ? cap.small[i] : cap.big[i];   // clusters at once
+      if (fit < 1) continue;
+      const double work = (double)bm * bm * ((kt + s - 1) / s) * bk * cost;   // of one block
+      const double fill = 200000.0 + (s > 1 ? 150000.0 + 60.0 * bm * bm : 0.0);
+      auto round = [&](int64_t clusters) {
+        const int64_t per_sm = (clusters * s + cap.sms - 1) / cap.sms;
+        return work * per_sm / std::min(1.0, per_sm * warps / 8.0) + fill;
+      };
+      double t = 0.0;
+      if (tiles / fit) t += (double)(tiles / fit) * round(fit);
+      if (tiles % fit) t += round(tiles % fit);
+      if (t < least) {
+        least = t;
+        best = Shape{(Kernel)kern, s};
+      }
+    }
+  }
+  return best;
 }
 
 // Device address of g_mp_error on the current device.
@@ -370,10 +705,32 @@ cudaError_t mp_error_ptr(uint32_t** out) {
   return cudaSuccess;
 }
 
+// Only k_minplus_tma waits on barriers and can set the error word.  Until it has
+// run on a device the word is 0, and the calls below skip their memset and copy.
+cudaError_t mark_tma_used() {
+  DeviceState* d = nullptr;
+  cudaError_t e = current_state(&d);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(g_dev_mu);
+  d->tma_used = true;
+  return cudaSuccess;
+}
+cudaError_t tma_used(bool* used) {
+  DeviceState* d = nullptr;
+  cudaError_t e = current_state(&d);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(g_dev_mu);
+  *used = d->tma_used;
+  return cudaSuccess;
+}
+
 // Stream-ordered clear of the error word (allocates nothing).
 cudaError_t clear_mp_error(cudaStream_t st) {
+  bool used = false;
+  cudaError_t e = tma_used(&used);
+  if (e != cudaSuccess || !used) return e;
   uint32_t* p = nullptr;
-  cudaError_t e = mp_error_ptr(&p);
+  e = mp_error_ptr(&p);
   if (e != cudaSuccess) return e;
   return cudaMemsetAsync(p, 0, sizeof(uint32_t), st);
 }
@@ -381,28 +738,78 @@ cudaError_t clear_mp_error(cudaStream_t st) {
 // Wait for the stream, then read the error word: B2_TIMEOUT when a wait of a
 // product issued since the last clear gave up.
 b2_status read_mp_error(cudaStream_t st) {
-  uint32_t* p = nullptr;
-  B2_CUDA_TRY(mp_error_ptr(&p));
+  bool used = false;
+  B2_CUDA_TRY(tma_used(&used));
   uint32_t err = 0;
-  B2_CUDA_TRY(cudaMemcpyAsync(&err, p, sizeof(err), cudaMemcpyDeviceToHost, st));
+  if (used) {
+    uint32_t* p = nullptr;
+    B2_CUDA_TRY(mp_error_ptr(&p));
+    B2_CUDA_TRY(cudaMemcpyAsync(&err, p, sizeof(err), cudaMemcpyDeviceToHost, st));
+  }
   B2_CUDA_TRY(cudaStreamSynchronize(st));
   return err ? B2_TIMEOUT : B2_SUCCESS;
+}
+
+template <typename T, class TL>
+cudaError_t launch_cp(const Operands<T>& P, int splits, cudaStream_t st) {
+  const int64_t tiles = (int64_t)((P.M + TL::BM - 1) / TL::BM) * ((P.N + TL::BN - 1) / TL::BN);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cp_config<TL>(tiles, splits, st, &attr);
+  return cudaLaunchKernelEx(&cfg, k_minplus_cp<T, TL>, P, splits);
+}
+
+template <typename T>
+bool tma_can_read(const T* p, int ld) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld & 3) == 0;
+}
+
+cudaError_t launch_tma(const int* A, const int* B, int* C, int M, int N, int K, int lda, int ldb, int ldc,
+                       cudaStream_t st, const int* Aold, uint32_t* changed, bool* launched) {
+  CUtensorMap ma, mb;
+  *launched = make_map<int>(&ma, A, M, K, lda, BK, BM, true) && make_map<int>(&mb, B, K, N, ldb, BN, BK, false);
+  if (!*launched) return cudaSuccess;
+  const cudaError_t e = mark_tma_used();
+  if (e != cudaSuccess) return e;
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  k_minplus_tma<int><<<tiles, NT, kTmaSmem, st>>>(ma, mb, C, M, N, K, ldc, Aold, lda, changed);
+  return cudaGetLastError();
+}
+cudaError_t launch_tma(const float*, const float*, float*, int, int, int, int, int, int, cudaStream_t, const float*,
+                       uint32_t*, bool* launched) {
+  *launched = false;   // pick_shape never asks for it
+  return cudaSuccess;
 }
 
 template <typename T>
 cudaError_t launch_minplus(const T* A, const T* B, T* C, int M, int N, int K, int lda, int ldb, int ldc,
                            cudaStream_t st, const T* Aold, uint32_t* changed) {
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  CUtensorMap ma, mb;
-  const bool tma = make_map<T>(&ma, A, M, K, lda, BK, BM, true) && make_map<T>(&mb, B, K, N, ldb, BN, BK, false);
-  if (tma) {
-    cudaError_t ea = ensure_smem_attr<T>();
-    if (ea != cudaSuccess) return ea;
-    k_minplus_tma<T><<<tiles, NT, kTmaSmem, st>>>(ma, mb, C, M, N, K, ldc, Aold, lda, changed);
-  } else {
-    k_minplus_plain<T><<<tiles, NT, 0, st>>>(A, B, C, M, N, K, lda, ldb, ldc, Aold, changed);
+  const Capacity* cap = nullptr;
+  cudaError_t e = ensure_kernels<T>(&cap);
+  if (e != cudaSuccess) return e;
+  const bool a_vec = tma_can_read(A, lda);
+  Shape sh = pick_shape(M, N, K, *cap, a_vec && tma_can_read(B, ldb), std::is_same<T, int>::value);
+  if (sh.kernel == kTma) {
+    bool launched = false;
+    e = launch_tma(A, B, C, M, N, K, lda, ldb, ldc, st, Aold, changed, &launched);
+    if (launched || e != cudaSuccess) return e;
+    sh = Shape{kBig, 1};   // no tensor map (driver entry point missing)
   }
-  return cudaGetLastError();
+  Operands<T> P;
+  P.A = A;
+  P.B = B;
+  P.C = C;
+  P.M = M;
+  P.N = N;
+  P.K = K;
+  P.lda = lda;
+  P.ldb = ldb;
+  P.ldc = ldc;
+  P.Aold = Aold;
+  P.changed = changed;
+  P.a_vec = a_vec;
+  const uintptr_t c = reinterpret_cast<uintptr_t>(C);
+  P.c_vec = (c & 15) == 0 && (ldc & 3) == 0 ? 4 : (c & 7) == 0 && (ldc & 1) == 0 ? 2 : 1;
+  return sh.kernel == kBig ? launch_cp<T, Big>(P, sh.splits, st) : launch_cp<T, Small>(P, sh.splits, st);
 }
 
 template <typename T>
@@ -454,7 +861,7 @@ b2_status apsp(T* D, int N, b2_stream s, int32_t* squarings) {
 }
 
 // ---- ALU peak calibration (roofline denominator for min-plus) -------------
-// The GEMM's own instruction mix on registers only: an 8 x 8 accumulator tile
+// The GEMMs' instruction mix on registers only: an 8 x 8 accumulator tile
 // per thread updated per k step exactly like mma_tile (int32: one
 // __viaddmin_s32 per pair; fp32: two FADD and one 3-input min per two pairs),
 // with no shared-memory or global traffic.  The A operand of row i at step k
