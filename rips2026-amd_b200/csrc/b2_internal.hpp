@@ -26,6 +26,10 @@ inline b2_status from_cuda(cudaError_t e) {
   return B2_CUDA_ERROR;
 }
 
+// Stream-ordered memory pool for scratch arrays of the current device
+// (b2_spgemm.cu); it keeps up to 4 GiB cached between calls.
+cudaError_t scratch_pool(cudaMemPool_t* out);
+
 // Number of ring buckets in the delta-stepping window (aligned windows of
 // kRing consecutive buckets; buckets past the window go to the far pile).
 constexpr int kRing = 16;

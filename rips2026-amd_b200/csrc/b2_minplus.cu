@@ -218,10 +218,13 @@ __device__ __forceinline__ void store_tile(T* C, int M, int N, int ldc, int m0, 
 
 // TMA pipeline kernel.  `Aold` (nullable): compare results against it and set
 // *changed (APSP squaring, where C <= A elementwise because diag(A) = 0).
+// `previous` (nullable): the last squaring's word; where it is 0 that squaring
+// changed nothing and there is nothing left to do.
 template <typename T>
 __global__ void __launch_bounds__(NT, 2)
     k_minplus_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, T* C, int M,
-                  int N, int K, int ldc, const T* Aold, int lda, uint32_t* changed) {
+                  int N, int K, int ldc, const T* Aold, int lda, uint32_t* changed, const uint32_t* previous) {
+  if (previous && *previous == 0u) return;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   T* As = reinterpret_cast<T*>(base);
@@ -302,6 +305,7 @@ struct Operands {
   int M, N, K, lda, ldb, ldc;
   const T* Aold;             // APSP: the result is compared with it ...
   uint32_t* changed;         // ... and any difference sets this word
+  const uint32_t* previous;  // APSP: as in k_minplus_tma
   int a_vec;                 // A rows start on 16 bytes
   int c_vec;                 // 4: C rows start on 16 bytes, 2: on 8, 1: neither
 };
@@ -412,6 +416,7 @@ template <typename T, class TL>
 __global__ void __launch_bounds__(TL::NT, TL::NT == 256 ? 2 : 8)
     k_minplus_cp(const Operands<T> P, int splits) {
   extern __shared__ __align__(16) unsigned char cp_smem[];
+  if (P.previous && *P.previous == 0u) return;   // the whole cluster
   T* As = reinterpret_cast<T*>(cp_smem);
   T* Bs = As + STAGES * TL::kA;
   constexpr int NTX = TL::BN / 8, NTY = TL::BM / 8;
@@ -764,25 +769,26 @@ bool tma_can_read(const T* p, int ld) {
 }
 
 cudaError_t launch_tma(const int* A, const int* B, int* C, int M, int N, int K, int lda, int ldb, int ldc,
-                       cudaStream_t st, const int* Aold, uint32_t* changed, bool* launched) {
+                       cudaStream_t st, const int* Aold, uint32_t* changed, const uint32_t* previous, bool* launched) {
   CUtensorMap ma, mb;
   *launched = make_map<int>(&ma, A, M, K, lda, BK, BM, true) && make_map<int>(&mb, B, K, N, ldb, BN, BK, false);
   if (!*launched) return cudaSuccess;
   const cudaError_t e = mark_tma_used();
   if (e != cudaSuccess) return e;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  k_minplus_tma<int><<<tiles, NT, kTmaSmem, st>>>(ma, mb, C, M, N, K, ldc, Aold, lda, changed);
+  k_minplus_tma<int><<<tiles, NT, kTmaSmem, st>>>(ma, mb, C, M, N, K, ldc, Aold, lda, changed, previous);
   return cudaGetLastError();
 }
 cudaError_t launch_tma(const float*, const float*, float*, int, int, int, int, int, int, cudaStream_t, const float*,
-                       uint32_t*, bool* launched) {
+                       uint32_t*, const uint32_t*, bool* launched) {
   *launched = false;   // pick_shape never asks for it
   return cudaSuccess;
 }
 
 template <typename T>
 cudaError_t launch_minplus(const T* A, const T* B, T* C, int M, int N, int K, int lda, int ldb, int ldc,
-                           cudaStream_t st, const T* Aold, uint32_t* changed) {
+                           cudaStream_t st, const T* Aold = nullptr, uint32_t* changed = nullptr,
+                           const uint32_t* previous = nullptr) {
   const Capacity* cap = nullptr;
   cudaError_t e = ensure_kernels<T>(&cap);
   if (e != cudaSuccess) return e;
@@ -790,7 +796,7 @@ cudaError_t launch_minplus(const T* A, const T* B, T* C, int M, int N, int K, in
   Shape sh = pick_shape(M, N, K, *cap, a_vec && tma_can_read(B, ldb), std::is_same<T, int>::value);
   if (sh.kernel == kTma) {
     bool launched = false;
-    e = launch_tma(A, B, C, M, N, K, lda, ldb, ldc, st, Aold, changed, &launched);
+    e = launch_tma(A, B, C, M, N, K, lda, ldb, ldc, st, Aold, changed, previous, &launched);
     if (launched || e != cudaSuccess) return e;
     sh = Shape{kBig, 1};   // no tensor map (driver entry point missing)
   }
@@ -806,6 +812,7 @@ cudaError_t launch_minplus(const T* A, const T* B, T* C, int M, int N, int K, in
   P.ldc = ldc;
   P.Aold = Aold;
   P.changed = changed;
+  P.previous = previous;
   P.a_vec = a_vec;
   const uintptr_t c = reinterpret_cast<uintptr_t>(C);
   P.c_vec = (c & 15) == 0 && (ldc & 3) == 0 ? 4 : (c & 7) == 0 && (ldc & 1) == 0 ? 2 : 1;
@@ -817,8 +824,60 @@ b2_status gemm(const T* A, const T* B, T* C, int M, int N, int K, int lda, int l
   // argument rules of minplus_gemm_f32 (minplus_hip.cpp:132-142)
   if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0 || lda < K || ldb < N || ldc < N) return B2_INVALID_ARGUMENT;
   B2_CUDA_TRY(clear_mp_error((cudaStream_t)s));
-  return from_cuda(launch_minplus<T>(A, B, C, M, N, K, lda, ldb, ldc, (cudaStream_t)s, nullptr, nullptr));
+  return from_cuda(launch_minplus<T>(A, B, C, M, N, K, lda, ldb, ldc, (cudaStream_t)s));
 }
+
+// D <- tmp where the last squaring changed something (an unchanged or skipped
+// one leaves the same matrix in both).
+__global__ void k_copy_if(const uint32_t* changed, size_t n, const uint32_t* __restrict__ src,
+                          uint32_t* __restrict__ dst) {
+  if (*changed == 0u) return;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    dst[i] = src[i];
+}
+
+constexpr int kMaxSquarings = 31;   // ceil(log2(N - 1)) for any int N
+
+// Repeated squaring between D and tmp.  Every product that may be needed is
+// queued at once; the device stops by itself: a product sets its word of `flags`
+// when it changes an entry, and a product whose predecessor's word is 0 returns
+// at once (about 2 us), so the host waits once, not after every product.
+template <typename T>
+b2_status square_until_fixed(T* D, T* tmp, uint32_t* flags, int N, cudaStream_t st, int* done) {
+  int maxsq = 0;
+  while ((1ll << maxsq) < (long long)(N - 1)) ++maxsq;   // ceil(log2(N-1)) products reach N-1 hops
+  const size_t words = (size_t)std::max(maxsq, 1);
+  B2_CUDA_TRY(clear_mp_error(st));
+  B2_CUDA_TRY(cudaMemsetAsync(flags, 0, words * sizeof(uint32_t), st));
+  T* cur = D;
+  T* nxt = tmp;
+  for (int it = 0; it < maxsq; ++it) {
+    B2_CUDA_TRY(launch_minplus<T>(cur, cur, nxt, N, N, N, N, N, N, st, cur, flags + it,
+                                  it ? flags + it - 1 : nullptr));
+    std::swap(cur, nxt);
+  }
+  if (cur != D) {
+    k_copy_if<<<1184, 256, 0, st>>>(flags + maxsq - 1, (size_t)N * N, (const uint32_t*)tmp, (uint32_t*)D);
+    B2_CUDA_TRY(cudaGetLastError());
+  }
+  uint32_t h[kMaxSquarings] = {};
+  B2_CUDA_TRY(cudaMemcpyAsync(h, flags, words * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  const b2_status r = read_mp_error(st);
+  if (r != B2_SUCCESS) return r;
+  *done = maxsq;
+  for (int it = 0; it < maxsq; ++it)
+    if (h[it] == 0) {   // D unchanged: fixpoint reached
+      *done = it + 1;
+      break;
+    }
+  return B2_SUCCESS;
+}
+
+// The second matrix and the flags come from the library's stream-ordered pool
+// up to this size (a cudaMalloc and cudaFree of it cost 1-2 ms, as much as all
+// the products of a 1000-vertex graph); past it from cudaMalloc, so that the
+// pool's cache stays small.
+constexpr size_t kApspPoolMax = (size_t)256 << 20;
 
 template <typename T>
 b2_status apsp(T* D, int N, b2_stream s, int32_t* squarings) {
@@ -826,38 +885,23 @@ b2_status apsp(T* D, int N, b2_stream s, int32_t* squarings) {
   cudaStream_t st = (cudaStream_t)s;
   if (squarings) *squarings = 0;
   if (N == 1) return B2_SUCCESS;
-  B2_CUDA_TRY(clear_mp_error(st));
-  T* tmp = nullptr;
-  uint32_t* flag = nullptr;
-  uint32_t* hflag = nullptr;
-  B2_CUDA_TRY(cudaMalloc((void**)&tmp, (size_t)N * N * sizeof(T)));
-  cudaError_t e = cudaMalloc((void**)&flag, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&hflag, sizeof(uint32_t));
+  const size_t matrix = ((size_t)N * N * sizeof(T) + 255) & ~(size_t)255;
+  const size_t bytes = matrix + 256;
+  const bool pooled = bytes <= kApspPoolMax;
+  unsigned char* buf = nullptr;
+  if (pooled) {
+    cudaMemPool_t pool;
+    B2_CUDA_TRY(scratch_pool(&pool));
+    B2_CUDA_TRY(cudaMallocFromPoolAsync((void**)&buf, bytes, pool, st));
+  } else {
+    B2_CUDA_TRY(cudaMalloc((void**)&buf, bytes));
+  }
   int done = 0;
-  int maxsq = 0;
-  while ((1ll << maxsq) < (long long)(N - 1)) ++maxsq;   // ceil(log2(N-1)) products reach N-1 hops
-  T* cur = D;
-  T* nxt = tmp;
-  for (int it = 0; it < maxsq && e == cudaSuccess; ++it) {
-    e = cudaMemsetAsync(flag, 0, sizeof(uint32_t), st);
-    if (e == cudaSuccess) e = launch_minplus<T>(cur, cur, nxt, N, N, N, N, N, N, st, cur, flag);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hflag, flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) break;
-    ++done;
-    std::swap(cur, nxt);
-    if (*hflag == 0) break;   // D unchanged: fixpoint reached
-  }
-  if (e == cudaSuccess && cur != D) {
-    e = cudaMemcpyAsync(D, cur, (size_t)N * N * sizeof(T), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
-  cudaFree(tmp);
-  cudaFree(flag);
-  if (hflag) cudaFreeHost(hflag);
+  const b2_status r = square_until_fixed<T>(D, (T*)buf, (uint32_t*)(buf + matrix), N, st, &done);
+  if (pooled) cudaFreeAsync(buf, st);
+  else cudaFree(buf);
   if (squarings) *squarings = done;
-  if (e != cudaSuccess) return from_cuda(e);
-  return read_mp_error(st);
+  return r;
 }
 
 // ---- ALU peak calibration (roofline denominator for min-plus) -------------
@@ -974,14 +1018,14 @@ extern "C" b2_status b2_minplus_calibrate(int32_t is_float, double* pairs_per_se
 //     cudaMalloc / cudaFree would synchronize the device and add jitter;
 //   * code running while a device-wide allocation freeze is in effect.
 // b2_apsp_f32_noalloc runs the same repeated squaring as b2_apsp_f32, but its
-// ping-pong matrix and change flag live in the fixed array below instead of a
+// ping-pong matrix and change flags live in the fixed array below instead of a
 // cudaMalloc'd buffer.  Limits and rules:
 //   * N * N * 4 bytes must fit in the array (N <= 2048); larger N is rejected
 //     with B2_NOT_SUPPORTED before anything runs;
 //   * the array is a module global: every GPU that loads this library holds
 //     its 16 MiB until the process exits;
 //   * every call on a device shares the one array, and it keeps the previous
-//     call's contents (the change flag is cleared before each product): calls
+//     call's contents (the change flags are cleared at the start of a call): calls
 //     that overlap on the GPU (different streams or threads) race and must be
 //     serialized by the caller;
 //   * the first call on each device looks up the array's device address
@@ -990,7 +1034,7 @@ extern "C" b2_status b2_minplus_calibrate(int32_t is_float, double* pairs_per_se
 namespace b2 {
 namespace {
 constexpr size_t kNoAllocScratchBytes = (size_t)16 << 20;   // 16 MiB: 2048 x 2048 floats
-// scratch matrix, then the change flag in the last 256 bytes
+// scratch matrix, then the squarings' change flags in the last 256 bytes
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + 256];
 
 std::mutex g_noalloc_mu;
@@ -1025,31 +1069,9 @@ extern "C" b2_status b2_apsp_f32_noalloc(float* d_D, int32_t N, b2_stream stream
   if (N == 1) return B2_SUCCESS;
   unsigned char* base = nullptr;
   B2_CUDA_TRY(noalloc_scratch(&base));
-  B2_CUDA_TRY(clear_mp_error(st));
-  float* tmp = (float*)base;
-  uint32_t* flag = (uint32_t*)(base + kNoAllocScratchBytes);
-  int maxsq = 0;
-  while ((1ll << maxsq) < (long long)(N - 1)) ++maxsq;
-  float* cur = d_D;
-  float* nxt = tmp;
   int done = 0;
-  cudaError_t e = cudaSuccess;
-  for (int it = 0; it < maxsq; ++it) {
-    uint32_t hflag = 0;
-    e = cudaMemsetAsync(flag, 0, sizeof(uint32_t), st);
-    if (e == cudaSuccess) e = launch_minplus<float>(cur, cur, nxt, N, N, N, N, N, N, st, cur, flag);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hflag, flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) break;
-    ++done;
-    std::swap(cur, nxt);
-    if (hflag == 0) break;
-  }
-  if (e == cudaSuccess && cur != d_D) {
-    e = cudaMemcpyAsync(d_D, cur, (size_t)N * N * sizeof(float), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
+  const b2_status r =
+      square_until_fixed<float>(d_D, (float*)base, (uint32_t*)(base + kNoAllocScratchBytes), N, st, &done);
   if (squarings) *squarings = done;
-  if (e != cudaSuccess) return from_cuda(e);
-  return read_mp_error(st);
+  return r;
 }

@@ -523,6 +523,8 @@ int grid_rows(int64_t rows) {
 // Library-owned stream-ordered pool for scratch arrays, one per device; it
 // keeps up to kPoolKeep bytes cached after a call returns.
 constexpr uint64_t kPoolKeep = 4ull << 30;
+}  // namespace
+
 cudaError_t scratch_pool(cudaMemPool_t* out) {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
@@ -549,6 +551,8 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
   *out = p;
   return cudaSuccess;
 }
+
+namespace {
 
 // Scratch array from the pool, released (stream-ordered) on scope exit.
 template <typename T>

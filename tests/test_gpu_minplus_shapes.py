@@ -76,3 +76,35 @@ def test_gemm_split_nan_inf(b2, orc, cuda):
     R = orc.minplus_gemm(A, B)
     assert np.isinf(C[:, 7]).all()
     assert np.array_equal(np.isnan(C), np.isnan(R)) and np.array_equal(C[~np.isnan(R)], R[~np.isnan(R)])
+
+
+# chains need every squaring (odd and even counts: the result ends in either
+# buffer); a star is done after one and a complete graph changes nothing in the
+# second, so the queued products after that must leave the matrix alone
+@pytest.mark.parametrize("dtype", [np.float32, np.int32])
+@pytest.mark.parametrize("kind,n", [("chain", 9), ("chain", 17), ("chain", 130), ("chain", 300), ("star", 40),
+                                    ("star", 150), ("random", 65), ("random", 259), ("chain", 3)])
+def test_apsp_stops_on_the_device(b2, orc, cuda, dtype, kind, n):
+    torch = cuda
+    rng = np.random.default_rng(n)
+    miss = np.inf if dtype == np.float32 else MISS
+    D = np.full((n, n), miss, dtype)
+    if kind == "chain":
+        D[np.arange(n - 1), np.arange(1, n)] = 1
+    elif kind == "star":
+        D[0, 1:] = 2
+        D[1:, 0] = 3
+    else:
+        D[:] = rng.integers(1, 100, (n, n)).astype(dtype)
+    np.fill_diagonal(D, 0)
+    ref, count, limit = D.copy(), 0, int(np.ceil(np.log2(max(n - 1, 1))))
+    while count < limit:
+        nxt = orc.minplus_gemm(ref, ref)
+        count += 1
+        same = np.array_equal(nxt, ref)
+        ref = nxt
+        if same:
+            break
+    got = torch.from_numpy(D).cuda()
+    assert b2.apsp(got) == count
+    assert np.array_equal(got.cpu().numpy(), ref)
