@@ -12,18 +12,19 @@
 // Plan (one pass over the expansion for ordinary rows):
 //   1. k_row_bound : candidates per row (sum of |B row k| over A's row);
 //                    validates A's and B's row pointers and A's columns and
-//                    lists the rows with more than kWarpRowMax candidates;
+//                    lists the rows of more than 128 and of more than 512
+//                    candidates;
 //   2. scan        : candidate offsets (CUB) = each row's slot in a scratch
 //                    array sized by the bound;
-//   3. k_rows_warp : one warp per ordinary row gathers its candidates into
-//                    shared memory as 64-bit keys (column << 32 | order-
-//                    preserving value bits), sorts them in registers with a
-//                    bitonic network (32 x P keys, P = 1..16), and writes the
-//                    first key of every column run (= the run's minimum) to
-//                    the row's scratch slot with its count;
-//   4. long rows   : expand-sort-compress over the listed rows only
-//                    (k_expand, CUB segmented sort, k_compress into the same
-//                    scratch slots);
+//   3. k_rows      : half a warp per row of up to 128 candidates, a warp per row
+//                    of up to 512: gather, sort (column, slot) keys in
+//                    registers, write each column's minimum to the row's
+//                    scratch slot;
+//   4. long rows   : k_rows_dense accumulates them in shared memory, one word
+//                    per column; for matrices of more than kDenseCols *
+//                    kDensePasses columns, expand-sort-compress over the listed
+//                    rows (k_expand, CUB segmented sort, k_compress into the
+//                    same scratch slots);
 //   5. scan of the counts (CUB) -> C.rowptr, then k_compact copies every row
 //      from its scratch slot to the exact-size outputs: memory this call
 //      allocates (the reference's one-call form), or the caller's own buffers
@@ -43,6 +44,7 @@
 
 #include "b2_common.cuh"
 #include "b2_internal.hpp"
+#include "b2_relax.cuh"
 
 namespace b2 {
 namespace {
@@ -50,9 +52,8 @@ namespace {
 constexpr int32_t kMiss32 = 1073741823;
 constexpr int32_t kDropCol = 0x7fffffff;   // sorts after every real column
 constexpr int kWarpRowMax = 512;           // candidates of a row sorted in one warp's registers
-constexpr int kRowWarps = 8;               // warps per block of k_rows_warp
-constexpr int kPairMax = 64;                // candidates of a row sorted by half a warp (k_rows_pair)
-constexpr unsigned long long kNoKey = ~0ull;
+constexpr int kSmallRowMax = 128;          // candidates of a row sorted in half a warp's registers
+constexpr int kRowWarps = 8;               // warps per block of k_rows
 
 enum SpStatus : uint32_t { kSpOk = 0, kSpBadIndex = 1, kSpBadRowptr = 2 };
 
@@ -94,332 +95,547 @@ struct VKey<int32_t> {
   __device__ __forceinline__ static int32_t dec(uint32_t k) { return (int32_t)(k ^ 0x80000000u); }
 };
 
+// Device counters read back in one copy after k_row_bound.
+struct SpCounters {
+  unsigned long long heavy, lng, mid;   // entries of the three row lists
+  uint32_t status;
+  uint32_t too_long;   // a row of 2^32 candidates or more
+};
+
+// Candidates per row, validation, and the lists of the rows that need
+// more than half a warp: `mid` (up to kWarpRowMax candidates) and the long ones, which
+// share one array of M entries: those of at least `heavy_from` candidates from
+// its front, the others from its back.  Eight lanes per row (a row of A rarely
+// has more entries; one warp per row left most lanes idle: 0.14 -> 0.07 ms for
+// 2^20 rows of 8), list appends aggregated per warp.
 __global__ void k_row_bound(int64_t M, int64_t K, int64_t annz, int64_t bnnz, const int64_t* __restrict__ arp,
                             const int32_t* __restrict__ aci, const int64_t* __restrict__ brp,
-                            unsigned long long* __restrict__ ub, uint32_t* status, int64_t* __restrict__ long_rows,
-                            unsigned long long* __restrict__ long_count) {
+                            unsigned long long* __restrict__ ub, SpCounters* cnt, int64_t* __restrict__ long_rows,
+                            int64_t* __restrict__ mid_rows, unsigned long long heavy_from,
+                            unsigned long long long_slots) {
+  const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (int64_t i = warp; i < M; i += nwarps) {
-    const int64_t a0 = arp[i], a1 = arp[i + 1];
+  for (int64_t base = warp * 4; base < M; base += nwarps * 4) {
+    const int64_t i = base + (lane >> 3);
     unsigned long long s = 0;
-    if (a0 < 0 || a1 < a0 || a1 > annz) {
-      if (lane == 0) atomicCAS(status, kSpOk, (uint32_t)kSpBadRowptr);
-    } else {
-      for (int64_t p = a0 + lane; p < a1; p += 32) {
-        const int32_t k = aci[p];
-        if (k < 0 || (int64_t)k >= K) {
-          atomicCAS(status, kSpOk, (uint32_t)kSpBadIndex);
-          continue;
-        }
-        const int64_t b0 = brp[k], b1 = brp[k + 1];
-        if (b0 < 0 || b1 < b0 || b1 > bnnz) {
-          atomicCAS(status, kSpOk, (uint32_t)kSpBadRowptr);
-          continue;
-        }
-        s += (unsigned long long)(b1 - b0);
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-      ub[i] = s;
-      if (s > (unsigned long long)kWarpRowMax) long_rows[atomicAdd(long_count, 1ull)] = i;
-    }
-  }
-}
-
-// ---- ordinary rows: one warp, registers -----------------------------------
-__device__ __forceinline__ unsigned long long shfl_xor64(unsigned long long x, int m) {
-  const uint32_t lo = __shfl_xor_sync(0xffffffffu, (uint32_t)x, m);
-  const uint32_t hi = __shfl_xor_sync(0xffffffffu, (uint32_t)(x >> 32), m);
-  return ((unsigned long long)hi << 32) | lo;
-}
-
-// Sort the row's n <= 32 P staged keys (element e = r * 32 + lane holds
-// key[r]; padding is kNoKey), then write the head of every column run.
-template <typename T, int P>
-__device__ __forceinline__ uint32_t sort_and_emit(const unsigned long long* __restrict__ sk, uint32_t n,
-                                                  int32_t* __restrict__ tcol, T* __restrict__ tval) {
-  const uint32_t lane = threadIdx.x & 31u;
-  unsigned long long key[P];
-#pragma unroll
-  for (int r = 0; r < P; ++r) {
-    const uint32_t e = (uint32_t)r * 32u + lane;
-    key[r] = e < n ? sk[e] : kNoKey;
-  }
-  // bitonic network over 32 P elements, ascending
-#pragma unroll
-  for (int k = 2; k <= 32 * P; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j >= 32) {
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-          const int rp = r ^ (j >> 5);
-          if (rp > r) {
-            const bool up = ((r * 32) & k) == 0;
-            const unsigned long long x = key[r], y = key[rp];
-            if ((x > y) == up) {
-              key[r] = y;
-              key[rp] = x;
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-          const uint32_t e = (uint32_t)r * 32u + lane;
-          const bool up = (e & (uint32_t)k) == 0;
-          const unsigned long long o = shfl_xor64(key[r], j);
-          const bool lower = (lane & (uint32_t)j) == 0;
-          const bool take_min = lower == up;
-          key[r] = take_min ? (o < key[r] ? o : key[r]) : (o > key[r] ? o : key[r]);
-        }
-      }
-    }
-  }
-  // heads of column runs, in order
-  uint32_t cnt = 0;
-  uint32_t carry = 0xFFFFFFFFu;   // column of element r * 32 - 1
-#pragma unroll
-  for (int r = 0; r < P; ++r) {
-    const uint32_t col = (uint32_t)(key[r] >> 32);
-    uint32_t pc = __shfl_up_sync(0xffffffffu, col, 1);
-    if (lane == 0) pc = carry;
-    const bool head = key[r] != kNoKey && col != pc;
-    const uint32_t b = __ballot_sync(0xffffffffu, head);
-    if (head) {
-      const uint32_t pos = cnt + __popc(b & ((1u << lane) - 1u));
-      tcol[pos] = (int32_t)col;
-      tval[pos] = VKey<T>::dec((uint32_t)key[r]);
-    }
-    cnt += __popc(b);
-    carry = __shfl_sync(0xffffffffu, col, 31);
-  }
-  return cnt;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kRowWarps * 32, 4)
-    k_rows_warp(int64_t M, int64_t N, const int64_t* __restrict__ arp, const int32_t* __restrict__ aci,
-                const T* __restrict__ av, const int64_t* __restrict__ brp, const int32_t* __restrict__ bci,
-                const T* __restrict__ bv, const unsigned long long* __restrict__ off, int32_t* __restrict__ tcol,
-                T* __restrict__ tval, int64_t* __restrict__ cnt, uint32_t* status) {
-  __shared__ unsigned long long s_keys[kRowWarps][kWarpRowMax];
-  const uint32_t lane = threadIdx.x & 31u;
-  unsigned long long* sk = s_keys[threadIdx.x >> 5];
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t i = warp; i < M; i += nwarps) {
-    const unsigned long long o0 = off[i], ub = off[i + 1] - o0;
-    if (ub > (unsigned long long)kWarpRowMax) continue;   // long row: expand-sort-compress
-    if (ub <= (unsigned long long)kPairMax) continue;      // small row: k_rows_pair
-    // gather: up to 32 A entries at a time; lane t holds entry t's B range
-    uint32_t n = 0;
-    const int64_t a0 = arp[i], a1 = arp[i + 1];
-    for (int64_t pa = a0; pa < a1; pa += 32) {
-      const int64_t p = pa + lane;
-      T a = T(0);
-      int64_t b0 = 0;
-      uint32_t len = 0;
-      if (p < a1) {
-        const int32_t k = aci[p];
-        a = av[p];
-        if (SpVal<T>::present(a)) {
-          b0 = brp[k];
-          len = (uint32_t)(brp[k + 1] - b0);
-        }
-      }
-      const uint32_t incl = warp_incl_scan(len);
-      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-      const uint32_t excl = incl - len;
-      for (uint32_t s0 = 0; s0 < total; s0 += 32) {
-        const uint32_t sl = s0 + lane;
-        // owner: the last lane whose range starts at or before slot sl
-        uint32_t t = 0;
-#pragma unroll
-        for (uint32_t step = 16; step >= 1; step >>= 1) {
-          const uint32_t e = __shfl_sync(0xffffffffu, excl, t + step);
-          if (e <= sl) t += step;
-        }
-        const uint32_t ex_t = __shfl_sync(0xffffffffu, excl, t);
-        const long long b0_t = __shfl_sync(0xffffffffu, (long long)b0, t);
-        const T a_t = __shfl_sync(0xffffffffu, a, t);
-        if (sl < total) {
-          const int64_t q = b0_t + (int64_t)(sl - ex_t);
-          const int32_t j = bci[q];
-          T c = T(0);
-          bool ok = SpVal<T>::combine(a_t, bv[q], c);
-          if (j < 0 || (int64_t)j >= N) {
-            atomicCAS(status, kSpOk, (uint32_t)kSpBadIndex);
-            ok = false;
-          }
-          sk[n + sl] = ok ? (((unsigned long long)(uint32_t)j << 32) | VKey<T>::enc(c)) : kNoKey;
-        }
-      }
-      n += total;
-    }
-    __syncwarp();
-    uint32_t kept;
-    if (n <= 32) kept = sort_and_emit<T, 1>(sk, n, tcol + o0, tval + o0);
-    else if (n <= 64) kept = sort_and_emit<T, 2>(sk, n, tcol + o0, tval + o0);
-    else if (n <= 128) kept = sort_and_emit<T, 4>(sk, n, tcol + o0, tval + o0);
-    else if (n <= 256) kept = sort_and_emit<T, 8>(sk, n, tcol + o0, tval + o0);
-    else kept = sort_and_emit<T, 16>(sk, n, tcol + o0, tval + o0);
-    if (lane == 0) cnt[i] = kept;
-    __syncwarp();
-  }
-}
-
-// ---- long rows: expand-sort-compress over a row list -----------------------
-// ---- small rows: two rows per warp, one per half-warp ----------------------
-// Rows with at most kPairMax candidates (every row of a sparse random graph)
-// take half a warp each, so a warp keeps two rows' dependent gathers in
-// flight.  Same steps as k_rows_warp inside 16 lanes: gather the row's
-// candidates as keys into shared memory, bitonic-sort 16 x 4 keys in
-// registers (shuffles never cross the half), emit the head of every column
-// run.  Loop trip counts are the larger half's, so every shuffle runs on the
-// full warp.
-
-template <typename T>
-__global__ void __launch_bounds__(kRowWarps * 32)
-    k_rows_pair(int64_t M, int64_t N, const int64_t* __restrict__ arp, const int32_t* __restrict__ aci,
-                const T* __restrict__ av, const int64_t* __restrict__ brp, const int32_t* __restrict__ bci,
-                const T* __restrict__ bv, const unsigned long long* __restrict__ off, int32_t* __restrict__ tcol,
-                T* __restrict__ tval, int64_t* __restrict__ cnt, uint32_t* status) {
-  __shared__ unsigned long long s_keys[kRowWarps][2][kPairMax];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t half = lane >> 4, hl = lane & 15u;
-  unsigned long long* sk = s_keys[threadIdx.x >> 5][half];
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t i0 = warp * 2; i0 < M; i0 += nwarps * 2) {
-    const int64_t i = i0 + half;
-    unsigned long long o0 = 0, ub = 0;
     if (i < M) {
-      o0 = off[i];
-      ub = off[i + 1] - o0;
-    }
-    const bool mine = i < M && ub <= (unsigned long long)kPairMax;   // other rows: k_rows_warp
-    int64_t a0 = 0, a1 = 0;
-    if (mine && ub > 0) {
-      a0 = arp[i];
-      a1 = arp[i + 1];
-    }
-    // gather, 16 A entries per pass
-    const int64_t alen = a1 - a0;
-    const int64_t alen_max = max(alen, (int64_t)__shfl_xor_sync(0xffffffffu, (long long)alen, 16));
-    uint32_t n = 0;
-    for (int64_t pa = 0; pa < alen_max; pa += 16) {
-      const int64_t p = a0 + pa + hl;
-      T a = T(0);
-      int64_t b0 = 0;
-      uint32_t len = 0;
-      if (pa + hl < alen) {
-        const int32_t k = aci[p];
-        a = av[p];
-        if (SpVal<T>::present(a)) {
-          b0 = brp[k];
-          len = (uint32_t)(brp[k + 1] - b0);
-        }
-      }
-      uint32_t incl = len;
-#pragma unroll
-      for (int o = 1; o < 16; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o, 16);
-        if (hl >= (uint32_t)o) incl += y;
-      }
-      const uint32_t total = __shfl_sync(0xffffffffu, incl, 15, 16);
-      const uint32_t excl = incl - len;
-      const uint32_t total_max = max(total, __shfl_xor_sync(0xffffffffu, total, 16));
-      for (uint32_t s0 = 0; s0 < total_max; s0 += 16) {
-        const uint32_t sl = s0 + hl;
-        uint32_t t = 0;   // owner: the last lane of the half whose range starts at or before slot sl
-#pragma unroll
-        for (uint32_t step = 8; step >= 1; step >>= 1) {
-          const uint32_t e = __shfl_sync(0xffffffffu, excl, t + step, 16);
-          if (e <= sl) t += step;
-        }
-        const uint32_t ex_t = __shfl_sync(0xffffffffu, excl, t, 16);
-        const long long b0_t = __shfl_sync(0xffffffffu, (long long)b0, t, 16);
-        const T a_t = __shfl_sync(0xffffffffu, a, t, 16);
-        if (sl < total) {
-          const int64_t q = b0_t + (int64_t)(sl - ex_t);
-          const int32_t j = bci[q];
-          T c = T(0);
-          bool ok = SpVal<T>::combine(a_t, bv[q], c);
-          if (j < 0 || (int64_t)j >= N) {
-            atomicCAS(status, kSpOk, (uint32_t)kSpBadIndex);
-            ok = false;
+      const int64_t a0 = arp[i], a1 = arp[i + 1];
+      if (a0 < 0 || a1 < a0 || a1 > annz) {
+        if (sub == 0) atomicCAS(&cnt->status, kSpOk, (uint32_t)kSpBadRowptr);
+      } else {
+        for (int64_t p = a0 + sub; p < a1; p += 8) {
+          const int32_t k = aci[p];
+          if (k < 0 || (int64_t)k >= K) {
+            atomicCAS(&cnt->status, kSpOk, (uint32_t)kSpBadIndex);
+            continue;
           }
-          sk[n + sl] = ok ? (((unsigned long long)(uint32_t)j << 32) | VKey<T>::enc(c)) : kNoKey;
+          const int64_t b0 = brp[k], b1 = brp[k + 1];
+          if (b0 < 0 || b1 < b0 || b1 > bnnz) {
+            atomicCAS(&cnt->status, kSpOk, (uint32_t)kSpBadRowptr);
+            continue;
+          }
+          s += (unsigned long long)(b1 - b0);
         }
+      }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const bool lead = sub == 0 && i < M;
+    const bool is_long = lead && s > (unsigned long long)kWarpRowMax;
+    const bool is_heavy = is_long && s >= heavy_from;
+    const bool is_mid = lead && !is_long && s > (unsigned long long)kSmallRowMax;
+    if (is_long && s > 0xFFFFFFFFull) cnt->too_long = 1u;
+    if (lead) ub[i] = is_long && long_slots && s > long_slots ? long_slots : s;
+    const uint32_t below = (1u << lane) - 1u;
+    const uint32_t bh = __ballot_sync(0xffffffffu, is_heavy);
+    const uint32_t bl = __ballot_sync(0xffffffffu, is_long && !is_heavy);
+    const uint32_t bm = __ballot_sync(0xffffffffu, is_mid);
+    if (bh | bl | bm) {
+      unsigned long long ph = 0, pl = 0, pm = 0;
+      if (lane == 0) {
+        if (bh) ph = atomicAdd(&cnt->heavy, (unsigned long long)__popc(bh));
+        if (bl) pl = atomicAdd(&cnt->lng, (unsigned long long)__popc(bl));
+        if (bm) pm = atomicAdd(&cnt->mid, (unsigned long long)__popc(bm));
+      }
+      ph = __shfl_sync(0xffffffffu, ph, 0);
+      pl = __shfl_sync(0xffffffffu, pl, 0);
+      pm = __shfl_sync(0xffffffffu, pm, 0);
+      if (is_heavy) long_rows[ph + __popc(bh & below)] = i;
+      else if (is_long) long_rows[M - 1 - (int64_t)(pl + __popc(bl & below))] = i;
+      else if (is_mid) mid_rows[pm + __popc(bm & below)] = i;
+    }
+  }
+}
+
+template <typename T>
+struct RowArgs {
+  int64_t M, N;
+  const int64_t* __restrict__ arp;
+  const int32_t* __restrict__ aci;
+  const T* __restrict__ av;
+  const int64_t* __restrict__ brp;
+  const int32_t* __restrict__ bci;
+  const T* __restrict__ bv;
+  const unsigned long long* __restrict__ off;
+  int32_t* __restrict__ tcol;
+  T* __restrict__ tval;
+  int64_t* __restrict__ cnt;
+  uint32_t* status;
+};
+
+// ---- ordinary rows: a warp or half a warp, registers ------------------------
+// A row of up to 128 candidates takes half a warp (two rows' gathers in flight
+// per warp), one of up to 512 a whole warp.  The lanes of a row gather its
+// candidates, sort them by column in registers and write each column's minimum.
+//
+// What is sorted is (column, slot), not (column, value): with the column in the
+// upper bits of a 32-bit word and the candidate's slot in the lower ones a
+// compare-exchange is one shuffle and one minimum or maximum, where 64-bit
+// (column, value) keys took two shuffles, a two-word comparison and two
+// selects.  Values wait in shared memory under their slot.  Matrices whose
+// columns do not fit beside the slot (2^25 columns for half a warp, 2^23 for a
+// whole one) use the same code with 64-bit words.
+//
+// Every comparison of the network is ascending, so padding never moves and a row
+// takes as many registers a lane as it needs, not a power of two: 70 candidates
+// on 16 lanes sort 5 registers.  Candidates land in registers directly, all
+// their loads in flight at once, when the row of A has at most one entry per
+// lane; longer ones go through shared memory.
+//
+// Bound by instruction issue (0.75 per cycle and scheduler).  A (x) A, 2^20 rows
+// of 8 (67 M candidates), int32: row kernels 2.41 ms with 64-bit (column, value)
+// keys -> 0.77 ms; the call 2.90 -> 1.19 ms.
+template <typename K>
+struct RowKey;
+template <>
+struct RowKey<uint32_t> {
+  __device__ __forceinline__ static uint32_t shfl_xor(uint32_t x, int m) { return __shfl_xor_sync(0xffffffffu, x, m); }
+};
+template <>
+struct RowKey<unsigned long long> {
+  __device__ __forceinline__ static unsigned long long shfl_xor(unsigned long long x, int m) {
+    return __shfl_xor_sync(0xffffffffu, x, m);
+  }
+};
+
+// Batcher's odd-even merge sort of key[0 .. PR) in one lane's registers.  Every
+// comparison puts the smaller key at the lower index, so the network of the next
+// power of two serves any PR.
+template <typename K, int PR, int P>
+__device__ __forceinline__ void sort_lane(K (&key)[P]) {
+  constexpr int W = PR <= 4 ? 4 : PR <= 8 ? 8 : 16;
+#pragma unroll
+  for (int p = 1; p < W; p *= 2)
+#pragma unroll
+    for (int k = p; k >= 1; k /= 2)
+#pragma unroll
+      for (int x = 0; x < PR - k; ++x)
+        if (x >= k % p && (x - k % p) % (2 * k) < k && x / (2 * p) == (x + k) / (2 * p)) {
+          const K lo = key[x], hi = key[x + k];
+          key[x] = min(lo, hi);
+          key[x + k] = max(lo, hi);
+        }
+}
+
+// Ascending sort of the first PR registers of each group of LANES lanes, element
+// e = lane * PR + r: lanes sort their own registers, then runs of 2, 4, ... lanes
+// merge (mirrored comparison, half-cleaners across lanes, sort within lanes).
+// Ten steps of a 16-lane sort need shuffles; with elements dealt to the lanes in
+// turn 25 would.  The merges are one loop, not unrolled: with a fully unrolled
+// network per PR, warps of different PR evicted each other's instructions
+// (no-instruction stalls 27 of 33 cycles per issue, 2.25 ms).
+template <typename K, int LANES, int PR, int P>
+__device__ __forceinline__ void sort_keys(K (&key)[P], uint32_t hl) {
+#pragma unroll 1
+  for (int run = 1;; run *= 2) {   // lanes per sorted run
+    sort_lane<K, PR>(key);
+    if (run == LANES) break;
+    const bool lower = (hl & (uint32_t)run) == 0;
+#pragma unroll
+    for (int r = 0; r < (PR + 1) / 2; ++r) {
+      const K x = RowKey<K>::shfl_xor(key[PR - 1 - r], 2 * run - 1);
+      const K y = RowKey<K>::shfl_xor(key[r], 2 * run - 1);
+      key[r] = lower ? min(key[r], x) : max(key[r], x);
+      if (r != PR - 1 - r) key[PR - 1 - r] = lower ? min(key[PR - 1 - r], y) : max(key[PR - 1 - r], y);
+    }
+#pragma unroll 1
+    for (int j = run / 2; j > 0; j /= 2) {
+      const bool low = (hl & (uint32_t)j) == 0;
+#pragma unroll
+      for (int r = 0; r < PR; ++r) {
+        const K o = RowKey<K>::shfl_xor(key[r], j);
+        key[r] = low ? min(key[r], o) : max(key[r], o);
+      }
+    }
+  }
+}
+
+// Sort and leave the keys in order in skey[0 .. LANES * regs).
+template <typename K, int LANES, int PR, int P>
+__device__ __forceinline__ void sort_to_shared(K (&key)[P], uint32_t hl, K* skey) {
+  sort_keys<K, LANES, PR>(key, hl);
+  __syncwarp();   // staged keys have been read
+#pragma unroll
+  for (int r = 0; r < PR; ++r) skey[hl * PR + r] = key[r];
+}
+
+// One lane's share of a chunk of up to LANES entries of a row of A.
+template <typename T, typename K>
+struct Entry {
+  // an index into B, in 32 bits where the keys are (only used with nnz(B) < 2^31)
+  typedef typename std::conditional<sizeof(K) == 4, int32_t, long long>::type Index;
+  T a;
+  Index base;        // candidate slot sl of this entry is base + sl
+  uint32_t excl, len;
+};
+
+// Load the chunk and lay its B ranges out one after the other; entries without
+// candidates are moved out of the way, so that range starts are distinct.
+// Returns the chunk's candidates (per row).
+template <typename T, typename K, int LANES>
+__device__ __forceinline__ uint32_t load_entries(const RowArgs<T>& R, int64_t p, bool in, uint32_t hl, uint32_t shift,
+                                                 Entry<T, K>& e) {
+  typedef typename Entry<T, K>::Index Index;
+  Index b0 = 0;
+  e.a = T(0);
+  e.len = 0;
+  if (in) {
+    const int32_t k = R.aci[p];
+    e.a = R.av[p];
+    const int64_t x = R.brp[k], y = R.brp[k + 1];
+    if (SpVal<T>::present(e.a)) {
+      b0 = (Index)x;
+      e.len = (uint32_t)(y - x);
+    }
+  }
+  constexpr uint32_t kAll = LANES == 32 ? 0xffffffffu : (1u << (LANES & 31)) - 1u;
+  const uint32_t some = (__ballot_sync(0xffffffffu, e.len > 0) >> shift) & kAll;
+  if (!__all_sync(0xffffffffu, (some & (some + 1)) == 0)) {   // a gap: compact
+    const uint32_t n = __popc(some);
+    const uint32_t src = hl < n ? nth_set_bit(some, hl) : 0u;
+    e.a = __shfl_sync(0xffffffffu, e.a, src, LANES);
+    b0 = __shfl_sync(0xffffffffu, b0, src, LANES);
+    const uint32_t l = __shfl_sync(0xffffffffu, e.len, src, LANES);
+    e.len = hl < n ? l : 0u;
+  }
+  uint32_t incl = e.len;
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o, LANES);
+    if (hl >= (uint32_t)o) incl += y;
+  }
+  e.excl = incl - e.len;
+  e.base = b0 - (Index)e.excl;
+  return __shfl_sync(0xffffffffu, incl, LANES - 1, LANES);
+}
+
+// Owner of slot w0 + hl: the ranges that start at or before it, counted from
+// the bits of this window's starts; `started` counts those of earlier windows.
+template <typename T, typename K, int LANES>
+__device__ __forceinline__ uint32_t slot_owner(const Entry<T, K>& e, uint32_t w0, uint32_t hl, uint32_t shift,
+                                               uint32_t& started) {
+  const uint32_t d = e.excl - w0;
+  const uint32_t bit = (e.len > 0 && d < (uint32_t)LANES) ? 1u << (d + shift) : 0u;
+  uint32_t starts = __reduce_or_sync(0xffffffffu, bit) >> shift;
+  if (LANES < 32) starts &= (1u << (LANES & 31)) - 1u;
+  const uint32_t own = started + __popc(starts & (0xffffffffu >> (31u - hl))) - 1u;
+  started += __popc(starts);
+  return own & (LANES - 1);
+}
+
+// Key of candidate `slot`, its value left in sval[slot]; ~0 for none.
+template <typename T, typename K, int SB>
+__device__ __forceinline__ K make_key(const RowArgs<T>& R, T a, T b, int32_t j, uint32_t slot, uint32_t* sval,
+                                      bool& bad) {
+  T c = T(0);
+  bool ok = SpVal<T>::combine(a, b, c);
+  if ((uint32_t)j >= (uint32_t)R.N) {   // N < 2^31
+    bad = true;
+    ok = false;
+  }
+  sval[slot] = VKey<T>::enc(c);
+  return ok ? ((K)(uint32_t)j << SB) | (K)slot : ~(K)0;
+}
+
+// One row per group of LANES lanes, of at most LANES * regs candidates (regs <= P).
+template <typename T, typename K, int LANES, int P>
+__device__ __forceinline__ void do_row(const RowArgs<T>& R, int64_t i, bool mine, unsigned long long o0, int64_t a0,
+                                       int64_t alen, int regs, uint32_t hl, uint32_t shift, K* skey,
+                                       uint32_t* sval) {
+  constexpr int SB = sizeof(K) == 8 ? 32 : (LANES == 16 ? 7 : 9);   // slot bits
+  constexpr K kMask = ((K)1 << SB) - 1;
+  constexpr uint32_t kAll = LANES == 32 ? 0xffffffffu : (1u << (LANES & 31)) - 1u;
+  typedef typename Entry<T, K>::Index Index;
+  K key[P];
+  uint32_t n;   // candidates of this row
+  bool bad = false;
+  if (__all_sync(0xffffffffu, alen <= LANES)) {
+    Entry<T, K> e;
+    n = load_entries<T, K, LANES>(R, a0 + hl, (int64_t)hl < alen, hl, shift, e);
+    int32_t j[P];
+    T a[P], b[P];
+    uint32_t started = 0;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      if (r >= 4 && r >= regs) break;
+      const uint32_t sl = (uint32_t)(r * LANES) + hl;
+      const uint32_t t = slot_owner<T, K, LANES>(e, (uint32_t)(r * LANES), hl, shift, started);
+      a[r] = __shfl_sync(0xffffffffu, e.a, t, LANES);
+      const Index q = __shfl_sync(0xffffffffu, e.base, t, LANES) + (Index)sl;
+      j[r] = 0;
+      b[r] = T(0);
+      if (sl < n) {
+        j[r] = R.bci[q];
+        b[r] = R.bv[q];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const uint32_t sl = (uint32_t)(r * LANES) + hl;
+      key[r] = ~(K)0;
+      if (r >= 4 && r >= regs) continue;
+      if (sl < n) key[r] = make_key<T, K, SB>(R, a[r], b[r], j[r], sl, sval, bad);
+    }
+  } else {
+    int64_t most = alen;
+    if (LANES < 32) most = max(most, (int64_t)__shfl_xor_sync(0xffffffffu, (long long)most, 16));
+    n = 0;
+    for (int64_t pa = 0; pa < most; pa += LANES) {
+      Entry<T, K> e;
+      const uint32_t total =
+          load_entries<T, K, LANES>(R, a0 + pa + hl, pa + (int64_t)hl < alen, hl, shift, e);
+      uint32_t longest = total;
+      if (LANES < 32) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, 16));
+      uint32_t started = 0;
+      for (uint32_t w0 = 0; w0 < longest; w0 += LANES) {
+        const uint32_t sl = w0 + hl;
+        const uint32_t t = slot_owner<T, K, LANES>(e, w0, hl, shift, started);
+        const T a = __shfl_sync(0xffffffffu, e.a, t, LANES);
+        const Index q = __shfl_sync(0xffffffffu, e.base, t, LANES) + (Index)sl;
+        if (sl < total) skey[n + sl] = make_key<T, K, SB>(R, a, R.bv[q], R.bci[q], n + sl, sval, bad);
       }
       n += total;
     }
     __syncwarp();
-    // sort 64 keys per half: element e = r * 16 + hl
-    constexpr int P = kPairMax / 16;
-    unsigned long long key[P];
 #pragma unroll
     for (int r = 0; r < P; ++r) {
-      const uint32_t e = (uint32_t)r * 16u + hl;
-      key[r] = (mine && e < n) ? sk[e] : kNoKey;
+      const uint32_t sl = (uint32_t)(r * LANES) + hl;
+      key[r] = sl < n ? skey[sl] : ~(K)0;
     }
-#pragma unroll
-    for (int k = 2; k <= kPairMax; k <<= 1) {
-#pragma unroll
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        if (j >= 16) {
-#pragma unroll
-          for (int r = 0; r < P; ++r) {
-            const int rp = r ^ (j >> 4);
-            if (rp > r) {
-              const bool up = ((r * 16) & k) == 0;
-              const unsigned long long x = key[r], y = key[rp];
-              if ((x > y) == up) {
-                key[r] = y;
-                key[rp] = x;
-              }
-            }
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < P; ++r) {
-            const uint32_t e = (uint32_t)r * 16u + hl;
-            const bool up = (e & (uint32_t)k) == 0;
-            const unsigned long long o = shfl_xor64(key[r], j);
-            const bool lower = (hl & (uint32_t)j) == 0;
-            const bool take_min = lower == up;
-            key[r] = take_min ? (o < key[r] ? o : key[r]) : (o > key[r] ? o : key[r]);
-          }
-        }
+  }
+  if (__any_sync(0xffffffffu, bad) && bad) atomicCAS(R.status, kSpOk, (uint32_t)kSpBadIndex);
+  if (P == 8) {
+    if (regs <= 4) sort_to_shared<K, LANES, 4>(key, hl, skey);
+    else if (regs == 5) sort_to_shared<K, LANES, 5>(key, hl, skey);
+    else if (regs == 6) sort_to_shared<K, LANES, 6>(key, hl, skey);
+    else if (regs == 7) sort_to_shared<K, LANES, 7>(key, hl, skey);
+    else sort_to_shared<K, LANES, 8>(key, hl, skey);
+  } else {
+    if (regs <= 8) sort_to_shared<K, LANES, 8>(key, hl, skey);
+    else if (regs <= 12) sort_to_shared<K, LANES, 12 <= P ? 12 : P>(key, hl, skey);
+    else sort_to_shared<K, LANES, P>(key, hl, skey);
+  }
+  __syncwarp();   // sorted keys and all values are in shared memory
+  // heads of column runs, in order
+  int32_t* tc = R.tcol + o0;
+  T* tv = R.tval + o0;
+  uint32_t kept = 0;
+#pragma unroll 1
+  for (int r = 0; r < regs; ++r) {
+    const uint32_t e = (uint32_t)(r * LANES) + hl;
+    const K me = skey[e], before = e ? skey[e - 1] : ~(K)0;
+    const bool head = me != ~(K)0 && ((before >> SB) != (me >> SB) || before == ~(K)0);
+    const uint32_t bal = __ballot_sync(0xffffffffu, head);
+    if (head) {
+      uint32_t v = sval[(uint32_t)(me & kMask)];
+      for (uint32_t q = e + 1; q < (uint32_t)(regs * LANES); ++q) {
+        const K other = skey[q];
+        if ((other >> SB) != (me >> SB) || other == ~(K)0) break;
+        v = min(v, sval[(uint32_t)(other & kMask)]);
       }
+      const uint32_t pos = kept + __popc((bal >> shift) & ((1u << hl) - 1u));
+      tc[pos] = (int32_t)(me >> SB);
+      tv[pos] = VKey<T>::dec(v);
     }
-    // heads of column runs, in order
-    uint32_t kept = 0;
-    uint32_t carry = 0xFFFFFFFFu;
-#pragma unroll
-    for (int r = 0; r < P; ++r) {
-      const uint32_t col = (uint32_t)(key[r] >> 32);
-      uint32_t pc = __shfl_up_sync(0xffffffffu, col, 1, 16);
-      if (hl == 0) pc = carry;
-      const bool head = mine && key[r] != kNoKey && col != pc;
-      const uint32_t b = __ballot_sync(0xffffffffu, head) & (half ? 0xFFFF0000u : 0x0000FFFFu);
-      if (head) {
-        const uint32_t pos = kept + __popc(b & ((1u << lane) - 1u));
-        tcol[o0 + pos] = (int32_t)col;
-        tval[o0 + pos] = VKey<T>::dec((uint32_t)key[r]);
-      }
-      kept += __popc(b);
-      carry = __shfl_sync(0xffffffffu, col, 15, 16);
+    kept += __popc((bal >> shift) & kAll);
+  }
+  if (mine && hl == 0) R.cnt[i] = kept;
+  __syncwarp();
+}
+
+// LANES = 16: every row of up to kSmallRowMax candidates, two per warp.
+// LANES = 32: the listed rows.
+template <typename T, typename K, int LANES>
+__global__ void __launch_bounds__(kRowWarps * 32)
+    k_rows(const RowArgs<T> R, const int64_t* __restrict__ rows, int64_t nrows) {
+  constexpr int kRpw = 32 / LANES, kCap = LANES == 16 ? kSmallRowMax : kWarpRowMax;
+  __shared__ K s_key[kRowWarps][kRpw][kCap];
+  __shared__ uint32_t s_val[kRowWarps][kRpw][kCap];
+  const uint32_t lane = threadIdx.x & 31u, hl = lane & (LANES - 1), grp = lane / LANES, shift = lane - hl;
+  K* skey = s_key[threadIdx.x >> 5][grp];
+  uint32_t* sval = s_val[threadIdx.x >> 5][grp];
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t x = warp * kRpw; x < nrows; x += nwarps * kRpw) {
+    const bool in = x + grp < nrows;
+    const int64_t i = in ? (rows ? rows[x + grp] : x + grp) : 0;
+    unsigned long long o0 = 0, ub = 0;
+    int64_t a0 = 0, alen = 0;
+    if (in) {
+      o0 = R.off[i];
+      ub = R.off[i + 1] - o0;
+      a0 = R.arp[i];
+      alen = R.arp[i + 1] - a0;
     }
-    if (mine && hl == 0) cnt[i] = kept;
-    __syncwarp();
+    const bool mine = in && ub <= (unsigned long long)kCap;
+    if (!mine || ub == 0) {
+      ub = 0;
+      alen = 0;
+    }
+    uint32_t most = (uint32_t)ub;
+    if (LANES < 32) most = max(most, __shfl_xor_sync(0xffffffffu, most, 16));
+    const uint32_t regs = (most + LANES - 1) / LANES;
+    if (regs == 0) {
+      if (mine && hl == 0) R.cnt[i] = 0;
+      continue;
+    }
+    do_row<T, K, LANES, kCap / LANES>(R, i, mine, o0, a0, alen, (int)regs, hl, shift, skey, sval);
   }
 }
 
+// ---- long rows of matrices with few columns: dense accumulation --------------
+// A block takes a row.  Its candidates go into an array of one 32-bit word per
+// column in shared memory (order-preserving value bits, atomicMin), which is
+// then read in column order: no expansion to memory, no sort, no limit on the
+// row's candidates.  Up to kDenseCols columns fit one pass; wider matrices take
+// kDensePasses passes over the row at most, past that the expansion below is
+// used.  Rows of at least kHeavyRow candidates are dealt first, so that none
+// starts last.  Bound by the gather from L2 and shared-memory atomics.
+// RMAT scale 14, edge factor 8: 21.5 ms per call with the rows expanded, sorted
+// by CUB and reduced by one warp each -> 0.82 ms.  RMAT 17 (131072 columns, three
+// passes), edge factor 2: 27.1 -> 6.3 ms.
+constexpr int kDenseCols = 49152;                      // 192 KB
+constexpr int kDensePasses = 4;
+constexpr unsigned long long kHeavyRow = 32768;
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT) k_rows_dense(const RowArgs<T> R, const int64_t* __restrict__ rows, int64_t nheavy,
+                                                   int64_t nlong, int cap, unsigned long long* next) {
+  extern __shared__ uint32_t s_acc[];   // cap words
+  __shared__ uint32_t s_excl[NT + 1];
+  __shared__ long long s_base[NT];
+  __shared__ T s_a[NT];
+  __shared__ uint32_t s_warp[NT / 32];
+  __shared__ unsigned long long s_item;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+  for (int c = (int)tid; c < cap; c += NT) s_acc[c] = 0xFFFFFFFFu;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) s_item = atomicAdd(next, 1ull);
+    __syncthreads();
+    const int64_t item = (int64_t)s_item;
+    if (item >= nheavy + nlong) break;
+    const int64_t i = item < nheavy ? rows[item] : rows[R.M - 1 - (item - nheavy)];
+    const int64_t a0 = R.arp[i], a1 = R.arp[i + 1];
+    const unsigned long long o0 = R.off[i];
+    uint32_t kept = 0;
+    for (int64_t c0 = 0; c0 < R.N; c0 += cap) {
+      const uint32_t cols = (uint32_t)min((int64_t)cap, R.N - c0);
+      for (int64_t pa = a0; pa < a1; pa += NT) {
+        // this chunk's entries and the block-wide offsets of their B ranges
+        uint32_t len = 0;
+        long long b0 = 0;
+        T a = T(0);
+        if (pa + tid < a1) {
+          const int32_t k = R.aci[pa + tid];
+          a = R.av[pa + tid];
+          b0 = R.brp[k];   // (of absent entries too: their B rows' columns are checked)
+          len = (uint32_t)(R.brp[k + 1] - b0);
+        }
+        const uint32_t incl = warp_incl_scan(len);
+        if (lane == 31) s_warp[w] = incl;
+        __syncthreads();
+        if (w == 0) {
+          const uint32_t x = lane < NT / 32 ? s_warp[lane] : 0u;
+          const uint32_t y = warp_incl_scan(x);
+          if (lane < NT / 32) s_warp[lane] = y - x;
+          if (lane == 31) s_excl[NT] = y;
+        }
+        __syncthreads();
+        const uint32_t excl = s_warp[w] + incl - len;
+        s_excl[tid] = excl;
+        s_base[tid] = b0 - (long long)excl;
+        s_a[tid] = a;
+        __syncthreads();
+        const uint32_t total = s_excl[NT];
+#pragma unroll 4
+        for (uint32_t sl = tid; sl < total; sl += NT) {
+          uint32_t t = 0;   // the last entry whose range starts at or before sl
+#pragma unroll
+          for (uint32_t step = NT / 2; step >= 1; step >>= 1)
+            if (s_excl[t + step] <= sl) t += step;
+          const long long q = s_base[t] + sl;
+          const int32_t j = R.bci[q];
+          T c = T(0);
+          const bool ok = SpVal<T>::present(s_a[t]) && SpVal<T>::combine(s_a[t], R.bv[q], c);
+          if (j < 0 || (int64_t)j >= R.N) atomicCAS(R.status, kSpOk, (uint32_t)kSpBadIndex);
+          else if (ok && (uint32_t)(j - c0) < cols) atomicMin(&s_acc[(uint32_t)(j - c0)], VKey<T>::enc(c));
+        }
+        __syncthreads();   // the chunk's entries have been used
+      }
+      // columns in order: each warp owns a range of them; count, then write and clear
+      const uint32_t per = (((cols + NT / 32 - 1) / (NT / 32)) + 31u) & ~31u;
+      const uint32_t lo = min(w * per, cols), hi = min(lo + per, cols);
+      __syncthreads();
+      uint32_t mine = 0;
+      for (uint32_t c = lo + lane; c < hi; c += 32) mine += s_acc[c] != 0xFFFFFFFFu ? 1u : 0u;
+      mine = __reduce_add_sync(0xffffffffu, mine);
+      if (lane == 0) s_warp[w] = mine;
+      __syncthreads();
+      uint32_t before = 0, all = 0;
+      for (uint32_t x = 0; x < NT / 32; ++x) {
+        const uint32_t y = s_warp[x];
+        before += x < w ? y : 0u;
+        all += y;
+      }
+      unsigned long long pos = o0 + kept + before;
+      for (uint32_t c = lo; c < hi; c += 32) {
+        const bool in = c + lane < hi;
+        const uint32_t v = in ? s_acc[c + lane] : 0xFFFFFFFFu;
+        const bool have = v != 0xFFFFFFFFu;
+        const uint32_t bal = __ballot_sync(0xffffffffu, have);
+        if (have) {
+          const unsigned long long at = pos + __popc(bal & ((1u << lane) - 1u));
+          R.tcol[at] = (int32_t)(c0 + c + lane);
+          R.tval[at] = VKey<T>::dec(v);
+          s_acc[c + lane] = 0xFFFFFFFFu;
+        }
+        pos += __popc(bal);
+      }
+      kept += all;
+      __syncthreads();
+    }
+    if (tid == 0) R.cnt[i] = kept;
+  }
+}
+
+template <typename T, int NT>
+cudaError_t launch_dense(const RowArgs<T>& R, const int64_t* rows, int64_t nheavy, int64_t nlong, int cap, int sms,
+                         unsigned long long* next, cudaStream_t st) {
+  const size_t smem = (size_t)cap * 4;
+  cudaError_t e = cudaFuncSetAttribute(k_rows_dense<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kDenseCols * 4);
+  int per = 0;
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rows_dense<T, NT>, NT, smem);
+  if (e != cudaSuccess) return e;
+  if (per < 1) return cudaErrorInvalidConfiguration;
+  const int64_t blocks = std::min<int64_t>(nheavy + nlong, (int64_t)per * sms);
+  k_rows_dense<T, NT><<<(int)blocks, NT, smem, st>>>(R, rows, nheavy, nlong, cap, next);
+  return cudaGetLastError();
+}
+
+// ---- long rows of wide matrices: expand-sort-compress over a row list --------
 template <typename T>
 __global__ void k_expand(int64_t L, const int64_t* __restrict__ rows, int64_t N, const int64_t* __restrict__ arp,
                          const int32_t* __restrict__ aci, const T* __restrict__ av, const int64_t* __restrict__ brp,
@@ -626,37 +842,43 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
     plan.nnz = 0;
     return B2_SUCCESS;
   }
-  DBuf<unsigned long long> ub, off, lcount;
-  DBuf<int64_t> lrows;
-  DBuf<uint32_t> status;
+  DBuf<unsigned long long> ub, off;
+  DBuf<int64_t> lrows, mrows;
+  DBuf<SpCounters> counters;
   DBuf<unsigned char> tmp;
   if (ub.alloc((size_t)M + 1, st) != cudaSuccess || off.alloc((size_t)M + 1, st) != cudaSuccess ||
-      status.alloc(1, st) != cudaSuccess || lrows.alloc((size_t)M, st) != cudaSuccess ||
-      lcount.alloc(1, st) != cudaSuccess)
+      counters.alloc(1, st) != cudaSuccess || lrows.alloc((size_t)M, st) != cudaSuccess ||
+      mrows.alloc((size_t)M, st) != cudaSuccess)
     return B2_OUT_OF_MEMORY;
-  cudaError_t e = cudaMemsetAsync(status.p, 0, 4, st);
+  // long rows accumulate densely where their columns fit kDensePasses passes;
+  // such a row needs at most N result slots (kept past the ordinary rows' limit,
+  // by which the row kernels tell them apart)
+  const bool dense = N <= (int64_t)kDenseCols * kDensePasses;
+  const unsigned long long heavy_from = dense ? kHeavyRow : 0ull;
+  const unsigned long long long_slots =
+      dense ? std::max<unsigned long long>((unsigned long long)N, (unsigned long long)kWarpRowMax + 1) : 0ull;
+  cudaError_t e = cudaMemsetAsync(counters.p, 0, sizeof(SpCounters), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(ub.p + M, 0, 8, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(lcount.p, 0, 8, st);
   if (e == cudaSuccess) {
-    k_row_bound<<<grid_rows(M), 256, 0, st>>>(M, K, A->nnz, B->nnz, arp, A->colind, brp, ub.p, status.p, lrows.p,
-                                              lcount.p);
+    k_row_bound<<<grid_rows((M + 3) / 4), 256, 0, st>>>(M, K, A->nnz, B->nnz, arp, A->colind, brp, ub.p, counters.p,
+                                                        lrows.p, mrows.p, heavy_from, long_slots);
     e = cudaGetLastError();
   }
   size_t tb = 0;
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb, ub.p, off.p, M + 1, st);
   if (e == cudaSuccess) e = tmp.alloc(tb, st);
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp.p, tb, ub.p, off.p, M + 1, st);
-  unsigned long long hv[2] = {0, 0};   // total candidates, long rows
-  uint32_t hs = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hv[0], off.p + M, 8, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hv[1], lcount.p, 8, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, status.p, 4, cudaMemcpyDeviceToHost, st);
+  unsigned long long U = 0;   // result slots
+  SpCounters hc = {};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&U, off.p + M, 8, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&hc, counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return from_cuda(e);
-  if (hs == kSpBadIndex) return B2_INVALID_INDEX;
-  if (hs == kSpBadRowptr) return B2_INVALID_ROWPTR;
-  const unsigned long long U = hv[0];
-  const int64_t L = (int64_t)hv[1];
+  if (hc.status == kSpBadIndex) return B2_INVALID_INDEX;
+  if (hc.status == kSpBadRowptr) return B2_INVALID_ROWPTR;
+  if (hc.too_long) return B2_NOT_SUPPORTED;   // the row kernels count a row's candidates in 32 bits
+  const int64_t nheavy = (int64_t)hc.heavy, nlong = (int64_t)hc.lng, nmid = (int64_t)hc.mid;
+  uint32_t* const status = &counters.p->status;
   DBuf<int32_t> tcol;
   DBuf<T> tval;
   DBuf<int64_t> cnt;
@@ -667,22 +889,38 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t want = (M + kRowWarps - 1) / kRowWarps;
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * 6));
-    const int pair_blocks =
-        (int)std::max<int64_t>(1, std::min<int64_t>((M + 2 * kRowWarps - 1) / (2 * kRowWarps), (int64_t)sms * 16));
-    k_rows_pair<T><<<pair_blocks, kRowWarps * 32, 0, st>>>(M, N, arp, A->colind, (const T*)A->values, brp,
-                                                         B->colind, (const T*)B->values, off.p, tcol.p, tval.p,
-                                                         cnt.p, status.p);
-    e = cudaGetLastError();
+    const RowArgs<T> R = {M,      N,     arp,    A->colind, (const T*)A->values, brp,   B->colind, (const T*)B->values,
+                          off.p, tcol.p, tval.p, cnt.p,     status};
+    if (dense && nheavy + nlong > 0) {   // first: the longest of them take longest
+      DBuf<unsigned long long> next;
+      if (next.alloc(1, st) != cudaSuccess) return B2_OUT_OF_MEMORY;
+      e = cudaMemsetAsync(next.p, 0, 8, st);
+      const int cap = (int)std::min<int64_t>((N + 31) / 32 * 32, kDenseCols);
+      // 512 threads while two blocks or more fit an SM, else 1024
+      if (e == cudaSuccess)
+        e = cap <= 24576 ? launch_dense<T, 512>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st)
+                         : launch_dense<T, 1024>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st);
+    }
+    const bool b32 = B->nnz < (1ll << 31);   // 32-bit indices into B beside the 32-bit keys
+    auto blocks = [&](int64_t warps, int per_sm) {
+      return (int)std::max<int64_t>(1, std::min<int64_t>((warps + kRowWarps - 1) / kRowWarps, (int64_t)sms * per_sm));
+    };
     if (e == cudaSuccess) {
-      k_rows_warp<T><<<blocks, kRowWarps * 32, 0, st>>>(M, N, arp, A->colind, (const T*)A->values, brp, B->colind,
-                                                      (const T*)B->values, off.p, tcol.p, tval.p, cnt.p, status.p);
+      const int g = blocks((M + 1) / 2, 16);
+      if (N < (1ll << 25) && b32) k_rows<T, uint32_t, 16><<<g, kRowWarps * 32, 0, st>>>(R, nullptr, M);
+      else k_rows<T, unsigned long long, 16><<<g, kRowWarps * 32, 0, st>>>(R, nullptr, M);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && nmid > 0) {
+      const int g = blocks(nmid, 16);
+      if (N < (1ll << 23) && b32) k_rows<T, uint32_t, 32><<<g, kRowWarps * 32, 0, st>>>(R, mrows.p, nmid);
+      else k_rows<T, unsigned long long, 32><<<g, kRowWarps * 32, 0, st>>>(R, mrows.p, nmid);
       e = cudaGetLastError();
     }
   } else {
     e = cudaMemsetAsync(cnt.p, 0, (size_t)M * sizeof(int64_t), st);
   }
+  const int64_t L = dense ? 0 : nheavy;   // rows to expand
   // long rows: expand, segmented sort, compress into their scratch slots
   DBuf<unsigned long long> lub, loff;
   DBuf<int32_t> col0, col1;
@@ -709,7 +947,7 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
         val1.alloc(LU, st) != cudaSuccess)
       return B2_OUT_OF_MEMORY;
     k_expand<T><<<grid_rows(L), 256, 0, st>>>(L, lrows.p, N, arp, A->colind, (const T*)A->values, brp, B->colind,
-                                              (const T*)B->values, loff.p, col0.p, val0.p, status.p);
+                                              (const T*)B->values, loff.p, col0.p, val0.p, status);
     e = cudaGetLastError();
     size_t tbs = 0;
     if (e == cudaSuccess)
@@ -732,7 +970,8 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp4.p, tb4, cnt.p, crp.p, M + 1, st);
   int64_t nnz = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&nnz, crp.p + M, 8, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, status.p, 4, cudaMemcpyDeviceToHost, st);
+  uint32_t hs = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, status, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return from_cuda(e);
   if (hs == kSpBadIndex) return B2_INVALID_INDEX;
