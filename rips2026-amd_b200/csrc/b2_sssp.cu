@@ -182,6 +182,10 @@ struct WarpQ {
 struct Tally {
   unsigned long long edges = 0, impr = 0, pushes = 0;
   uint64_t keep = 0;   // L2 evict_last cache policy for label traffic
+  // delta: what the manager wants to know of a phase, kept per lane until the
+  // phase ends (flush_phase) so that the frontier items share no address
+  uint32_t min_key = 0xFFFFFFFFu;   // smallest label expanded (none: no valid vertex)
+  uint32_t heavy = 0;               // heavy out-edges of the members
   WarpQ q;
 };
 
@@ -530,24 +534,11 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
     }
   }
   if (MODE == kModeDelta) {
-    if (__any_sync(0xffffffffu, valid) && lane == 0 && ldcg(&c->bucket_valid) == 0) c->bucket_valid = 1;
+    if (valid) t.min_key = min(t.min_key, du);
     if (members) {
       // settled in this light round: its heavy suffix is relaxed once by the heavy phase
       const bool want = valid && has_heavy && atomicExch(&P.hstamp[v], R.hround) != R.hround;
-      if (P.in_rowptr) {
-        // push cost of the heavy pass and the bucket's smallest label (the pull's early-exit bound)
-        unsigned long long hv = want ? (unsigned long long)(row_end - hi) : 0ull;
-        uint32_t mk = valid ? du : 0xFFFFFFFFu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          hv += __shfl_xor_sync(0xffffffffu, hv, o);
-          mk = min(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-        }
-        if (lane == 0) {
-          if (hv) atomicAdd(&c->member_heavy, hv);
-          if (mk != 0xFFFFFFFFu) atomicMin(&c->cur_min_key, mk);
-        }
-      }
+      if (want) t.heavy += (uint32_t)(row_end - hi);
       stage(t.q.memb, t.q.nm, want, v);
       if (t.q.nm > kMemBuf / 2) {
         publish(P, &c->members_count, kQMembers, t.q.memb, t.q.nm, 14);
@@ -694,6 +685,47 @@ template <class W, bool PRED, int MODE>
 __device__ __forceinline__ void frontier_chunk(const Params& P, const PhaseRec& R, uint32_t base, Tally& t) {
   uint32_t carry = 0;
   frontier_item<W, PRED, MODE>(P, R, base / 32, false, false, carry, t);
+}
+
+// End of a relaxation phase: this warp's members' heavy edges and smallest
+// expanded label go to its slot in shared memory; flush_block adds the block's
+// slots to the control block once, before it arrives at the barrier.  A global
+// addition and minimum per 32-vertex item (100 K on one line in the large
+// phases of RMAT-24, with every item's read of bucket_valid queued behind them)
+// held the solve up: RMAT-24 8.35 -> 6.57 ms, 4096^2 grid 5.53 -> 4.98 ms.
+struct WarpPhase {
+  unsigned long long heavy;
+  uint32_t min_key;
+  uint32_t pad;
+};
+__device__ __forceinline__ void flush_phase(WarpPhase* slot, Tally& t) {
+  const uint32_t mk = __reduce_min_sync(0xffffffffu, t.min_key);
+  const uint32_t lo = __reduce_add_sync(0xffffffffu, t.heavy & 0xffffu);
+  const uint32_t hi = __reduce_add_sync(0xffffffffu, t.heavy >> 16);
+  if (lane_id() == 0) {
+    slot->heavy = ((unsigned long long)hi << 16) + lo;
+    slot->min_key = mk;
+  }
+  t.min_key = 0xFFFFFFFFu;
+  t.heavy = 0;
+}
+// (warp 0, after a block barrier)
+__device__ __forceinline__ void flush_block(const Params& P, WarpPhase* slots) {
+  const uint32_t lane = lane_id();
+  const bool in = lane < (uint32_t)kWarpsPerBlock;
+  const uint32_t mk = __reduce_min_sync(0xffffffffu, in ? slots[lane].min_key : 0xFFFFFFFFu);
+  if (mk == 0xFFFFFFFFu) return;   // nothing expanded
+  unsigned long long hv = in ? slots[lane].heavy : 0ull;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) hv += __shfl_xor_sync(0xffffffffu, hv, o);
+  if (lane == 0) {
+    Control* c = P.ctl;
+    c->bucket_valid = 1;
+    if (P.in_rowptr) {
+      atomicMin(&c->cur_min_key, mk);
+      if (hv) atomicAdd(&c->member_heavy, hv);
+    }
+  }
 }
 
 constexpr uint32_t kHubGrab = B2_HUB_GRAB;   // hub chunks per work item
@@ -1248,6 +1280,7 @@ template <class W, bool PRED, int MODE>
 __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(Params P) {
   using L = Label<PRED>;
   __shared__ PhaseRec s_rec;
+  __shared__ WarpPhase s_phase[kWarpsPerBlock];
   extern __shared__ uint32_t s_stage[];   // kStageWords per warp
   Tally t;
   t.keep = l2_keep_policy();
@@ -1279,6 +1312,7 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(Params P) {
     PhaseRec R = s_rec;
     if (R.kind == kPhaseDone) break;
     R.fcount = min(R.fcount, P.qcap);
+    const bool expands = R.kind == kPhaseProcess || (R.kind == kPhaseLocal && blockIdx.x == 0);
     if (R.kind == kPhaseProcess) {
       process_phase<W, PRED, MODE>(P, R, t);
     } else if (R.kind == kPhaseLocal) {
@@ -1371,6 +1405,11 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(Params P) {
           P.out_pred[o] = pr;
         }
       }
+    }
+    if (MODE == kModeDelta && expands) {
+      flush_phase(s_phase + (threadIdx.x >> 5), t);
+      __syncthreads();
+      if (threadIdx.x < 32) flush_block(P, s_phase);
     }
     if (MODE == kModeBF) {
       ok = grid_barrier((GridBarrier*)c, gridDim.x, P.budget_ns, [&] { c->work_next = 0; manager_bf(P); });
