@@ -70,6 +70,7 @@ struct PhaseRec {
   uint32_t dbase_b;
   uint32_t dense;       // 0: read the frontier queue; kDenseNear / kDenseSlot: sweep the stamps
   uint32_t fstamp;      // stamp value marking the frontier's vertices in a sweep
+  uint32_t direct;      // 1: a small frontier, relaxed without the filter load
 };
 
 // One entry per executed phase when tracing is on (manager-written).
@@ -81,6 +82,8 @@ struct TraceEntry {
   unsigned long long t_ns;  // end of the phase, ns since the first barrier
 };
 constexpr uint32_t kTraceCap = 4096;
+constexpr int kRecWords = sizeof(PhaseRec) / 4;
+static_assert(kRecWords <= 32, "one lane polls each word of the record");
 
 enum PhaseKind : uint32_t {
   kPhaseInit = 0,
@@ -115,33 +118,39 @@ enum QueueId : uint32_t {
   kQNone = 0xFFFFFFFFu,
 };
 
-struct Control {
+// Words that many warps hit at once each have a 128-byte line of their own:
+// atomics on one line queue up in one L2 slice, and a warp that polls or reads a
+// word waits behind those on its neighbours.
+struct alignas(128) Control {
   // grid barrier (must stay first; see b2_common.cuh GridBarrier)
   uint32_t bar_arrive;
   uint32_t bar_gen;
   uint32_t error;
   uint32_t error_site;
-  PhaseRec rec;
+  PhaseRec rec;            // the last phase's record (read by the host)
+  // The running phase's record: word i with the number of the barrier that
+  // released it in the upper half, so that a waiting block polls the record itself.
+  alignas(128) unsigned long long box[32];
   // counters produced during phases
-  uint32_t near_count[2];
-  uint32_t far_count[2];
-  uint32_t slot_count[kRing];
-  uint32_t far_min;        // lower bound of buckets in the active far pile
+  alignas(128) uint32_t near_count[2];
+  alignas(128) uint32_t far_count[2];
+  alignas(128) uint32_t slot_count[kRing];
+  alignas(128) uint32_t hub_count[2];   // chunk entries in each hub list
+  alignas(128) uint32_t members_count;  // entries in the heavy-round member list
+  alignas(128) uint32_t far_min;        // lower bound of buckets in the active far pile
   uint32_t far_min_next;   // exact min of the kept entries during a split
-  uint32_t hub_count[2];   // chunk entries in each hub list
-  uint32_t work_next;      // dynamic work counter of the running phase
   uint32_t bucket_valid;   // a valid vertex was processed in the current bucket
   uint32_t probe_valid;    // PROBE phase result
-  uint32_t members_count;  // entries in the heavy-round member list
+  uint32_t cur_min_key;    // smallest label processed in the current bucket (pull bound)
+  uint32_t heavy_pulls;    // heavy passes run by pull
+  unsigned long long member_heavy;   // heavy out-edges of the current bucket's members (push cost)
+  // manager state
   uint32_t trace_n;
   uint32_t stamp_ctr;      // next dedup stamp (manager and local loop)
   uint32_t local_q;        // LOCAL phase: queue holding the next frontier
   uint32_t local_iters;    // LOCAL phase: sub-phases run inside it
   uint32_t fusion_off;     // a LOCAL sub-phase scanned too many edges: no more fusion this solve
   uint32_t local_total;    // sub-phases run by all LOCAL phases
-  unsigned long long member_heavy;       // heavy out-edges of the current bucket's members (push cost)
-  uint32_t cur_min_key;                  // smallest label processed in the current bucket (pull bound)
-  uint32_t heavy_pulls;                  // heavy passes run by pull
   uint32_t delta_updates;
   // results
   uint32_t iterations;
@@ -151,7 +160,7 @@ struct Control {
   uint32_t first_unchanged;
   uint32_t done;
   unsigned long long t_start;   // globaltimer at the first barrier (solve budget)
-  unsigned long long edges;
+  alignas(128) unsigned long long edges;
   unsigned long long improvements;
   unsigned long long pushes;
 };

@@ -67,12 +67,6 @@ constexpr int kThreads = 512;
 #ifndef B2_HUB_UNROLL
 #define B2_HUB_UNROLL 4
 #endif
-#ifndef B2_HUB_GRAB
-#define B2_HUB_GRAB 2
-#endif
-#ifndef B2_STATIC_NUM   // share of a phase's items dealt round-robin: NUM / 4 (the rest from a counter)
-#define B2_STATIC_NUM 4
-#endif
 constexpr int kUnroll = B2_UNROLL;   // edge slots per lane per step
 
 struct Params {
@@ -145,21 +139,6 @@ __device__ __forceinline__ void set_error(const Params& P, uint32_t code, uint32
   atomicExch(&P.ctl->error_site, site);
 }
 
-__device__ __forceinline__ PhaseRec load_rec(const Control* c) {
-  PhaseRec r;
-  const volatile uint32_t* src = (const volatile uint32_t*)&c->rec;
-  uint32_t* dst = (uint32_t*)&r;
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(PhaseRec) / 4); ++i) dst[i] = src[i];
-  return r;
-}
-__device__ __forceinline__ void store_rec(Control* c, const PhaseRec& r) {
-  volatile uint32_t* dst = (volatile uint32_t*)&c->rec;
-  const uint32_t* src = (const uint32_t*)&r;
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(PhaseRec) / 4); ++i) dst[i] = src[i];
-}
-
 // Per-warp push staging (shared memory).  Worklist insertions are collected
 // per warp and published with one global atomicAdd per flush, so the queue
 // counters (one address each) see ~1/100 of the per-push atomics; flushes
@@ -168,24 +147,27 @@ constexpr int kWarpsPerBlock = kThreads / 32;
 constexpr uint32_t kNearBuf = 256, kFarBuf = 256, kSlotBuf = 256, kMemBuf = 128;
 constexpr uint32_t kDenseSpan = 256;   // vertices per sweep work item (8 per lane)
 constexpr uint32_t kListBuf = kDenseSpan + 32;   // one span's vertices + fewer than 32 carried
-constexpr uint32_t kStageWords = kNearBuf + kFarBuf + 2 * kSlotBuf + kMemBuf + kListBuf;
+constexpr uint32_t kStageWords = kNearBuf + kFarBuf + 2 * kSlotBuf + kMemBuf + kListBuf + kRing;
 constexpr size_t kStageBytes = (size_t)kWarpsPerBlock * kStageWords * 4;
 struct WarpQ {
-  uint32_t* nearb;   // kNearBuf vertex ids
-  uint32_t* farb;    // kFarBuf
-  uint32_t* slotb;   // kSlotBuf (vertex, slot) pairs as 2 words
-  uint32_t* memb;    // kMemBuf
-  uint32_t* listb;   // kListBuf frontier vertices found by a sweep
+  uint32_t* buf;   // this warp's kStageWords
   uint32_t nn = 0, nf = 0, ns = 0, nm = 0;
+  __device__ __forceinline__ uint32_t* nearb() const { return buf; }                               // vertex ids
+  __device__ __forceinline__ uint32_t* farb() const { return buf + kNearBuf; }                     // vertex ids
+  __device__ __forceinline__ uint32_t* slotb() const { return buf + kNearBuf + kFarBuf; }          // (vertex, slot)
+  __device__ __forceinline__ uint32_t* memb() const { return buf + kNearBuf + kFarBuf + 2 * kSlotBuf; }
+  __device__ __forceinline__ uint32_t* histb() const { return memb() + kMemBuf + kListBuf; }   // kRing counters
+  __device__ __forceinline__ uint32_t* listb() const { return memb() + kMemBuf; }   // frontier found by a sweep
 };
 
 struct Tally {
-  unsigned long long edges = 0, impr = 0, pushes = 0;
+  uint32_t edges = 0, impr = 0, pushes = 0;   // of this phase (flush_phase)
   uint64_t keep = 0;   // L2 evict_last cache policy for label traffic
   // delta: what the manager wants to know of a phase, kept per lane until the
   // phase ends (flush_phase) so that the frontier items share no address
   uint32_t min_key = 0xFFFFFFFFu;   // smallest label expanded (none: no valid vertex)
   uint32_t heavy = 0;               // heavy out-edges of the members
+  uint32_t far_min = 0xFFFFFFFFu;   // smallest bucket pushed past the window
   WarpQ q;
 };
 
@@ -197,95 +179,69 @@ __device__ __forceinline__ void stage(uint32_t* buf, uint32_t& cnt, bool want, u
   cnt += __popc(b);
 }
 
-// Publish a staged buffer to queue `qid` with one atomic (warp-collective).
-__device__ __forceinline__ void publish(const Params& P, uint32_t* counter, uint32_t qid, const uint32_t* buf,
-                                        uint32_t cnt, uint32_t site) {
-  if (cnt == 0) return;
-  __syncwarp();
-  uint32_t base = 0;
-  if (lane_id() == 0) base = atomicAdd(counter, cnt);
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if ((uint64_t)base + cnt > P.qcap) {
-    if (lane_id() == 0) set_error(P, kErrQueueOverflow, site);
-    return;
-  }
-  uint32_t* dst = queue_ptr(P, qid) + base;
-  for (uint32_t i = lane_id(); i < cnt; i += 32) dst[i] = buf[i];
-  __syncwarp();
-}
-
-// Window-slot entries carry their slot: publish one slot group at a time.
-__device__ __forceinline__ void publish_slots(const Params& P, WarpQ& q) {
-  Control* c = P.ctl;
-  __syncwarp();
-  uint32_t remaining = q.ns;
-  // entries are (v, slot) pairs; process in rounds, one distinct slot per round
-  while (remaining) {
-    uint32_t s0 = q.slotb[2 * 0 + 1];
-    // lane-strided scan: count entries with slot s0
-    uint32_t mine = 0;
-    for (uint32_t i = lane_id(); i < q.ns; i += 32)
-      if (q.slotb[2 * i + 1] == s0) ++mine;
-    const uint32_t incl = warp_incl_scan(mine);
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t base = 0;
-    if (lane_id() == 0) base = atomicAdd(&c->slot_count[s0], total);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if ((uint64_t)base + total > P.qcap) {
-      if (lane_id() == 0) set_error(P, kErrQueueOverflow, 12);
-      q.ns = 0;
-      return;
-    }
-    uint32_t pos = base + incl - mine;
-    uint32_t* dst = queue_ptr(P, kQSlot0 + s0);
-    for (uint32_t i = lane_id(); i < q.ns; i += 32)
-      if (q.slotb[2 * i + 1] == s0) dst[pos++] = q.slotb[2 * i];
-    __syncwarp();
-    if (total == q.ns) {   // one slot only (the usual case)
-      q.ns = 0;
-      return;
-    }
-    // compact the entries of other slots to the front, 32 at a time: every
-    // lane reads its entry before any lane writes, and a write position never
-    // passes the chunk being read
-    uint32_t kept = 0;
-    for (uint32_t i0 = 0; i0 < q.ns; i0 += 32) {
-      const uint32_t i = i0 + lane_id();
-      uint32_t ev = 0, es = s0;
-      if (i < q.ns) { ev = q.slotb[2 * i]; es = q.slotb[2 * i + 1]; }
-      const bool keep = es != s0;
-      const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-      __syncwarp();
-      if (keep) {
-        const uint32_t d = kept + __popc(bal & ((1u << lane_id()) - 1u));
-        q.slotb[2 * d] = ev;
-        q.slotb[2 * d + 1] = es;
-      }
-      kept += __popc(bal);
-      __syncwarp();
-    }
-    q.ns = kept;
-    remaining = kept;
-  }
-}
-
+// Publish staged buffers to their queues (warp-collective): those more than
+// half full, or all of them (`force`, at the end of a phase).  The reservations
+// of every buffer, and of every window slot among the staged (vertex, slot)
+// pairs, are one atomic instruction, a lane per counter.  One buffer and one slot
+// after the other cost a round trip each: with long weights a warp's last
+// pushes go to several slots, and phases of a few vertices were mostly that.
 template <int MODE>
 __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, WarpQ& q, bool force) {
+  const uint32_t nn = (force || q.nn > kNearBuf / 2) ? q.nn : 0u;
+  uint32_t nf = 0, nm = 0, ns = 0;
+  if (MODE != kModeBF) {
+    nf = (force || q.nf > kFarBuf / 2) ? q.nf : 0u;
+    nm = (force || q.nm > kMemBuf / 2) ? q.nm : 0u;
+    ns = (force || q.ns > kSlotBuf / 2) ? q.ns : 0u;
+  }
+  if ((nn | nf | nm | ns) == 0) return;
   Control* c = P.ctl;
-  if (q.nn && (force || q.nn > kNearBuf / 2)) {
-    publish(P, &c->near_count[R.push_q & 1], R.push_q, q.nearb, q.nn, 11);
-    q.nn = 0;
+  const uint32_t lane = lane_id();
+  // lanes 0-2: near, far, members; lanes 16 + s: window slot s
+  uint32_t mine = lane == 0 ? nn : lane == 1 ? nf : lane == 2 ? nm : 0u;
+  uint32_t* counter = lane == 0 ? &c->near_count[R.push_q & 1]
+                    : lane == 1 ? &c->far_count[R.far_sel]
+                    : lane == 2 ? &c->members_count
+                                : &c->slot_count[lane & (kRing - 1)];
+  uint32_t* hist = q.histb();
+  if (MODE != kModeBF && ns) {
+    if (lane < (uint32_t)kRing) hist[lane] = 0;
+    __syncwarp();
+    for (uint32_t i = lane; i < ns; i += 32) {   // slot -> (slot, rank within it)
+      const uint32_t s = q.slotb()[2 * i + 1];
+      q.slotb()[2 * i + 1] = s | (atomicAdd(&hist[s], 1u) << 8);
+    }
+    __syncwarp();
+    if (lane >= 16) mine = hist[lane - 16];
   }
-  if (MODE == kModeBF) return;
-  if (q.nf && (force || q.nf > kFarBuf / 2)) {
-    publish(P, &c->far_count[R.far_sel], kQFar0 + R.far_sel, q.farb, q.nf, 13);
-    q.nf = 0;
+  uint32_t base = 0;
+  if (mine) base = atomicAdd(counter, mine);
+  const bool over = (uint64_t)base + mine > P.qcap;
+  if (__any_sync(0xffffffffu, over)) {
+    if (over) set_error(P, kErrQueueOverflow, lane < 3 ? 11 + (lane ? 1 + lane : 0) : 12);
+  } else {
+    if (MODE != kModeBF && ns) {
+      __syncwarp();
+      if (lane >= 16) hist[lane - 16] = base;
+      __syncwarp();
+      for (uint32_t i = lane; i < ns; i += 32) {
+        const uint32_t sr = q.slotb()[2 * i + 1], s = sr & 0xffu;
+        queue_ptr(P, kQSlot0 + s)[hist[s] + (sr >> 8)] = q.slotb()[2 * i];
+      }
+    }
+    const uint32_t bn = __shfl_sync(0xffffffffu, base, 0);
+    for (uint32_t i = lane; i < nn; i += 32) queue_ptr(P, R.push_q)[bn + i] = q.nearb()[i];
+    if (MODE != kModeBF) {
+      const uint32_t bf = __shfl_sync(0xffffffffu, base, 1), bm = __shfl_sync(0xffffffffu, base, 2);
+      for (uint32_t i = lane; i < nf; i += 32) queue_ptr(P, kQFar0 + R.far_sel)[bf + i] = q.farb()[i];
+      for (uint32_t i = lane; i < nm; i += 32) queue_ptr(P, kQMembers)[bm + i] = q.memb()[i];
+    }
   }
-  if (q.nm && (force || q.nm > kMemBuf / 2)) {
-    publish(P, &c->members_count, kQMembers, q.memb, q.nm, 14);
-    q.nm = 0;
-  }
-  if (q.ns && (force || q.ns > kSlotBuf / 2)) publish_slots(P, q);
+  __syncwarp();
+  if (nn) q.nn = 0;
+  if (nf) q.nf = 0;
+  if (nm) q.nm = 0;
+  if (ns) q.ns = 0;
   // (a relax batch adds at most 4 x 32 entries per buffer, so flushing past
   //  half of a 256-entry buffer never overflows it)
 }
@@ -297,10 +253,9 @@ template <class W, int MODE>
 __device__ __forceinline__ void route(const Params& P, const PhaseRec& R, bool improved, uint32_t v,
                                       uint32_t cand, Tally& t) {
   if (!__any_sync(0xffffffffu, improved)) return;
-  Control* c = P.ctl;
   if (MODE == kModeBF) {
     const bool want = improved && atomicExch(&P.pstamp[v], R.stamp) != R.stamp;
-    stage(t.q.nearb, t.q.nn, want, v);
+    stage(t.q.nearb(), t.q.nn, want, v);
     t.pushes += want ? 1 : 0;
     return;
   }
@@ -314,7 +269,7 @@ __device__ __forceinline__ void route(const Params& P, const PhaseRec& R, bool i
   }
   if (__any_sync(0xffffffffu, cls == 1)) {
     const bool want = (cls == 1) && atomicExch(&P.pstamp[v], R.stamp) != R.stamp;
-    stage(t.q.nearb, t.q.nn, want, v);
+    stage(t.q.nearb(), t.q.nn, want, v);
     t.pushes += want ? 1 : 0;
   }
   if (__any_sync(0xffffffffu, cls == 2)) {
@@ -322,8 +277,8 @@ __device__ __forceinline__ void route(const Params& P, const PhaseRec& R, bool i
     const uint32_t bal = __ballot_sync(0xffffffffu, want);
     if (want) {
       const uint32_t pos = t.q.ns + __popc(bal & ((1u << lane_id()) - 1u));
-      t.q.slotb[2 * pos] = v;
-      t.q.slotb[2 * pos + 1] = b - R.win;
+      t.q.slotb()[2 * pos] = v;
+      t.q.slotb()[2 * pos + 1] = b - R.win;
     }
     t.q.ns += __popc(bal);
     t.pushes += want ? 1 : 0;
@@ -335,9 +290,8 @@ __device__ __forceinline__ void route(const Params& P, const PhaseRec& R, bool i
       bmin = b;
       want = atomicExch(&P.farflag[v], 1u) == 0u;
     }
-    bmin = __reduce_min_sync(0xffffffffu, bmin);
-    if (lane_id() == 0 && bmin != 0xFFFFFFFFu) atomicMin(&c->far_min, bmin);
-    stage(t.q.farb, t.q.nf, want, v);
+    t.far_min = min(t.far_min, bmin);
+    stage(t.q.farb(), t.q.nf, want, v);
     t.pushes += want ? 1 : 0;
   }
 }
@@ -354,7 +308,6 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
 #pragma unroll
   for (int q = 0; q < U; ++q) any_imp = any_imp || imp[q];
   if (!__any_sync(0xffffffffu, any_imp)) return;
-  Control* c = P.ctl;
   uint32_t b[U], onear[U], obuck[U];
   int cls[U];   // 0 none, 1 near, 2 window slot, 3 far
 #pragma unroll
@@ -390,7 +343,7 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
     const uint32_t v = ed[q].x;
     if (__any_sync(0xffffffffu, cls[q] == 1)) {
       const bool want = cls[q] == 1 && onear[q] != R.stamp;
-      stage(t.q.nearb, t.q.nn, want, v);
+      stage(t.q.nearb(), t.q.nn, want, v);
       t.pushes += want ? 1 : 0;
     }
     if (MODE != kModeBF) {
@@ -399,8 +352,8 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
         const uint32_t bal = __ballot_sync(0xffffffffu, want);
         if (want) {
           const uint32_t pos = t.q.ns + __popc(bal & ((1u << lane_id()) - 1u));
-          t.q.slotb[2 * pos] = v;
-          t.q.slotb[2 * pos + 1] = b[q] - R.win;
+          t.q.slotb()[2 * pos] = v;
+          t.q.slotb()[2 * pos + 1] = b[q] - R.win;
         }
         t.q.ns += __popc(bal);
         t.pushes += want ? 1 : 0;
@@ -408,9 +361,8 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
       if (__any_sync(0xffffffffu, cls[q] == 3)) {
         const bool lowered = cls[q] == 3 && obuck[q] > b[q];
         const bool want = lowered && ofar[q] == 0u;
-        const uint32_t bmin = __reduce_min_sync(0xffffffffu, lowered ? b[q] : 0xFFFFFFFFu);
-        if (lane_id() == 0 && bmin != 0xFFFFFFFFu) atomicMin(&c->far_min, bmin);
-        stage(t.q.farb, t.q.nf, want, v);
+        if (lowered) t.far_min = min(t.far_min, b[q]);
+        stage(t.q.farb(), t.q.nf, want, v);
         t.pushes += want ? 1 : 0;
       }
     }
@@ -419,7 +371,9 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
 }
 
 // Relax U edge slots per lane: label loads first, then the atomics of every
-// slot (issued before any result is read), then routing.
+// slot (issued before any result is read), then routing.  A phase of a small
+// frontier (R.direct) issues its atomics at once: they are few, and the load that
+// would spare most of them is one more round trip.
 template <class W, bool PRED, int MODE, int U>
 __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, const bool (&act)[U],
                                             const uint32_t (&src)[U], const uint32_t (&dsrc)[U],
@@ -432,7 +386,8 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
 #pragma unroll
   for (int q = 0; q < U; ++q) {
     cand[q] = act[q] ? W::extend(dsrc[q], ed[q].y) : kInfKey;
-    cur[q] = ld_keep_if(cand[q] != kInfKey, lab + ed[q].x, t.keep, L::kInf);
+    
+    cur[q] = ld_keep_if(cand[q] != kInfKey && !R.direct, lab + ed[q].x, t.keep, L::kInf);
   }
 #pragma unroll
   for (int q = 0; q < U; ++q) {
@@ -521,6 +476,7 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
   uint32_t du = kInfKey;
   uint64_t lo = 0, hi = 0, row_end = 0;
   bool valid = false, has_heavy = false;
+  uint32_t member_before = R.hround, heavy = 0;
   if (present) {
     // the row bounds do not depend on the label: both loads go out together
     // (one dependent memory round trip less per item)
@@ -535,43 +491,57 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
   }
   if (MODE == kModeDelta) {
     if (valid) t.min_key = min(t.min_key, du);
+    // settled in this light round: its heavy suffix is relaxed once by the heavy
+    // phase (the answer is read after the rows' edges: finish_members)
     if (members) {
-      // settled in this light round: its heavy suffix is relaxed once by the heavy phase
-      const bool want = valid && has_heavy && atomicExch(&P.hstamp[v], R.hround) != R.hround;
-      if (want) t.heavy += (uint32_t)(row_end - hi);
-      stage(t.q.memb, t.q.nm, want, v);
-      if (t.q.nm > kMemBuf / 2) {
-        publish(P, &c->members_count, kQMembers, t.q.memb, t.q.nm, 14);
-        t.q.nm = 0;
-      }
+      const bool ask = valid && has_heavy;
+      member_before = atom_exch_if(ask, &P.hstamp[v], R.hround, R.hround);
+      if (ask) heavy = (uint32_t)(row_end - hi);
     }
   }
+  auto finish_members = [&] {
+    if (MODE != kModeDelta || !members) return;
+    const bool want = member_before != R.hround;
+    if (want) t.heavy += heavy;
+    if (t.q.nm > kMemBuf - 32) flush_all<MODE>(P, R, t.q, false);
+    stage(t.q.memb(), t.q.nm, want, v);
+  };
   uint32_t deg = valid ? (uint32_t)min(hi - lo, (uint64_t)0xFFFFFFFFull) : 0u;
   // high-degree ranges -> one hub-list entry per 256-edge chunk, written by
   // the whole warp, taken by any warp in the next phase
   const uint32_t hub_deg = R.kind == kPhaseLocal ? 0xFFFFFFFFu : P.hub_degree;
-  uint32_t hubs = __ballot_sync(0xffffffffu, deg >= hub_deg);
-  while (hubs) {
-    const uint32_t hl = __ffs(hubs) - 1;
-    hubs &= hubs - 1;
-    const uint32_t hv = __shfl_sync(0xffffffffu, v, hl);
-    const uint32_t nch = (__shfl_sync(0xffffffffu, deg, hl) + kHubChunk - 1) / kHubChunk;
+  const bool is_hub = deg >= hub_deg;
+  uint32_t hubs = __ballot_sync(0xffffffffu, is_hub);
+  if (hubs) {
+    const uint32_t mine = is_hub ? (deg + kHubChunk - 1) / kHubChunk : 0u;
+    const uint32_t incl = warp_incl_scan(mine);
+    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
     uint32_t hb = 0;
-    if (lane == 0) hb = atomicAdd(&c->hub_count[R.hub_out & 1], nch);
+    if (lane == 0) hb = atomicAdd(&c->hub_count[R.hub_out & 1], all);
     hb = __shfl_sync(0xffffffffu, hb, 0);
-    if ((uint64_t)hb + nch <= P.hub_cap) {
-      HubEntry* H = P.hubs + (size_t)(R.hub_out & 1) * P.hub_cap;
-      for (uint32_t j = lane; j < nch; j += 32)
-        *reinterpret_cast<uint2*>(H + hb + j) = make_uint2(hv, j);
+    if ((uint64_t)hb + all <= P.hub_cap) {
+      HubEntry* H = P.hubs + (size_t)(R.hub_out & 1) * P.hub_cap + hb;
+      do {
+        const uint32_t hl = __ffs(hubs) - 1;
+        hubs &= hubs - 1;
+        const uint32_t hv = __shfl_sync(0xffffffffu, v, hl);
+        const uint32_t nch = __shfl_sync(0xffffffffu, mine, hl);
+        const uint32_t first = __shfl_sync(0xffffffffu, incl, hl) - nch;
+        for (uint32_t j = lane; j < nch; j += 32)
+          *reinterpret_cast<uint2*>(H + first + j) = make_uint2(hv, j);
+      } while (hubs);
     } else if (lane == 0) {
       set_error(P, kErrQueueOverflow, 20);
     }
-    if (lane == hl) deg = 0;
+    if (is_hub) deg = 0;
   }
   // compact the lanes that have edges to relax
   const uint32_t nz = __ballot_sync(0xffffffffu, deg > 0);
   const uint32_t k = __popc(nz);
-  if (k == 0) return;
+  if (k == 0) {
+    finish_members();
+    return;
+  }
   const bool has = lane < k;
   const uint32_t sl = nth_set_bit(nz, has ? lane : 0u);
   const uint32_t cv = __shfl_sync(0xffffffffu, v, sl);
@@ -605,6 +575,7 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
     }
     relax_batch<W, PRED, MODE, kUnroll>(P, R, act, src, dsrc, ed, t);
   }
+  finish_members();
 }
 
 // Append the frontier's vertices among [span * 256, span * 256 + 256) (stamp
@@ -655,7 +626,7 @@ __device__ __forceinline__ void frontier_item(const Params& P, const PhaseRec& R
   const uint32_t base = item * g;
   uint32_t total, limit;
   if (dense) {
-    total = flush ? carry : sweep_span(P, R, item, t.q.listb, carry);
+    total = flush ? carry : sweep_span(P, R, item, t.q.listb(), carry);
     limit = flush ? total : (total & ~31u);
   } else {
     total = min(g, R.fcount - base);
@@ -664,16 +635,16 @@ __device__ __forceinline__ void frontier_item(const Params& P, const PhaseRec& R
   for (uint32_t j0 = 0; j0 < limit; j0 += 32) {
     const bool present = j0 + lane < total;
     uint32_t v = 0;
-    if (present) v = dense ? t.q.listb[j0 + lane] : ldcg(queue_ptr(P, R.fq) + base + lane);
+    if (present) v = dense ? t.q.listb()[j0 + lane] : ldcg(queue_ptr(P, R.fq) + base + lane);
     expand_vertices<W, PRED, MODE>(P, R, v, present, t);
   }
   if (dense) {
     const uint32_t rest = total - limit;   // < 32
     if (limit && rest) {
       __syncwarp();
-      const uint32_t v = lane < rest ? t.q.listb[limit + lane] : 0u;
+      const uint32_t v = lane < rest ? t.q.listb()[limit + lane] : 0u;
       __syncwarp();
-      if (lane < rest) t.q.listb[lane] = v;
+      if (lane < rest) t.q.listb()[lane] = v;
       __syncwarp();
     }
     carry = rest;
@@ -688,31 +659,44 @@ __device__ __forceinline__ void frontier_chunk(const Params& P, const PhaseRec& 
 }
 
 // End of a relaxation phase: this warp's members' heavy edges and smallest
-// expanded label go to its slot in shared memory; flush_block adds the block's
+// expanded label and far bucket go to its slot in shared memory; flush_block adds the block's
 // slots to the control block once, before it arrives at the barrier.  A global
 // addition and minimum per 32-vertex item (100 K on one line in the large
 // phases of RMAT-24, with every item's read of bucket_valid queued behind them)
 // held the solve up: RMAT-24 8.35 -> 6.57 ms, 4096^2 grid 5.53 -> 4.98 ms.
 struct WarpPhase {
+  unsigned long long edges, impr, pushes;   // of the whole solve
   unsigned long long heavy;
   uint32_t min_key;
-  uint32_t pad;
+  uint32_t far_min;
 };
 __device__ __forceinline__ void flush_phase(WarpPhase* slot, Tally& t) {
+  const uint32_t ed = __reduce_add_sync(0xffffffffu, t.edges);
+  const uint32_t im = __reduce_add_sync(0xffffffffu, t.impr);
+  const uint32_t pu = __reduce_add_sync(0xffffffffu, t.pushes);
   const uint32_t mk = __reduce_min_sync(0xffffffffu, t.min_key);
   const uint32_t lo = __reduce_add_sync(0xffffffffu, t.heavy & 0xffffu);
   const uint32_t hi = __reduce_add_sync(0xffffffffu, t.heavy >> 16);
+  const uint32_t fm = __reduce_min_sync(0xffffffffu, t.far_min);
   if (lane_id() == 0) {
+    slot->edges += ed;
+    slot->impr += im;
+    slot->pushes += pu;
     slot->heavy = ((unsigned long long)hi << 16) + lo;
     slot->min_key = mk;
+    slot->far_min = fm;
   }
   t.min_key = 0xFFFFFFFFu;
   t.heavy = 0;
+  t.far_min = 0xFFFFFFFFu;
+  t.edges = t.impr = t.pushes = 0;
 }
 // (warp 0, after a block barrier)
 __device__ __forceinline__ void flush_block(const Params& P, WarpPhase* slots) {
   const uint32_t lane = lane_id();
   const bool in = lane < (uint32_t)kWarpsPerBlock;
+  const uint32_t fm = __reduce_min_sync(0xffffffffu, in ? slots[lane].far_min : 0xFFFFFFFFu);
+  if (lane == 0 && fm != 0xFFFFFFFFu) atomicMin(&P.ctl->far_min, fm);
   const uint32_t mk = __reduce_min_sync(0xffffffffu, in ? slots[lane].min_key : 0xFFFFFFFFu);
   if (mk == 0xFFFFFFFFu) return;   // nothing expanded
   unsigned long long hv = in ? slots[lane].heavy : 0ull;
@@ -728,15 +712,12 @@ __device__ __forceinline__ void flush_block(const Params& P, WarpPhase* slots) {
   }
 }
 
-constexpr uint32_t kHubGrab = B2_HUB_GRAB;   // hub chunks per work item
 
-// A relaxation phase: hub chunks of the previous phase (two per item), then
-// 32-vertex frontier chunks (or 256-vertex sweep items).  Whole rounds of
-// items are dealt round-robin to the warps (no atomics); only the last partial
-// round (fewer items than warps) is handed out from a phase counter.  Handing
-// out a quarter of the items from the counter, so that no warp idles behind a
-// long item, measured 8 % slower on a grid and 2 % on RMAT-24: thousands of
-// warps contend for one counter.
+// A relaxation phase: hub chunks of the previous phase, then
+// 32-vertex frontier chunks (or 256-vertex sweep items), dealt round-robin to
+// the warps, neighbouring items to different blocks.  A phase counter for the
+// last partial round (or for more) costs every warp one atomic on one address
+// per phase: 4096^2 grid 4.42 ms with it, 4.25 without; RMAT-24 the same.
 //
 // Queue items hold g vertices: 32 when the frontier gives every warp at least
 // one full item, else the largest power of two that still does, down to one
@@ -746,34 +727,23 @@ constexpr uint32_t kHubGrab = B2_HUB_GRAB;   // hub chunks per work item
 template <class W, bool PRED, int MODE>
 __device__ void process_phase(const Params& P, const PhaseRec& R, Tally& t) {
   const uint32_t nhub = min(R.hub_in_chunks, P.hub_cap);
-  const uint32_t nhg = (nhub + kHubGrab - 1) / kHubGrab;
   const bool dense = MODE == kModeDelta && R.dense != kDenseOff;
-  const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // neighbouring items go to different blocks: a few items then run on as many SMs
+  const uint32_t gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   uint32_t g = 32;
   if (!dense)
     while (g > 1 && (R.fcount + g - 1) / g < nwarps) g >>= 1;
   const uint32_t nfc = dense ? (P.n + kDenseSpan - 1) / kDenseSpan : (R.fcount + g - 1) / g;
-  const uint32_t items = nhg + nfc;
-  const uint32_t rounds = (items * B2_STATIC_NUM / 4) / nwarps;
-  const uint32_t nstatic = rounds * nwarps;
-  Control* c = P.ctl;
+  const uint32_t items = nhub + nfc;
   uint32_t carry = 0;   // swept vertices waiting in the warp's list
-  for (uint32_t r = 0;; ++r) {
-    uint32_t item = 0;
-    if (r < rounds) {
-      item = r * nwarps + gwarp;
-    } else {
-      if (lane_id() == 0) item = atomicAdd(&c->work_next, 1u);
-      item = __shfl_sync(0xffffffffu, item, 0) + nstatic;
-    }
+  for (uint32_t item = gwarp;; item += nwarps) {
     const bool done = item >= items;
     if (done && carry == 0) break;
-    if (!done && item < nhg) {
-      const uint32_t h1 = min(nhub, (item + 1) * kHubGrab);
-      for (uint32_t h = item * kHubGrab; h < h1; ++h) hub_chunk<W, PRED, MODE>(P, R, h, t);
+    if (!done && item < nhub) {
+      hub_chunk<W, PRED, MODE>(P, R, item, t);
     } else {
-      frontier_item<W, PRED, MODE>(P, R, done ? 0u : item - nhg, dense, done, carry, t, g);
+      frontier_item<W, PRED, MODE>(P, R, done ? 0u : item - nhub, dense, done, carry, t, g);
     }
     if (done) break;
   }
@@ -808,7 +778,7 @@ __device__ void pull_phase(const Params& P, const PhaseRec& R, Tally& t) {
         uint64_t e = __ldg(&P.in_rowptr[v]) + __ldg(&P.in_lightcnt[v]);
         const uint64_t e1 = __ldg(&P.in_rowptr[v + 1]);
         typename L::T best = cw;
-        unsigned long long scanned = 0;
+        uint32_t scanned = 0;
         for (; e < e1; ++e) {
           const uint2 ed = __ldg(&P.in_edges[e]);
           const uint32_t bound = W::extend(lb, ed.y);   // no member reaches v for less via this or later edges
@@ -857,7 +827,7 @@ __device__ __forceinline__ void trace_phase(const Params& P, const PhaseRec& r, 
 }
 
 template <bool PRED, int MODE>
-__device__ void manager_init(const Params& P) {
+__device__ void manager_init(const Params& P, PhaseRec& r) {
   using L = Label<PRED>;
   Control* c = P.ctl;
   typename L::T* lab = (typename L::T*)P.dist;
@@ -872,7 +842,6 @@ __device__ void manager_init(const Params& P) {
   c->far_min = 0xFFFFFFFFu;
   c->far_min_next = 0xFFFFFFFFu;
   c->t_start = globaltimer_ns();
-  PhaseRec r;
   memset(&r, 0, sizeof(r));
   r.kind = kPhaseProcess;
   r.phase = 1;
@@ -891,18 +860,14 @@ __device__ void manager_init(const Params& P) {
   r.dbase_b = 0;
   c->cur_min_key = 0xFFFFFFFFu;
   c->member_heavy = 0;
-  store_rec(c, r);
 }
 
 // Whole-solve budget: a phase sequence that outlives it ends the kernel with
 // kErrTimeout instead of looping.
-__device__ __forceinline__ bool over_budget(const Params& P, PhaseRec& nx) {
-  Control* c = P.ctl;
-  if (globaltimer_ns() - c->t_start > P.budget_ns || nx.phase > 0x7fffffffu) {
-    atomicCAS(&c->error, kErrNone, (uint32_t)kErrTimeout);
-    c->error_site = 2;
+__device__ __forceinline__ bool over_budget(const Params& P, unsigned long long t_start, PhaseRec& nx) {
+  if (globaltimer_ns() - t_start > P.budget_ns || nx.phase > 0x7fffffffu) {
+    set_error(P, kErrTimeout, 2);
     nx.kind = kPhaseDone;
-    store_rec(c, nx);
     return true;
   }
   return false;
@@ -926,74 +891,71 @@ __device__ __forceinline__ void consume_process_counters(Control* c, const Phase
 // round (python reference: one extra relaxation after max_iters,
 // minplus_bellman_ford.py:92-99).  At FINAL, aux = 1 means "output the
 // committed round".
-__device__ void manager_bf(const Params& P) {
+__device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, PhaseRec& nx) {
   Control* c = P.ctl;
-  const PhaseRec r = load_rec(c);
+  // every word the step may need, loaded at once (one round trip)
+  const uint32_t phases = vld(&c->phases), stamp_ctr = vld(&c->stamp_ctr);
+  const uint32_t hub_out = vld(&c->hub_count[r.hub_out & 1]), near = vld(&c->near_count[r.push_q & 1]);
+  const unsigned long long t_start = vld64(&c->t_start);
   trace_phase(P, r, r.iter);
-  PhaseRec nx = r;
+  nx = r;
   nx.phase = r.phase + 1;
-  c->phases = vld(&c->phases) + 1;
-  if (r.kind == kPhaseFinal) { nx.kind = kPhaseDone; store_rec(c, nx); return; }
-  if (over_budget(P, nx)) return;
+  c->phases = phases + 1;
+  if (r.kind == kPhaseFinal) { nx.kind = kPhaseDone; return; }
+  if (over_budget(P, t_start, nx)) return;
   if (r.kind == kPhaseCommit) {
     nx.kind = kPhaseProcess;
     nx.fq = r.fq;
     nx.fcount = r.fcount;
     nx.push_q = r.fq ^ 1u;
-    nx.stamp = P.phase_base + (c->stamp_ctr++);
+    nx.stamp = P.phase_base + stamp_ctr;
+    c->stamp_ctr = stamp_ctr + 1;
     nx.hub_in = r.hub_out ^ 1u;
     nx.hub_in_count = 0;
     nx.hub_in_chunks = 0;
     nx.iter = r.iter + 1;
     nx.aux = (r.aux == 2u) ? 1u : 0u;
-    store_rec(c, nx);
     return;
   }
   consume_process_counters(c, r);
-  const uint32_t hch = vld(&c->hub_count[r.hub_out & 1]);
-  const uint32_t hcnt = hch;
+  const uint32_t hch = hub_out;
   if (hch > 0) {   // hub chunks of this round: same round, same push queue and stamp
     nx.kind = kPhaseProcess;
     nx.fq = kQNone;
     nx.fcount = 0;
     nx.hub_in = r.hub_out;
-    nx.hub_in_count = hcnt;
+    nx.hub_in_count = hch;
     nx.hub_in_chunks = hch;
     nx.hub_out = r.hub_out ^ 1u;
-    store_rec(c, nx);
     return;
   }
-  const uint32_t nn = vld(&c->near_count[r.push_q & 1]);
+  const uint32_t nn = near;
   const bool changed = nn > 0;
   nx.hub_in_chunks = 0;
   nx.hub_in_count = 0;
   if (r.aux == 1u) {
     c->negative_cycle = changed ? 1u : 0u;
     nx.kind = kPhaseFinal;   // aux stays 1: output the committed round
-    store_rec(c, nx);
     return;
   }
   c->iterations = r.iter;
-  publish_progress(P.board, r.iter, changed ? 1u : 0u, globaltimer_ns() - c->t_start);
+  publish_progress(P.board, r.iter, changed ? 1u : 0u, globaltimer_ns() - t_start);
   if (!changed) {
     c->converged = 1;
     c->first_unchanged = r.iter;
     nx.kind = kPhaseFinal;
     nx.aux = 0u;
-    store_rec(c, nx);
     return;
   }
   if (r.iter >= P.max_iters && !P.detect_negcycle) {
     nx.kind = kPhaseFinal;
     nx.aux = 0u;
-    store_rec(c, nx);
     return;
   }
   nx.kind = kPhaseCommit;
   nx.fq = r.push_q;
   nx.fcount = nn;
   nx.aux = (r.iter >= P.max_iters) ? 2u : 0u;
-  store_rec(c, nx);
 }
 
 // A large near or slot frontier is found by a stamp sweep (see sweep_span).
@@ -1009,9 +971,9 @@ __device__ __forceinline__ void set_dense(const Params& P, PhaseRec& nx, uint32_
 // trip instead of one per decision.
 struct MgrSnap {
   uint32_t phases, probe_valid, local_q, local_total, local_iters, fusion_off, members, bucket_valid;
-  uint32_t iterations, heavy_pulls, far_min, far_min_next;
+  uint32_t iterations, heavy_pulls, far_min, far_min_next, stamp_ctr;
   uint32_t hub[2], near[2], far[2], slot[kRing];
-  unsigned long long member_heavy;
+  unsigned long long member_heavy, t_start;
 };
 __device__ __forceinline__ MgrSnap snapshot(const Control* c) {
   MgrSnap m;
@@ -1035,27 +997,28 @@ __device__ __forceinline__ MgrSnap snapshot(const Control* c) {
   }
 #pragma unroll
   for (int s = 0; s < kRing; ++s) m.slot[s] = vld(&c->slot_count[s]);
+  m.stamp_ctr = vld(&c->stamp_ctr);
   m.member_heavy = vld64(&c->member_heavy);
+  m.t_start = vld64(&c->t_start);
   return m;
 }
 
-__device__ void manager_delta(const Params& P) {
+__device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, PhaseRec& nx) {
   Control* c = P.ctl;
-  const PhaseRec r = load_rec(c);
   MgrSnap m = snapshot(c);
   trace_phase(P, r, r.cur);
-  PhaseRec nx = r;
+  nx = r;
   nx.dense = kDenseOff;
   nx.fstamp = 0u;
   nx.phase = r.phase + 1;
-  nx.stamp = P.phase_base + (c->stamp_ctr++);
+  nx.stamp = P.phase_base + m.stamp_ctr;
+  c->stamp_ctr = m.stamp_ctr + 1;
   c->phases = m.phases + 1;
-  if (r.kind == kPhaseFinal) { nx.kind = kPhaseDone; store_rec(c, nx); return; }
-  if (over_budget(P, nx)) return;
+  if (r.kind == kPhaseFinal) { nx.kind = kPhaseDone; return; }
+  if (over_budget(P, m.t_start, nx)) return;
   if (r.kind == kPhaseProbe) {
     c->converged = m.probe_valid ? 0u : 1u;
     nx.kind = kPhaseFinal;
-    store_rec(c, nx);
     return;
   }
   uint32_t win = r.win;
@@ -1097,7 +1060,6 @@ __device__ void manager_delta(const Params& P) {
         nx.fq = kQNone;
         nx.fcount = 0;
         nx.stamp = r.stamp;
-        store_rec(c, nx);
         return;
       }
       if (nn > 0) {              // a heavy relaxation landed in this bucket: new light round
@@ -1108,7 +1070,6 @@ __device__ void manager_delta(const Params& P) {
         nx.push_q = r.push_q ^ 1u;
         nx.hround = P.phase_base + nx.phase;
         set_dense(P, nx, kDenseNear, r.stamp);
-        store_rec(c, nx);
         return;
       }
     } else {
@@ -1120,7 +1081,6 @@ __device__ void manager_delta(const Params& P) {
         if (hch == 0 && nn <= P.fusion && !m.fusion_off) nx.kind = kPhaseLocal;
         // (a LOCAL phase's last pushes carry a stamp drawn inside it: no sweep after one)
         if (nn > 0 && r.kind != kPhaseLocal) set_dense(P, nx, kDenseNear, r.stamp);
-        store_rec(c, nx);
         return;
       }
       const uint32_t mc = m.members;
@@ -1141,7 +1101,6 @@ __device__ void manager_delta(const Params& P) {
           nx.fq = kQMembers;
           nx.fcount = mc;
         }
-        store_rec(c, nx);
         return;
       }
     }
@@ -1154,13 +1113,12 @@ __device__ void manager_delta(const Params& P) {
       c->bucket_valid = 0;
       // the previous bucket had a successor (the reference's `changed`,
       // delta_stepping_hip_CSR.cpp:744-756); the last one is reported at the end
-      if (m.iterations > 1) publish_progress(P.board, m.iterations - 1, 1u, globaltimer_ns() - c->t_start);
+      if (m.iterations > 1) publish_progress(P.board, m.iterations - 1, 1u, globaltimer_ns() - m.t_start);
     }
     if (m.iterations >= P.max_iters) {
       nx.kind = kPhaseProbe;
       nx.heavy = 0;
       nx.hub_in_chunks = 0;
-      store_rec(c, nx);
       return;
     }
     from_slot = r.cur - r.win + 1;
@@ -1186,7 +1144,6 @@ __device__ void manager_delta(const Params& P) {
     nx.push_q = kQNear0;   // both near queues are empty at a bucket boundary
     if (nx.fcount <= P.fusion && !m.fusion_off) nx.kind = kPhaseLocal;
     set_dense(P, nx, kDenseSlot, nx.cur);
-    store_rec(c, nx);
     return;
   }
   const uint32_t fc = m.far[far_sel];
@@ -1202,12 +1159,10 @@ __device__ void manager_delta(const Params& P) {
     nx.win = nwin;
     nx.cur = nwin;
     c->far_min_next = 0xFFFFFFFFu;
-    store_rec(c, nx);
     return;
   }
   c->converged = 1;
   nx.kind = kPhaseFinal;
-  store_rec(c, nx);
 }
 
 // Bucket fusion: block 0 alone runs consecutive light sub-phases of one
@@ -1234,12 +1189,12 @@ __device__ void local_phase(const Params& P, const PhaseRec& R0, Tally& t) {
   if (threadIdx.x == 0) s_edges = 0;
   __syncthreads();
   for (uint32_t iter = 0;; ++iter) {
-    const unsigned long long e0 = t.edges;
+    const uint32_t e0 = t.edges;
     const uint32_t nfc = (L.fcount + 31) / 32;
     for (uint32_t ch = w; ch < nfc; ch += nw) frontier_chunk<W, PRED, MODE>(P, L, ch * 32, t);
     flush_all<MODE>(P, L, t.q, true);
     {
-      unsigned long long de = t.edges - e0;
+      unsigned long long de = (uint32_t)(t.edges - e0);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) de += __shfl_down_sync(0xffffffffu, de, o);
       if ((threadIdx.x & 31u) == 0 && de) atomicAdd(&s_edges, de);
@@ -1275,23 +1230,108 @@ __device__ void local_phase(const Params& P, const PhaseRec& R0, Tally& t) {
   }
 }
 
+// Frontier entries relaxed without the filter load (411 x 300 grid 0.783 -> 0.773
+// ms; 256, 1024 and 8192 measure alike there, and on the large graphs).
+constexpr uint32_t kDirectMax = 1024;
+
+// Grid barrier between phases.  The last block to arrive runs the manager step
+// on one thread while all others wait, and releases them by writing the next
+// phase's record, tagged with the barrier's number, to ctl->box.  A waiting
+// block polls the record itself, one lane per word, so release and record are
+// one L2 round trip; arrivals count up and are never reset, and errors travel in
+// the record (kPhaseDone).  With a generation word, a record and an error word
+// read one after the other a phase of a one-vertex frontier took 11 us (296
+// blocks), five dependent round trips of it here.  Every wait is bounded by the
+// solve budget; whoever gives up sets the error word, which all waits poll.
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+template <typename Manager>
+__device__ __forceinline__ void next_phase(const Params& P, PhaseRec* s_rec, WarpPhase* slots, bool expanded,
+                                           uint32_t& barrier, Manager&& manager) {
+  Control* c = P.ctl;
+  __syncthreads();   // every warp is done with the phase and its record
+  ++barrier;
+  if (threadIdx.x < 32) {
+    const uint32_t lane = threadIdx.x;
+    if (expanded) flush_block(P, slots);
+    bool last = false;
+    if (lane == 0) {
+      uint32_t arrived;
+      asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(&c->bar_arrive) : "memory");
+      last = arrived == gridDim.x * barrier - 1u;
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    volatile uint32_t* rec = reinterpret_cast<volatile uint32_t*>(s_rec);
+    if (last) {
+      if (lane == 0) {
+        const uint32_t err = vld(&c->error);
+        const PhaseRec r = *s_rec;
+        PhaseRec nx;
+        manager(r, nx);
+        if (err != kErrNone) nx.kind = kPhaseDone;
+        nx.fcount = min(nx.fcount, P.qcap);
+        nx.direct = nx.kind == kPhaseProcess && nx.fcount <= kDirectMax && nx.hub_in_chunks == 0 &&
+                    nx.dense == kDenseOff;
+        *s_rec = nx;
+      }
+      __syncwarp();
+      fence_acq_rel();
+      if (lane < (uint32_t)kRecWords) {
+        const uint32_t w = rec[lane];
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(c->box + lane),
+                     "l"(((unsigned long long)barrier << 32) | w) : "memory");
+        if (s_rec->kind == kPhaseDone) reinterpret_cast<uint32_t*>(&c->rec)[lane] = w;
+      }
+    } else {
+      unsigned long long w = 0;
+      uint64_t t0 = 0;
+      bool gave_up = false;
+      for (uint32_t spins = 1;; ++spins) {
+        bool have = true;
+        if (lane < (uint32_t)kRecWords) {
+          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(c->box + lane) : "memory");
+          have = (uint32_t)(w >> 32) == barrier;
+        }
+        if (__all_sync(0xffffffffu, have)) break;
+        if ((spins & 63u) == 0) {
+          uint32_t stop = 0;
+          if (lane == 0) {
+            const uint64_t now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            stop = ld_relaxed_u32(&c->error) != kErrNone;
+            if (!stop && now - t0 > P.budget_ns) {
+              set_error(P, kErrTimeout, 1);
+              stop = 1;
+            }
+          }
+          if (__shfl_sync(0xffffffffu, stop, 0)) {
+            gave_up = true;
+            break;
+          }
+        }
+        __nanosleep(20);
+      }
+      fence_acq_rel();
+      if (gave_up) {
+        if (lane == 0) s_rec->kind = kPhaseDone;
+      } else if (lane < (uint32_t)kRecWords) {
+        rec[lane] = (uint32_t)w;
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // ---------------------------------------------------------------------------
 template <class W, bool PRED, int MODE>
-__global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(Params P) {
+__global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_constant__ Params P) {
   using L = Label<PRED>;
   __shared__ PhaseRec s_rec;
   __shared__ WarpPhase s_phase[kWarpsPerBlock];
   extern __shared__ uint32_t s_stage[];   // kStageWords per warp
   Tally t;
   t.keep = l2_keep_policy();
-  {
-    uint32_t* wb = s_stage + (threadIdx.x >> 5) * kStageWords;
-    t.q.nearb = wb;
-    t.q.farb = wb + kNearBuf;
-    t.q.slotb = wb + kNearBuf + kFarBuf;
-    t.q.memb = wb + kNearBuf + kFarBuf + 2 * kSlotBuf;
-    t.q.listb = t.q.memb + kMemBuf;
-  }
+  t.q.buf = s_stage + (threadIdx.x >> 5) * kStageWords;
+  if (threadIdx.x < (uint32_t)kWarpsPerBlock) s_phase[threadIdx.x] = WarpPhase{0, 0, 0, 0, 0xFFFFFFFFu, 0xFFFFFFFFu};
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   Control* c = P.ctl;
@@ -1305,14 +1345,14 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(Params P) {
       P.farflag[v] = 0u;
     }
   }
-  bool ok = grid_barrier((GridBarrier*)c, gridDim.x, P.budget_ns, [&] { manager_init<PRED, MODE>(P); });
-  while (ok) {
-    if (threadIdx.x == 0) s_rec = load_rec(c);
-    __syncthreads();
-    PhaseRec R = s_rec;
+  uint32_t barrier = 0;
+  next_phase(P, &s_rec, s_phase, false, barrier,
+             [&](const PhaseRec&, PhaseRec& nx) { manager_init<PRED, MODE>(P, nx); });
+  for (;;) {
+    const PhaseRec R = s_rec;
     if (R.kind == kPhaseDone) break;
-    R.fcount = min(R.fcount, P.qcap);
-    const bool expands = R.kind == kPhaseProcess || (R.kind == kPhaseLocal && blockIdx.x == 0);
+    const bool expands =
+        R.kind == kPhaseProcess || R.kind == kPhasePull || (R.kind == kPhaseLocal && blockIdx.x == 0);
     if (R.kind == kPhaseProcess) {
       process_phase<W, PRED, MODE>(P, R, t);
     } else if (R.kind == kPhaseLocal) {
@@ -1406,29 +1446,18 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(Params P) {
         }
       }
     }
-    if (MODE == kModeDelta && expands) {
-      flush_phase(s_phase + (threadIdx.x >> 5), t);
-      __syncthreads();
-      if (threadIdx.x < 32) flush_block(P, s_phase);
-    }
-    if (MODE == kModeBF) {
-      ok = grid_barrier((GridBarrier*)c, gridDim.x, P.budget_ns, [&] { c->work_next = 0; manager_bf(P); });
-    } else {
-      ok = grid_barrier((GridBarrier*)c, gridDim.x, P.budget_ns, [&] { c->work_next = 0; manager_delta(P); });
-    }
+    if (expands) flush_phase(s_phase + (threadIdx.x >> 5), t);
+    next_phase(P, &s_rec, s_phase, MODE == kModeDelta && expands, barrier, [&](const PhaseRec& r, PhaseRec& nx) {
+      if (MODE == kModeBF) manager_bf(P, r, nx);
+      else manager_delta(P, r, nx);
+    });
   }
-  // flush tallies (one atomic per warp)
-  unsigned long long e = t.edges, im = t.impr, pu = t.pushes;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    e += __shfl_down_sync(0xffffffffu, e, o);
-    im += __shfl_down_sync(0xffffffffu, im, o);
-    pu += __shfl_down_sync(0xffffffffu, pu, o);
-  }
-  if (lane_id() == 0) {
-    if (e) atomicAdd(&c->edges, e);
-    if (im) atomicAdd(&c->improvements, im);
-    if (pu) atomicAdd(&c->pushes, pu);
+  // totals of the solve (the last phase ended with a block barrier)
+  if (threadIdx.x < (uint32_t)kWarpsPerBlock) {
+    const WarpPhase& w = s_phase[threadIdx.x];
+    if (w.edges) atomicAdd(&c->edges, w.edges);
+    if (w.impr) atomicAdd(&c->improvements, w.impr);
+    if (w.pushes) atomicAdd(&c->pushes, w.pushes);
   }
 }
 
@@ -1776,7 +1805,7 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
   if (e != cudaSuccess) return from_cuda(e);
   const Control& hc = *w.h_ctl;
   if (P.board) progress_finish(g, o, prog_max, hc.iterations, hc.converged ? 0 : 1, &reported);
-  w.phase_epoch += std::max(hc.rec.phase, hc.stamp_ctr) + 2;
+  w.phase_epoch += std::max(std::max(hc.rec.phase, hc.phases), hc.stamp_ctr) + 2;
   w.trace_n = o.trace ? hc.trace_n : 0;
   b2_status ds = map_device_error(hc.error);
   if (stats) {
