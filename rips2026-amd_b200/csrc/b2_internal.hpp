@@ -63,7 +63,7 @@ struct PhaseRec {
   uint32_t iter;        // BF iteration being executed
   uint32_t heavy;       // 1: relax the heavy suffix (w > delta) of each frontier vertex
   uint32_t hround;      // stamp of the current heavy round (members dedup)
-  uint32_t aux;         // BF: round role (0 normal, 2 commit-before-probe, 1 probe); FINAL: source buffer
+  uint32_t aux;         // BF: 1 for the negative-cycle probe round (FINAL: output the labels it read)
   uint32_t dq;          // bucket width (uint32 graphs)
   uint32_t dinv;        // float bits of 1/width (float graphs)
   uint32_t dbase;       // distance key at which bucket dbase_b starts (0 until re-based)
@@ -88,7 +88,6 @@ static_assert(kRecWords <= 32, "one lane polls each word of the record");
 enum PhaseKind : uint32_t {
   kPhaseInit = 0,
   kPhaseProcess = 1,   // relax a frontier (+ hub chunks of the previous phase)
-  kPhaseCommit = 2,    // BF: dist_cur[v] = dist_next[v] for v in frontier
   kPhaseSplit = 3,     // delta: move far-pile entries into the new window
   kPhaseProbe = 4,     // delta: count valid pending entries (max_iters cut)
   kPhaseFinal = 5,     // write outputs

@@ -21,6 +21,19 @@
 // L2 load (filter) plus one hardware atomicMin on the 32-bit key or the
 // packed 64-bit key|pred word; pushes are warp-aggregated.
 //
+// Bellman-Ford rounds (Jacobi: round k's sources and comparisons use the labels
+// after round k - 1) keep two label arrays and swap their roles each round.
+// Round k reads array A, whose labels nobody lowers, and takes minima into B,
+// which still holds the labels after round k - 2: the frontier (the vertices that
+// changed in round k - 1) carries its labels over from A as it expands, and every
+// other vertex's label is the same in both.  A candidate below A's label improves
+// the vertex, and the one whose atomic finds B not yet below A's label is the
+// first to do so and pushes it, so no stamps and no commit phase are needed.  The
+// chunks of high-degree vertices are listed when those are pushed and run beside
+// the frontier of their round.  With a commit phase, and hub chunks in a phase of
+// their own, a round took three grid barriers: RMAT-17 with predecessors 0.58 ->
+// 0.36 ms, ER-4096 0.28 -> 0.19 ms.
+//
 // Delta-stepping (replaces the reference's host-driven current / pending /
 // heavy queues, delta_stepping_hip_CSR.cpp:367-529):
 //   * adjacency lists are sorted by weight when the graph is built, so the
@@ -75,8 +88,8 @@ struct Params {
   const uint64_t* __restrict__ rowptr;
   const uint2* __restrict__ edges;
   const uint32_t* __restrict__ lightcnt;   // null: relax whole rows in every sub-phase
-  void* dist;        // labels receiving atomicMin (BF: round k+1 values)
-  void* dist_cur;    // BF: labels of round k (read side)
+  void* dist;        // labels receiving atomicMin
+  void* dist_cur;    // BF: the second label array (see bf_read / bf_write)
   uint32_t* pstamp;
   uint32_t* bstamp;
   uint32_t* farflag;
@@ -103,6 +116,7 @@ struct Params {
   const uint32_t* __restrict__ in_lightcnt; // light prefix of each incoming row
   float pull_factor;      // pull when the members' heavy out-edges exceed pull_factor x n
   uint32_t is_float;
+  uint32_t has_hubs;      // some row has hub_degree edges or more
   uint32_t fusion;        // light frontiers up to this size run as a LOCAL phase (0: off)
   uint32_t dense_min;     // delta: near / slot frontiers of at least this many entries are swept
   uint32_t qcap;          // entries each worklist queue may hold (<= n; a push past it is kErrQueueOverflow)
@@ -132,6 +146,14 @@ __device__ __forceinline__ uint32_t bucket_of(const PhaseRec& R, uint32_t key) {
 
 __device__ __forceinline__ uint32_t* queue_ptr(const Params& P, uint32_t id) {
   return P.queues + (size_t)id * P.n;
+}
+
+// BF round R.iter: the array it reads and the one it lowers.
+__device__ __forceinline__ void* bf_read(const Params& P, const PhaseRec& R) {
+  return (R.iter & 1u) ? P.dist_cur : P.dist;
+}
+__device__ __forceinline__ void* bf_write(const Params& P, const PhaseRec& R) {
+  return (R.iter & 1u) ? P.dist : P.dist_cur;
 }
 
 __device__ __forceinline__ void set_error(const Params& P, uint32_t code, uint32_t site) {
@@ -177,6 +199,33 @@ __device__ __forceinline__ void stage(uint32_t* buf, uint32_t& cnt, bool want, u
   const uint32_t b = __ballot_sync(0xffffffffu, want);
   if (want) buf[cnt + __popc(b & ((1u << lane_id()) - 1u))] = v;
   cnt += __popc(b);
+}
+
+// List the 256-edge chunks of the high-degree vertices among the lanes, with one
+// reservation (warp-collective).
+__device__ __forceinline__ void append_hubs(const Params& P, const PhaseRec& R, uint32_t v, uint32_t deg, bool is_hub) {
+  uint32_t hubs = __ballot_sync(0xffffffffu, is_hub);
+  if (!hubs) return;
+  const uint32_t lane = lane_id();
+  const uint32_t mine = is_hub ? (deg + kHubChunk - 1) / kHubChunk : 0u;
+  const uint32_t incl = warp_incl_scan(mine);
+  const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+  uint32_t hb = 0;
+  if (lane == 0) hb = atomicAdd(&P.ctl->hub_count[R.hub_out & 1], all);
+  hb = __shfl_sync(0xffffffffu, hb, 0);
+  if ((uint64_t)hb + all > P.hub_cap) {
+    if (lane == 0) set_error(P, kErrQueueOverflow, 20);
+    return;
+  }
+  HubEntry* H = P.hubs + (size_t)(R.hub_out & 1) * P.hub_cap + hb;
+  do {
+    const uint32_t hl = __ffs(hubs) - 1;
+    hubs &= hubs - 1;
+    const uint32_t hv = __shfl_sync(0xffffffffu, v, hl);
+    const uint32_t nch = __shfl_sync(0xffffffffu, mine, hl);
+    const uint32_t first = __shfl_sync(0xffffffffu, incl, hl) - nch;
+    for (uint32_t j = lane; j < nch; j += 32) *reinterpret_cast<uint2*>(H + first + j) = make_uint2(hv, j);
+  } while (hubs);
 }
 
 // Publish staged buffers to their queues (warp-collective): those more than
@@ -231,6 +280,15 @@ __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, Wa
     }
     const uint32_t bn = __shfl_sync(0xffffffffu, base, 0);
     for (uint32_t i = lane; i < nn; i += 32) queue_ptr(P, R.push_q)[bn + i] = q.nearb()[i];
+    if (MODE == kModeBF && P.has_hubs) {
+      for (uint32_t i0 = 0; i0 < nn; i0 += 32) {
+        const bool in = i0 + lane < nn;
+        const uint32_t v = in ? q.nearb()[i0 + lane] : 0u;
+        const uint32_t deg =
+            in ? (uint32_t)min(__ldg(&P.rowptr[v + 1]) - __ldg(&P.rowptr[v]), (uint64_t)0xFFFFFFFFull) : 0u;
+        append_hubs(P, R, v, deg, deg >= P.hub_degree);
+      }
+    }
     if (MODE != kModeBF) {
       const uint32_t bf = __shfl_sync(0xffffffffu, base, 1), bm = __shfl_sync(0xffffffffu, base, 2);
       for (uint32_t i = lane; i < nf; i += 32) queue_ptr(P, kQFar0 + R.far_sel)[bf + i] = q.farb()[i];
@@ -253,12 +311,6 @@ template <class W, int MODE>
 __device__ __forceinline__ void route(const Params& P, const PhaseRec& R, bool improved, uint32_t v,
                                       uint32_t cand, Tally& t) {
   if (!__any_sync(0xffffffffu, improved)) return;
-  if (MODE == kModeBF) {
-    const bool want = improved && atomicExch(&P.pstamp[v], R.stamp) != R.stamp;
-    stage(t.q.nearb(), t.q.nn, want, v);
-    t.pushes += want ? 1 : 0;
-    return;
-  }
   uint32_t b = 0;
   int cls = 0;  // 1 near, 2 window slot, 3 far
   if (improved) {
@@ -315,26 +367,22 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
     b[q] = 0;
     cls[q] = 0;
     if (imp[q]) {
-      if (MODE == kModeBF) {
-        cls[q] = 1;
-      } else {
-        b[q] = bucket_of<W>(R, cand[q]);
-        cls[q] = b[q] <= R.cur ? 1 : (b[q] < R.win + (uint32_t)kRing ? 2 : 3);
-      }
+      b[q] = bucket_of<W>(R, cand[q]);
+      cls[q] = b[q] <= R.cur ? 1 : (b[q] < R.win + (uint32_t)kRing ? 2 : 3);
     }
     // defaults read as "already queued"
     onear[q] = atom_exch_if(cls[q] == 1, &P.pstamp[ed[q].x], R.stamp, R.stamp);
-    obuck[q] = MODE == kModeBF ? 0u : atom_min_if(cls[q] >= 2, &P.bstamp[ed[q].x], b[q], 0u);
+    obuck[q] = atom_min_if(cls[q] >= 2, &P.bstamp[ed[q].x], b[q], 0u);
   }
   uint32_t ofar[U];
   bool any_far = false;
 #pragma unroll
   for (int q = 0; q < U; ++q) {
-    const bool f = MODE != kModeBF && cls[q] == 3 && obuck[q] > b[q];
+    const bool f = cls[q] == 3 && obuck[q] > b[q];
     any_far = any_far || f;
     ofar[q] = f ? 0u : 1u;
   }
-  if (MODE != kModeBF && any_far) {
+  if (any_far) {
 #pragma unroll
     for (int q = 0; q < U; ++q) ofar[q] = atom_exch_if(ofar[q] == 0u, &P.farflag[ed[q].x], 1u, 1u);
   }
@@ -379,10 +427,40 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
                                             const uint32_t (&src)[U], const uint32_t (&dsrc)[U],
                                             const uint2 (&ed)[U], Tally& t) {
   using L = Label<PRED>;
-  typename L::T* lab = (typename L::T*)P.dist;
   uint32_t cand[U];
   typename L::T cur[U], old[U];
   bool imp[U];
+  if (MODE == kModeBF) {
+    typename L::T* rd = (typename L::T*)bf_read(P, R);
+    typename L::T* wr = (typename L::T*)bf_write(P, R);
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      cand[q] = act[q] ? W::extend(dsrc[q], ed[q].y) : kInfKey;
+      cur[q] = ld_keep_if(cand[q] != kInfKey, rd + ed[q].x, t.keep, (typename L::T)0);
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const typename L::T cw = L::make(cand[q], src[q]);
+      old[q] = atom_min_keep_if(cand[q] < L::key(cur[q]), wr + ed[q].x, cw, t.keep, (typename L::T)0);
+      if (PRED && cand[q] == L::key(cur[q]) && cw < cur[q]) {
+        // a smaller predecessor at an equal distance: the vertex is not expanded
+        // again, so both arrays take it
+        atomicMin(rd + ed[q].x, cw);
+        atomicMin(wr + ed[q].x, cw);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      imp[q] = cand[q] < L::key(cur[q]) && L::key(old[q]) >= L::key(cur[q]);   // first below the read label
+      t.edges += act[q] ? 1 : 0;
+      t.impr += imp[q] ? 1 : 0;
+      t.pushes += imp[q] ? 1 : 0;
+      stage(t.q.nearb(), t.q.nn, imp[q], ed[q].x);
+    }
+    flush_all<MODE>(P, R, t.q, false);
+    return;
+  }
+  typename L::T* lab = (typename L::T*)P.dist;
 #pragma unroll
   for (int q = 0; q < U; ++q) {
     cand[q] = act[q] ? W::extend(dsrc[q], ed[q].y) : kInfKey;
@@ -407,9 +485,9 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
 }
 
 template <class W, bool PRED, int MODE>
-__device__ __forceinline__ uint32_t src_key(const Params& P, uint32_t v) {
+__device__ __forceinline__ uint32_t src_key(const Params& P, const PhaseRec& R, uint32_t v) {
   using L = Label<PRED>;
-  const typename L::T* lab = (const typename L::T*)(MODE == kModeBF ? P.dist_cur : P.dist);
+  const typename L::T* lab = (const typename L::T*)(MODE == kModeBF ? bf_read(P, R) : P.dist);
   return L::key(ldcg(lab + v));
 }
 
@@ -442,7 +520,7 @@ __device__ __forceinline__ void hub_chunk(const Params& P, const PhaseRec& R, ui
   uint64_t rlo, rhi;
   bool hh;
   phase_range(P, R, v, rlo, rhi, hh);   // issued with the label load
-  const uint32_t du = src_key<W, PRED, MODE>(P, v);
+  const uint32_t du = src_key<W, PRED, MODE>(P, R, v);
   bool valid = du != kInfKey;
   if (MODE == kModeDelta) valid = valid && bucket_of<W>(R, du) == R.cur;
   if (!valid) return;
@@ -471,7 +549,6 @@ template <class W, bool PRED, int MODE>
 __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec& R, uint32_t v, bool present,
                                                 Tally& t) {
   const uint32_t lane = lane_id();
-  Control* c = P.ctl;
   const bool members = MODE == kModeDelta && P.lightcnt && !R.heavy;
   uint32_t du = kInfKey;
   uint64_t lo = 0, hi = 0, row_end = 0;
@@ -481,7 +558,13 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
     // the row bounds do not depend on the label: both loads go out together
     // (one dependent memory round trip less per item)
     phase_range(P, R, v, lo, hi, has_heavy, &row_end);
-    du = src_key<W, PRED, MODE>(P, v);
+    if (MODE == kModeBF) {   // carry the label over
+      const typename Label<PRED>::T w = ldcg((const typename Label<PRED>::T*)bf_read(P, R) + v);
+      atomicMin((typename Label<PRED>::T*)bf_write(P, R) + v, w);
+      du = Label<PRED>::key(w);
+    } else {
+      du = src_key<W, PRED, MODE>(P, R, v);
+    }
     valid = du != kInfKey;
     if (MODE == kModeDelta) valid = valid && bucket_of<W>(R, du) == R.cur;
     if (!valid) {
@@ -511,30 +594,8 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
   // the whole warp, taken by any warp in the next phase
   const uint32_t hub_deg = R.kind == kPhaseLocal ? 0xFFFFFFFFu : P.hub_degree;
   const bool is_hub = deg >= hub_deg;
-  uint32_t hubs = __ballot_sync(0xffffffffu, is_hub);
-  if (hubs) {
-    const uint32_t mine = is_hub ? (deg + kHubChunk - 1) / kHubChunk : 0u;
-    const uint32_t incl = warp_incl_scan(mine);
-    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t hb = 0;
-    if (lane == 0) hb = atomicAdd(&c->hub_count[R.hub_out & 1], all);
-    hb = __shfl_sync(0xffffffffu, hb, 0);
-    if ((uint64_t)hb + all <= P.hub_cap) {
-      HubEntry* H = P.hubs + (size_t)(R.hub_out & 1) * P.hub_cap + hb;
-      do {
-        const uint32_t hl = __ffs(hubs) - 1;
-        hubs &= hubs - 1;
-        const uint32_t hv = __shfl_sync(0xffffffffu, v, hl);
-        const uint32_t nch = __shfl_sync(0xffffffffu, mine, hl);
-        const uint32_t first = __shfl_sync(0xffffffffu, incl, hl) - nch;
-        for (uint32_t j = lane; j < nch; j += 32)
-          *reinterpret_cast<uint2*>(H + first + j) = make_uint2(hv, j);
-      } while (hubs);
-    } else if (lane == 0) {
-      set_error(P, kErrQueueOverflow, 20);
-    }
-    if (is_hub) deg = 0;
-  }
+  if (MODE == kModeDelta) append_hubs(P, R, v, deg, is_hub);   // (BF listed its chunks when it pushed v)
+  if (is_hub) deg = 0;
   // compact the lanes that have edges to relax
   const uint32_t nz = __ballot_sync(0xffffffffu, deg > 0);
   const uint32_t k = __popc(nz);
@@ -853,6 +914,15 @@ __device__ void manager_init(const Params& P, PhaseRec& r) {
   r.hround = P.phase_base + 1;
   r.hub_in = 1;
   r.hub_out = 0;
+  if (MODE == kModeBF) {   // a high-degree source: its chunks, as a push would have listed them
+    const uint64_t deg = P.rowptr[P.source + 1] - P.rowptr[P.source];
+    if (deg >= P.hub_degree) {
+      const uint32_t nch = (uint32_t)min((deg + kHubChunk - 1) / kHubChunk, (uint64_t)P.hub_cap);
+      HubEntry* H = P.hubs + (size_t)(r.hub_in & 1) * P.hub_cap;
+      for (uint32_t j = 0; j < nch; ++j) *reinterpret_cast<uint2*>(H + j) = make_uint2(P.source, j);
+      r.hub_in_chunks = nch;
+    }
+  }
   r.iter = 1;
   r.dq = P.delta_u;
   r.dinv = __float_as_uint(P.inv_delta);
@@ -886,16 +956,14 @@ __device__ __forceinline__ void consume_process_counters(Control* c, const Phase
   if (r.hub_in_chunks) c->hub_count[r.hub_in & 1] = 0u;
 }
 
-// BF round bookkeeping.  PhaseRec.aux is the round's role: 0 ordinary round,
-// 2 ordinary round whose commit precedes the negative-cycle probe, 1 the probe
-// round (python reference: one extra relaxation after max_iters,
-// minplus_bellman_ford.py:92-99).  At FINAL, aux = 1 means "output the
-// committed round".
+// BF round bookkeeping.  PhaseRec.aux = 1 marks the negative-cycle probe (python
+// reference: one extra relaxation after max_iters, minplus_bellman_ford.py:92-99),
+// and at FINAL "output the labels that round read".
 __device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, PhaseRec& nx) {
   Control* c = P.ctl;
   // every word the step may need, loaded at once (one round trip)
-  const uint32_t phases = vld(&c->phases), stamp_ctr = vld(&c->stamp_ctr);
-  const uint32_t hub_out = vld(&c->hub_count[r.hub_out & 1]), near = vld(&c->near_count[r.push_q & 1]);
+  const uint32_t phases = vld(&c->phases);
+  const uint32_t hch = vld(&c->hub_count[r.hub_out & 1]), nn = vld(&c->near_count[r.push_q & 1]);
   const unsigned long long t_start = vld64(&c->t_start);
   trace_phase(P, r, r.iter);
   nx = r;
@@ -903,59 +971,32 @@ __device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, Phas
   c->phases = phases + 1;
   if (r.kind == kPhaseFinal) { nx.kind = kPhaseDone; return; }
   if (over_budget(P, t_start, nx)) return;
-  if (r.kind == kPhaseCommit) {
-    nx.kind = kPhaseProcess;
-    nx.fq = r.fq;
-    nx.fcount = r.fcount;
-    nx.push_q = r.fq ^ 1u;
-    nx.stamp = P.phase_base + stamp_ctr;
-    c->stamp_ctr = stamp_ctr + 1;
-    nx.hub_in = r.hub_out ^ 1u;
-    nx.hub_in_count = 0;
-    nx.hub_in_chunks = 0;
-    nx.iter = r.iter + 1;
-    nx.aux = (r.aux == 2u) ? 1u : 0u;
-    return;
-  }
   consume_process_counters(c, r);
-  const uint32_t hch = hub_out;
-  if (hch > 0) {   // hub chunks of this round: same round, same push queue and stamp
-    nx.kind = kPhaseProcess;
-    nx.fq = kQNone;
-    nx.fcount = 0;
-    nx.hub_in = r.hub_out;
-    nx.hub_in_count = hch;
-    nx.hub_in_chunks = hch;
-    nx.hub_out = r.hub_out ^ 1u;
-    return;
-  }
-  const uint32_t nn = near;
   const bool changed = nn > 0;
-  nx.hub_in_chunks = 0;
-  nx.hub_in_count = 0;
   if (r.aux == 1u) {
     c->negative_cycle = changed ? 1u : 0u;
-    nx.kind = kPhaseFinal;   // aux stays 1: output the committed round
+    nx.kind = kPhaseFinal;   // aux stays 1
     return;
   }
   c->iterations = r.iter;
   publish_progress(P.board, r.iter, changed ? 1u : 0u, globaltimer_ns() - t_start);
-  if (!changed) {
-    c->converged = 1;
-    c->first_unchanged = r.iter;
+  if (!changed || (r.iter >= P.max_iters && !P.detect_negcycle)) {
+    if (!changed) {
+      c->converged = 1;
+      c->first_unchanged = r.iter;
+    }
     nx.kind = kPhaseFinal;
-    nx.aux = 0u;
     return;
   }
-  if (r.iter >= P.max_iters && !P.detect_negcycle) {
-    nx.kind = kPhaseFinal;
-    nx.aux = 0u;
-    return;
-  }
-  nx.kind = kPhaseCommit;
   nx.fq = r.push_q;
   nx.fcount = nn;
-  nx.aux = (r.iter >= P.max_iters) ? 2u : 0u;
+  nx.push_q = r.push_q ^ 1u;
+  nx.hub_in = r.hub_out;
+  nx.hub_in_count = hch;
+  nx.hub_in_chunks = hch;
+  nx.hub_out = r.hub_out ^ 1u;
+  nx.aux = r.iter >= P.max_iters ? 1u : 0u;
+  nx.iter = r.iter + 1;
 }
 
 // A large near or slot frontier is found by a stamp sweep (see sweep_span).
@@ -1359,12 +1400,6 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
       if (MODE == kModeDelta && blockIdx.x == 0) local_phase<W, PRED, MODE>(P, R, t);
     } else if (R.kind == kPhasePull) {
       if (MODE == kModeDelta) pull_phase<W, PRED>(P, R, t);
-    } else if (R.kind == kPhaseCommit) {
-      const uint32_t* F = queue_ptr(P, R.fq);
-      for (size_t i = tid; i < R.fcount; i += stride) {
-        const uint32_t v = ldcg(F + i);
-        ((typename L::T*)P.dist_cur)[v] = ldcg((const typename L::T*)P.dist + v);
-      }
     } else if (R.kind == kPhaseSplit) {
       const uint32_t* F = queue_ptr(P, R.fq);
       uint32_t kmin = 0xFFFFFFFFu;
@@ -1424,7 +1459,7 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
       if (any) c->probe_valid = 1u;
     } else if (R.kind == kPhaseFinal) {
       const typename L::T* srcl =
-          (const typename L::T*)((MODE == kModeBF && R.aux == 1u) ? P.dist_cur : P.dist);
+          (const typename L::T*)(MODE == kModeDelta ? P.dist : R.aux == 1u ? bf_read(P, R) : bf_write(P, R));
       // in output order: a degree-ordered graph gathers each slot's label
       // (mostly L2-resident) instead of scattering 4-byte writes
       for (size_t o = tid; o < P.n; o += stride) {
@@ -1675,6 +1710,7 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
   P.ctl = w.ctl;
   P.trace = o.trace ? w.trace : nullptr;
   P.hub_degree = std::max<uint32_t>(32u, o.hub_degree ? o.hub_degree : 256u);
+  P.has_hubs = (uint64_t)g->max_degree >= P.hub_degree ? 1u : 0u;
   P.out_dist = d_dist;
   P.out_pred = d_pred;
   P.is_float = isf ? 1u : 0u;
@@ -1773,9 +1809,14 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, st);
-  // small graphs: about one thread per vertex (every grid barrier costs an
-  // arrival per block, and a graph of a few thousand vertices cannot use more)
-  const int small_grid = (int)std::max<int64_t>(1, (g->n + kThreads - 1) / kThreads);
+  // graphs with fewer vertices than one block per SM has threads: one block per
+  // SM.  A few items then run on as many SMs, and a barrier of 148 blocks costs
+  // little more than one of 8 (Bellman-Ford, RMAT-13: 0.28 ms with one thread per
+  // vertex, 0.20 with 148 blocks, 0.19 with 296; ER-1000: 0.18 and 0.16).
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int small_grid = g->n <= (int64_t)sms * kThreads ? std::max(1, sms) : INT32_MAX;
 #define B2_LAUNCH(WT, PR, MD)                                              \
   do {                                                                     \
     grid = max_grid<WT, PR, MD>();                                         \
@@ -1832,7 +1873,14 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
       stats->delta_final = delta;
   }
   if (ds != B2_SUCCESS) return ds;
-  if (stats && o.collect_reach) return collect_reach(g, (pred || g->perm) ? w.dist_a : d_dist, pred, isf, st, stats);
+  if (stats && o.collect_reach) {
+    const void* lab = d_dist;
+    if (pred || g->perm) {   // the label array that the output came from
+      const bool second = mode == kModeBF && ((hc.rec.iter & 1u) != 0) == (hc.rec.aux == 1u);
+      lab = second ? P.dist_cur : P.dist;
+    }
+    return collect_reach(g, lab, pred, isf, st, stats);
+  }
   return B2_SUCCESS;
 }
 
