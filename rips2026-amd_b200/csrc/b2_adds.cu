@@ -69,8 +69,18 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;       // no vertex: a wait gave up
 constexpr unsigned long long kEmpty64 = ~0ull; // empty ring word (bucket rings and the hub ring)
 constexpr uint32_t kNotQueued = 0xFFFFFFFFu;   // qb[v]: not waiting in any bucket
 constexpr uint32_t kGrab = 32;                 // entries a warp takes from its block's pool (one per lane)
-constexpr uint32_t kBlockClaimMin = 64;        // entries a block claims from a bucket at once: its share
-constexpr uint32_t kBlockClaimMax = 1024;      //   of the bucket's unclaimed entries, within these bounds
+// Entries a block claims from a bucket at once: its share of the bucket's
+// unclaimed entries, but at most kBlockClaimMax and at least about
+// kBlockClaimEdges edges' worth (64 to kBlockClaimMax entries).  Claims are
+// compare-and-swaps of one word per bucket, so many small ones cost their square
+// (of n blocks that try, one succeeds at a time), and fewer than 512 entries
+// leave some of a block's 16 warps without a grab; but large claims of long rows
+// keep the other blocks idle.  With 64 / 128 / 256 / 512 / 1024 entries: grid
+// 900 x 1000 4.25 / 2.99 / 2.42 / 2.02 / 1.59 ms, ER-300000 of degree 12 2.30 /
+// 2.08 / 1.53 / 1.11 / 1.03, RMAT-18 2.04 / 1.53 / 1.29 / 1.27 / 1.23, RMAT-20
+// (mean degree 30) 3.7 / 3.6 / 4.1 / 4.8 / 5.2.
+constexpr uint32_t kBlockClaimMax = 1024;
+constexpr double kBlockClaimEdges = 4096.0;
 constexpr uint32_t kChunkEdges = 256;          // edges per hub chunk
 constexpr uint32_t kHubClaim = 32;             // hub chunks a block claims at once
 constexpr int kU = 4;                          // edge slots per lane per step
@@ -96,6 +106,7 @@ struct AParams {
   uint32_t active0;        // buckets from the head warps may take at the start of an epoch
   uint32_t active_max;     // the active range never widens past this
   uint32_t hub_degree;
+  uint32_t claim_min;      // entries a block claims at least (kBlockClaimEdges)
   uint32_t adapt;          // adjust the width at every new epoch
   uint32_t adapt_cap;      // entries per bucket that fill the grid once
   uint32_t warm;           // keep the labels in `warm_in` (initialize_distances = false)
@@ -635,7 +646,7 @@ __device__ bool refill(const AParams& P, BlockPool& sp) {
         if (got == R || (int32_t)(R - got) < 0) break;
         const uint32_t avail = R - got;
         const uint32_t share = avail / max(1u, gridDim.x);
-        const uint32_t k = min(avail, max(kBlockClaimMin, min(share, kBlockClaimMax)));
+        const uint32_t k = min(avail, max(P.claim_min, min(share, kBlockClaimMax)));
         if (atomicCAS(&c->slot[ss].claim, w, w + k) == w) {
           publish_range(&sp.ticket, sp.ent, got, k, ss);
           return true;
@@ -1162,6 +1173,8 @@ b2_status run_adds(b2_graph g, uint32_t source, void* d_dist, int32_t* d_pred, c
   else grid = pred ? adds_grid<WU32, true>() : adds_grid<WU32, false>();
   if (o.grid_blocks && (int)o.grid_blocks < grid) grid = (int)o.grid_blocks;
   if (grid <= 0) return B2_CUDA_ERROR;
+  P.claim_min = (uint32_t)std::min<double>(
+      kBlockClaimMax, std::max(64.0, std::floor(kBlockClaimEdges / std::max(1.0, g->mean_degree) / 32.0) * 32.0));
   P.adapt_cap = (uint32_t)grid * (kAThreads / 32) * kGrab;   // one grab per warp fills the grid
   if (stats) {
     memset(stats, 0, sizeof(*stats));
