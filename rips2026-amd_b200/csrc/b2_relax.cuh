@@ -112,6 +112,25 @@ __device__ __forceinline__ uint32_t atom_min_if(bool p, uint32_t* a, uint32_t x,
                : "+r"(old) : "l"(a), "r"(x), "r"((uint32_t)p) : "memory");
   return old;
 }
+__device__ __forceinline__ unsigned long long atom_min_if(bool p, unsigned long long* a, unsigned long long x,
+                                                          unsigned long long dflt) {
+  unsigned long long old = dflt;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q atom.global.min.u64 %0, [%1], %2;\n\t}"
+               : "+l"(old) : "l"(a), "l"(x), "r"((uint32_t)p) : "memory");
+  return old;
+}
+__device__ __forceinline__ uint32_t ld_cg_if(bool p, const uint32_t* a, uint32_t dflt) {
+  uint32_t v = dflt;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.cg.u32 %0, [%1];\n\t}"
+               : "+r"(v) : "l"(a), "r"((uint32_t)p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_cg_if(bool p, const unsigned long long* a, unsigned long long dflt) {
+  unsigned long long v = dflt;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.cg.u64 %0, [%1];\n\t}"
+               : "+l"(v) : "l"(a), "r"((uint32_t)p) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint32_t atom_exch_if(bool p, uint32_t* a, uint32_t x, uint32_t dflt) {
   uint32_t old = dflt;
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q atom.global.exch.b32 %0, [%1], %2;\n\t}"

@@ -33,6 +33,7 @@
 
 #include "b2_common.cuh"
 #include "b2_internal.hpp"
+#include "b2_relax.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -109,16 +110,19 @@ __device__ __forceinline__ uint32_t sbucket(const ServeQuery& q, uint32_t key) {
   return b >= 4294967040.0f ? 0xFFFFFFFEu : (uint32_t)b;
 }
 
+// Counters of the near phases are used three in turn: a phase counts its pushes
+// and long rows in one, reads the previous phase's after the barrier between
+// them, and clears the next phase's, which nobody reads any more.  So a phase
+// needs no barrier for its counters.
 struct SShared {
-  uint32_t ncount;     // current near frontier
-  uint32_t next_count; // pushes into the next near queue
+  uint32_t near[3];    // pushes into the near queue (frontier of the next phase)
+  uint32_t nhub[3];    // long rows of the frontier
   uint32_t fcount;     // far pile entries
   uint32_t fnext;      // kept far entries during a split
   uint32_t cur;        // current bucket
   uint32_t minb;       // split: smallest live bucket
-  uint32_t stop;
-  uint32_t nhub;
-  uint32_t hubs[kHubListCap];
+  uint32_t stop[3];    // budget verdict of a phase (0: go on)
+  uint32_t hubs[2][kHubListCap];   // by parity of the phase
   unsigned long long red[3];
 };
 
@@ -142,58 +146,85 @@ struct TeamCluster {
   __device__ static T* lead(T* p) { return cg::this_cluster().map_shared_rank(p, 0); }
 };
 
-// Relax kSU edges per lane (u's label key -> v): all edge loads are issued
-// first, then all label loads, then the atomics, so one lane keeps kSU
-// independent memory requests in flight; improved vertices go to the next
-// near queue or the far pile (warp-aggregated appends).
+// Relax kSU edges per lane (u's label key -> v; warp-collective): label loads,
+// then the label atomics, then the dedup exchanges, each issued for all edges
+// before a result is read, then one reservation for the warp's pushes into the
+// near queue and the far pile (a lane per counter).  A team's phases are a few
+// steps per warp, so their length is this chain: with every edge's atomic,
+// exchange and appends one after the other (16 round trips or more instead of
+// 4, those to the counters through distributed shared memory for a cluster) and
+// three barriers a phase, a burst of 256 queries over 9 graphs took 46.3 ms, with
+// this 40.2; 64 graphs at 10000 queries/s 6300 -> 7250 queries/s.
 constexpr int kSU = 4;
 
 template <class W, bool PRED>
-__device__ __forceinline__ void relax_edges(const ServeQuery& q, SShared& sh, const uint32_t (&ukey)[kSU],
-                                            const uint32_t (&u)[kSU], const uint2 (&e)[kSU], const bool (&valid)[kSU],
-                                            uint32_t next_stamp, uint32_t* qnext) {
+__device__ __forceinline__ void relax_edges(const ServeQuery& q, SShared& sh, uint32_t cur_bucket, uint32_t* count,
+                                            const uint32_t (&ukey)[kSU], const uint32_t (&u)[kSU],
+                                            const uint2 (&e)[kSU], const bool (&valid)[kSU], uint32_t next_stamp,
+                                            uint32_t* qnext) {
   using L = SLabel<PRED>;
   typename L::T* lab = (typename L::T*)q.labels;
-  uint32_t nd[kSU], cur[kSU];
+  uint32_t nd[kSU];
+  typename L::T cur[kSU], old[kSU];
 #pragma unroll
   for (int k = 0; k < kSU; ++k) {
     nd[k] = valid[k] ? W::extend(ukey[k], e[k].y) : kInfKey;
-    cur[k] = nd[k] != kInfKey ? L::key(__ldcg(lab + e[k].x)) : kInfKey;
+    cur[k] = ld_cg_if(nd[k] != kInfKey, lab + e[k].x, (typename L::T)0);
   }
-  bool imp[kSU];
+  bool any = false;
 #pragma unroll
   for (int k = 0; k < kSU; ++k) {
-    imp[k] = false;
     // with predecessors an equal distance may still lower the predecessor id
-    if (nd[k] != kInfKey && (PRED ? nd[k] <= cur[k] : nd[k] < cur[k])) {
-      const typename L::T old = L::atomic_min(lab + e[k].x, L::make(nd[k], u[k]));
-      imp[k] = nd[k] < L::key(old);
-    }
+    // (not issued: old = 0 reads as "no improvement")
+    const bool better = PRED ? nd[k] <= L::key(cur[k]) : nd[k] < L::key(cur[k]);
+    old[k] = atom_min_if(nd[k] != kInfKey && better, lab + e[k].x, L::make(nd[k], u[k]), (typename L::T)0);
   }
+  uint32_t near_before[kSU], far_before[kSU];
 #pragma unroll
   for (int k = 0; k < kSU; ++k) {
-    bool to_near = false, to_far = false;
-    const uint32_t v = e[k].x;
-    if (imp[k]) {
-      if (sbucket<W>(q, nd[k]) <= sh.cur) to_near = atomicExch(q.stamp + v, next_stamp) != next_stamp;
-      else to_far = atomicExch(q.farflag + v, 1u) == 0u;
-    }
-    const uint32_t pn = warp_append(&sh.next_count, to_near);
-    if (to_near) qnext[pn] = v;
-    const uint32_t pf = warp_append(&sh.fcount, to_far);
-    if (to_far) q.fa[pf] = v;
+    const bool imp = nd[k] < L::key(old[k]);
+    const bool now = imp && sbucket<W>(q, nd[k]) <= cur_bucket;
+    any = any || imp;
+    // defaults read as "already queued"
+    near_before[k] = atom_exch_if(now, q.stamp + e[k].x, next_stamp, next_stamp);
+    far_before[k] = atom_exch_if(imp && !now, q.farflag + e[k].x, 1u, 1u);
+  }
+  if (!__any_sync(0xffffffffu, any)) return;
+  uint32_t bn[kSU], bf[kSU], nn = 0, nf = 0;
+#pragma unroll
+  for (int k = 0; k < kSU; ++k) {
+    bn[k] = __ballot_sync(0xffffffffu, near_before[k] != next_stamp);
+    bf[k] = __ballot_sync(0xffffffffu, far_before[k] == 0u);
+    nn += __popc(bn[k]);
+    nf += __popc(bf[k]);
+  }
+  if ((nn | nf) == 0) return;
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  uint32_t base = 0;
+  if (lane < 2 && (lane == 0 ? nn : nf)) base = atomicAdd(lane == 0 ? count : &sh.fcount, lane == 0 ? nn : nf);
+  uint32_t pn = __shfl_sync(0xffffffffu, base, 0), pf = __shfl_sync(0xffffffffu, base, 1);
+#pragma unroll
+  for (int k = 0; k < kSU; ++k) {
+    if (near_before[k] != next_stamp) qnext[pn + __popc(bn[k] & below)] = e[k].x;
+    if (far_before[k] == 0u) q.fa[pf + __popc(bf[k] & below)] = e[k].x;
+    pn += __popc(bn[k]);
+    pf += __popc(bf[k]);
   }
 }
 
 // One near phase: warps take 32-vertex chunks of the frontier and walk the
 // chunk's edges lane-parallel; rows of kBlockHubDeg or more edges are
-// collected and relaxed afterwards by the whole block.
+// collected and relaxed afterwards by the whole team.  Ends with a barrier of
+// the team; returns the next frontier's size.
 template <class W, bool PRED, class Team>
-__device__ void near_phase(const ServeQuery& q, SShared& sh, const uint32_t* qcur, uint32_t* qnext,
-                           uint32_t next_stamp, unsigned long long& edges) {
+__device__ uint32_t near_phase(const ServeQuery& q, SShared& sh, const uint32_t* qcur, uint32_t cnt, uint32_t* qnext,
+                               uint32_t phase, uint32_t cur_bucket, unsigned long long& edges) {
   using L = SLabel<PRED>;
   const uint32_t lane = threadIdx.x & 31u, warp = Team::tid() >> 5;
-  const uint32_t cnt = sh.ncount;
+  const uint32_t set = phase % 3u, next_stamp = phase + 1;
+  uint32_t* count = &sh.near[set];
+  uint32_t* nhub = &sh.nhub[set];
+  uint32_t* hubs = sh.hubs[phase & 1u];
   typename L::T* lab = (typename L::T*)q.labels;
   for (uint32_t base = warp * 32; base < cnt; base += Team::threads()) {
     const uint32_t i = base + lane;
@@ -201,70 +232,90 @@ __device__ void near_phase(const ServeQuery& q, SShared& sh, const uint32_t* qcu
     uint64_t start = 0;
     if (i < cnt) {
       u = qcur[i];
-      ukey = L::key(__ldcg(lab + u));
       start = __ldg(q.rowptr + u);
       const uint64_t d = __ldg(q.rowptr + u + 1) - start;
+      ukey = L::key(__ldcg(lab + u));
       if (d >= kBlockHubDeg) {
-        const uint32_t slot = atomicAdd(&sh.nhub, 1u);
-        if (slot < kHubListCap) sh.hubs[slot] = u;
+        const uint32_t slot = atomicAdd(nhub, 1u);
+        if (slot < kHubListCap) hubs[slot] = u;
         else deg = (uint32_t)d;            // hub list full: this warp walks the row
       } else {
         deg = (uint32_t)d;
       }
     }
-    const uint32_t incl = warp_incl_scan(deg);
+    edges += deg;
+    // move the rows with edges to the front; an edge slot's owner is then the
+    // number of range starts at or before it (one warp-OR per 32 slots)
+    const uint32_t nz = __ballot_sync(0xffffffffu, deg > 0);
+    const uint32_t k0 = __popc(nz);
+    if (k0 == 0) continue;
+    const bool has = lane < k0;
+    const uint32_t sl = nth_set_bit(nz, has ? lane : 0u);
+    const uint32_t cu = __shfl_sync(0xffffffffu, u, sl);
+    const uint32_t ckey = __shfl_sync(0xffffffffu, ukey, sl);
+    const uint32_t sdeg = __shfl_sync(0xffffffffu, deg, sl);
+    const uint32_t cdeg = has ? sdeg : 0u;
+    const unsigned long long cst = shfl64(start, sl);
+    const uint32_t incl = warp_incl_scan(cdeg);
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    const uint32_t excl = incl - deg;
+    const uint32_t excl = incl - cdeg;
+    const unsigned long long ebase = cst - excl;
+    uint32_t started = 0;
     for (uint32_t e0 = 0; e0 < total; e0 += 32 * kSU) {
       uint32_t okey[kSU], ou[kSU];
       uint2 ed[kSU];
       bool valid[kSU];
 #pragma unroll
       for (int k = 0; k < kSU; ++k) {
-        const uint32_t e = e0 + 32u * k + lane;
-        // owner: first lane whose inclusive prefix exceeds e
-        uint32_t lo = 0;
-#pragma unroll
-        for (uint32_t s = 16; s > 0; s >>= 1) {
-          const uint32_t pv = __shfl_sync(0xffffffffu, incl, lo + s - 1);
-          if (pv <= e) lo += s;
-        }
-        const uint32_t owner = lo > 31 ? 31 : lo;
-        const uint32_t oex = __shfl_sync(0xffffffffu, excl, owner);
-        const uint64_t ost = __shfl_sync(0xffffffffu, start, owner);
-        okey[k] = __shfl_sync(0xffffffffu, ukey, owner);
-        ou[k] = __shfl_sync(0xffffffffu, u, owner);
+        const uint32_t w0 = e0 + 32u * k;
+        const uint32_t bit = (has && excl >= w0 && excl < w0 + 32) ? (1u << (excl - w0)) : 0u;
+        const uint32_t starts = __reduce_or_sync(0xffffffffu, bit);
+        uint32_t own = started + __popc(starts & lanemask_le()) - 1;
+        started += __popc(starts);
+        own = min(own, 31u);
+        const uint32_t e = w0 + lane;
+        okey[k] = __shfl_sync(0xffffffffu, ckey, own);
+        ou[k] = __shfl_sync(0xffffffffu, cu, own);
+        const unsigned long long at = shfl64(ebase, own) + e;
         valid[k] = e < total;
-        ed[k] = valid[k] ? __ldcs(q.edges + ost + (e - oex)) : make_uint2(0, 0);
+        ed[k] = valid[k] ? __ldcs(q.edges + at) : make_uint2(0, 0);
       }
-      relax_edges<W, PRED>(q, sh, okey, ou, ed, valid, next_stamp, qnext);
+      relax_edges<W, PRED>(q, sh, cur_bucket, count, okey, ou, ed, valid, next_stamp, qnext);
     }
-    edges += deg;
+  }
+  if (Team::tid() == 0) {   // the next phase's counters (read last in the previous phase)
+    sh.near[(phase + 1) % 3u] = 0;
+    sh.nhub[(phase + 1) % 3u] = 0;
   }
   Team::sync();
-  const uint32_t nh = min(sh.nhub, kHubListCap);
-  for (uint32_t h = 0; h < nh; ++h) {
-    const uint32_t u = sh.hubs[h];
-    const uint32_t ukey = L::key(__ldcg(lab + u));
-    const uint64_t start = __ldg(q.rowptr + u), end = __ldg(q.rowptr + u + 1);
-    const uint64_t len = end - start;
-    // every thread of the team runs the same number of iterations (warp_append needs whole warps)
-    for (uint64_t k0 = 0; k0 < len; k0 += (uint64_t)Team::threads() * kSU) {
-      uint32_t okey[kSU], ou[kSU];
-      uint2 ed[kSU];
-      bool valid[kSU];
+  const uint32_t listed = *nhub;
+  if (listed) {
+    const uint32_t nh = min(listed, kHubListCap);
+    for (uint32_t h = 0; h < nh; ++h) {
+      const uint32_t u = hubs[h];
+      const uint32_t ukey = L::key(__ldcg(lab + u));
+      const uint64_t start = __ldg(q.rowptr + u), end = __ldg(q.rowptr + u + 1);
+      const uint64_t len = end - start;
+      // every thread of the team runs the same number of iterations (relax_edges needs whole warps)
+      for (uint64_t k0 = 0; k0 < len; k0 += (uint64_t)Team::threads() * kSU) {
+        uint32_t okey[kSU], ou[kSU];
+        uint2 ed[kSU];
+        bool valid[kSU];
 #pragma unroll
-      for (int j = 0; j < kSU; ++j) {
-        const uint64_t k = k0 + (uint64_t)j * Team::threads() + Team::tid();
-        valid[j] = k < len;
-        okey[j] = ukey;
-        ou[j] = u;
-        ed[j] = valid[j] ? __ldcs(q.edges + start + k) : make_uint2(0, 0);
+        for (int j = 0; j < kSU; ++j) {
+          const uint64_t k = k0 + (uint64_t)j * Team::threads() + Team::tid();
+          valid[j] = k < len;
+          okey[j] = ukey;
+          ou[j] = u;
+          ed[j] = valid[j] ? __ldcs(q.edges + start + k) : make_uint2(0, 0);
+        }
+        relax_edges<W, PRED>(q, sh, cur_bucket, count, okey, ou, ed, valid, next_stamp, qnext);
       }
-      relax_edges<W, PRED>(q, sh, okey, ou, ed, valid, next_stamp, qnext);
+      if (Team::tid() == 0) edges += len;
     }
-    if (Team::tid() == 0) edges += len;
+    Team::sync();
   }
+  return *count;
 }
 
 template <class W, bool PRED, class Team>
@@ -282,44 +333,42 @@ __device__ void team_solve(ServeQuery& q, SShared& sh, uint64_t t0, uint64_t bud
     lab[q.source] = L::make(W::zero_key(), kNoPred);
     q.qa[0] = q.source;
     q.stamp[q.source] = 1u;
-    sh.ncount = 1;
-    sh.next_count = 0;
+    for (int k = 0; k < 3; ++k) {
+      sh.near[k] = 0;
+      sh.nhub[k] = 0;
+    }
     sh.fcount = 0;
-    sh.cur = sbucket<W>(q, W::zero_key());
-    sh.stop = 0;
-    sh.nhub = 0;
   }
   Team::sync();
   unsigned long long edges = 0;
   uint32_t phase = 1;
+  uint32_t cnt = 1;                                   // current near frontier
+  uint32_t cur = sbucket<W>(q, W::zero_key());        // current bucket
   uint32_t* qcur = q.qa;
   uint32_t* qnext = q.qb;
   uint32_t status = 0;
   for (;;) {
     // light phases of the current bucket
-    while (sh.ncount > 0) {
-      near_phase<W, PRED, Team>(q, sh, qcur, qnext, phase + 1, edges);
-      Team::sync();
+    uint32_t stop = 0;
+    while (cnt > 0) {
+      const uint32_t set = phase % 3u;
+      if (Team::tid() == 0)   // written before the phase's barrier, read after it, written again three phases on
+        sh.stop[set] = phase >= 0xFFFFFFF0u ? kErrQueueOverflow   // stamp space exhausted
+                       : globaltimer_ns() - t0 > budget_ns ? kErrTimeout : kErrNone;
+      cnt = near_phase<W, PRED, Team>(q, sh, qcur, cnt, qnext, phase, cur, edges);
       ++phase;
       uint32_t* t = qcur;
       qcur = qnext;
       qnext = t;
-      if (Team::tid() == 0) {
-        sh.ncount = sh.next_count;
-        sh.next_count = 0;
-        sh.nhub = 0;
-        if (globaltimer_ns() - t0 > budget_ns) sh.stop = kErrTimeout;
-        if (phase >= 0xFFFFFFF0u) sh.stop = kErrQueueOverflow;   // stamp space exhausted
-      }
-      Team::sync();
-      if (sh.stop) break;
+      stop = sh.stop[set];
+      if (stop) break;
     }
-    if (sh.stop) { status = sh.stop; break; }
+    if (stop) { status = stop; break; }
     if (sh.fcount == 0) break;
     // far split, pass 1: smallest live bucket above the current one
     if (Team::tid() == 0) sh.minb = kSNone;
     Team::sync();
-    const uint32_t fc = sh.fcount, cur = sh.cur;
+    const uint32_t fc = sh.fcount;
     uint32_t mb = kSNone;
     for (uint32_t i = Team::tid(); i < fc; i += Team::threads()) {
       const uint32_t b = sbucket<W>(q, L::key(__ldcg(lab + q.fa[i])));
@@ -331,7 +380,7 @@ __device__ void team_solve(ServeQuery& q, SShared& sh, uint64_t t0, uint64_t bud
     Team::sync();
     const uint32_t nb = sh.minb;
     if (nb == kSNone) break;                          // every far entry is settled
-    if (Team::tid() == 0) { sh.cur = nb; sh.fnext = 0; sh.next_count = 0; }
+    if (Team::tid() == 0) sh.fnext = 0;
     Team::sync();
     // pass 2: entries of bucket nb go to the near queue, later ones are kept
     const uint32_t st = phase + 1;
@@ -351,21 +400,23 @@ __device__ void team_solve(ServeQuery& q, SShared& sh, uint64_t t0, uint64_t bud
           keep = true;
         }
       }
-      const uint32_t pn = warp_append(&sh.next_count, to_near);
+      const uint32_t pn = warp_append(&sh.near[phase % 3u], to_near);   // cleared by the phase before
       if (to_near) qcur[pn] = v;
       const uint32_t pk = warp_append(&sh.fnext, keep);
       if (keep) q.fb[pk] = v;
     }
     Team::sync();
-    ++phase;
     uint32_t* t = q.fa;
     q.fa = q.fb;
     q.fb = t;
+    cnt = sh.near[phase % 3u];
     if (Team::tid() == 0) {
-      sh.ncount = sh.next_count;
-      sh.next_count = 0;
       sh.fcount = sh.fnext;
+      sh.near[(phase + 1) % 3u] = 0;
+      sh.nhub[(phase + 1) % 3u] = 0;
     }
+    cur = nb;
+    ++phase;
     Team::sync();
   }
   // output into the caller's buffers, then the completion record
