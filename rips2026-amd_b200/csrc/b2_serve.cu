@@ -76,6 +76,12 @@ struct ServeQuery {
 namespace {
 
 constexpr int kServeThreads = 512;
+// By default graphs of this many edges get a cluster too, however few their
+// vertices: one block takes 25 ms or more for a query on an RMAT-18 graph (7.6 M
+// edges, 2^18 vertices).  256 queries over 9 graphs up to RMAT-18: 37.5 ms with
+// 2^23, 24.3 with 2^22, 24.1 with 2^21; 64 graphs (RMAT 12-20, grids 64-2048):
+// 7275 / 7260 / 7225 queries/s, p99 at 1000 queries/s 32 / 26 / 27 ms.
+constexpr int64_t kBigEdges = (int64_t)1 << 22;
 constexpr uint32_t kBlockHubDeg = 512;     // rows at least this long are relaxed by the whole block
 constexpr uint32_t kHubListCap = 128;
 
@@ -1015,7 +1021,7 @@ extern "C" b2_status b2_server_add_graph(b2_server s, b2_graph g, int32_t* graph
   G.g = g;
   G.n = (uint32_t)g->n;
   G.isf = g->weight_type == B2_W_F32;
-  G.big = G.n >= s->big_n;
+  G.big = G.n >= s->big_n || (s->o.big_vertices == 0 && g->m >= kBigEdges);
   G.tuned = false;
   b2_status st = set_bucket_width(G, s->o.delta_scale > 0 ? s->o.delta_scale : 4.0);
   if (st != B2_SUCCESS) return st;
