@@ -247,6 +247,7 @@ enum AddsHead : uint32_t {
 struct Workspace {
   size_t n = 0;
   bool pred = false;
+  void* slab = nullptr;       // the one allocation that holds every device array below
   void* dist_a = nullptr;     // 4n or 8n bytes
   void* dist_b = nullptr;     // BF second buffer
   uint32_t* pstamp = nullptr; // near-queue dedup stamps
