@@ -887,6 +887,45 @@ __device__ __forceinline__ void trace_phase(const Params& P, const PhaseRec& r, 
   c->trace_n = i + 1;
 }
 
+// Every counter that a manager step may read, loaded by a warp in one round trip
+// into shared memory (a lane per word; the second half is the control block's
+// line from far_min on).  Loaded by the manager's one thread into registers and
+// local arrays the step took 2.2 us: 411 x 300 grid 0.775 -> 0.746 ms, RMAT-24 5.43
+// -> 5.26, 4096^2 grid 4.11 -> 4.01.
+struct MgrSnap {
+  uint32_t slot[kRing], near[2], far[2], hub[2], members, error, pad[8];
+  uint32_t far_min, far_min_next, bucket_valid, probe_valid, cur_min_key, heavy_pulls;
+  unsigned long long member_heavy;
+  uint32_t trace_n, stamp_ctr, local_q, local_iters, fusion_off, local_total, delta_updates;
+  uint32_t iterations, converged, negative_cycle, phases, first_unchanged, done;
+  unsigned long long t_start;
+};
+constexpr size_t kSnapLine = offsetof(MgrSnap, far_min);
+constexpr int kSnapLineWords = (int)((sizeof(MgrSnap) - kSnapLine) / 4);
+static_assert(kSnapLine == 128 && kSnapLineWords <= 32 &&
+                  offsetof(MgrSnap, member_heavy) - kSnapLine ==
+                      offsetof(Control, member_heavy) - offsetof(Control, far_min) &&
+                  offsetof(MgrSnap, stamp_ctr) - kSnapLine ==
+                      offsetof(Control, stamp_ctr) - offsetof(Control, far_min) &&
+                  offsetof(MgrSnap, phases) - kSnapLine == offsetof(Control, phases) - offsetof(Control, far_min) &&
+                  offsetof(MgrSnap, t_start) - kSnapLine == offsetof(Control, t_start) - offsetof(Control, far_min),
+              "the snapshot mirrors the control block's line");
+__device__ __forceinline__ void snapshot(const Control* c, MgrSnap* m) {
+  const uint32_t lane = lane_id();
+  const uint32_t* a = lane < 16 ? c->slot_count + lane
+                      : lane < 18 ? c->near_count + (lane - 16)
+                      : lane < 20 ? c->far_count + (lane - 18)
+                      : lane < 22 ? c->hub_count + (lane - 20)
+                      : lane == 22 ? &c->members_count
+                                   : &c->error;
+  const uint32_t x = vld(a);
+  const uint32_t y = lane < (uint32_t)kSnapLineWords ? vld(&c->far_min + lane) : 0u;
+  uint32_t* w = reinterpret_cast<uint32_t*>(m);
+  w[lane] = x;
+  if (lane < (uint32_t)kSnapLineWords) w[32 + lane] = y;
+  __syncwarp();
+}
+
 template <bool PRED, int MODE>
 __device__ void manager_init(const Params& P, PhaseRec& r) {
   using L = Label<PRED>;
@@ -949,29 +988,21 @@ __device__ __forceinline__ void consume_queue(Control* c, uint32_t fq) {
   else if (fq >= kQSlot0 && fq < kQSlot0 + kRing) c->slot_count[fq - kQSlot0] = 0;
 }
 
-__device__ __forceinline__ void consume_process_counters(Control* c, const PhaseRec& r) {
-  if (r.fq == kQNear0 || r.fq == kQNear1) c->near_count[r.fq] = 0;
-  else if (r.fq == kQMembers) c->members_count = 0;
-  else if (r.fq >= kQSlot0 && r.fq < kQSlot0 + kRing) c->slot_count[r.fq - kQSlot0] = 0;
-  if (r.hub_in_chunks) c->hub_count[r.hub_in & 1] = 0u;
-}
 
 // BF round bookkeeping.  PhaseRec.aux = 1 marks the negative-cycle probe (python
 // reference: one extra relaxation after max_iters, minplus_bellman_ford.py:92-99),
 // and at FINAL "output the labels that round read".
-__device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, PhaseRec& nx) {
+// (nx arrives as a copy of r)
+__device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, const MgrSnap& m, PhaseRec& nx) {
   Control* c = P.ctl;
-  // every word the step may need, loaded at once (one round trip)
-  const uint32_t phases = vld(&c->phases);
-  const uint32_t hch = vld(&c->hub_count[r.hub_out & 1]), nn = vld(&c->near_count[r.push_q & 1]);
-  const unsigned long long t_start = vld64(&c->t_start);
+  const uint32_t hch = m.hub[r.hub_out & 1], nn = m.near[r.push_q & 1];
   trace_phase(P, r, r.iter);
-  nx = r;
   nx.phase = r.phase + 1;
-  c->phases = phases + 1;
+  c->phases = m.phases + 1;
   if (r.kind == kPhaseFinal) { nx.kind = kPhaseDone; return; }
-  if (over_budget(P, t_start, nx)) return;
-  consume_process_counters(c, r);
+  if (over_budget(P, m.t_start, nx)) return;
+  consume_queue(c, r.fq);
+  if (r.hub_in_chunks) c->hub_count[r.hub_in & 1] = 0u;
   const bool changed = nn > 0;
   if (r.aux == 1u) {
     c->negative_cycle = changed ? 1u : 0u;
@@ -979,7 +1010,7 @@ __device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, Phas
     return;
   }
   c->iterations = r.iter;
-  publish_progress(P.board, r.iter, changed ? 1u : 0u, globaltimer_ns() - t_start);
+  publish_progress(P.board, r.iter, changed ? 1u : 0u, globaltimer_ns() - m.t_start);
   if (!changed || (r.iter >= P.max_iters && !P.detect_negcycle)) {
     if (!changed) {
       c->converged = 1;
@@ -1007,48 +1038,10 @@ __device__ __forceinline__ void set_dense(const Params& P, PhaseRec& nx, uint32_
   }
 }
 
-// Every counter a delta manager step may read, loaded at once: independent
-// volatile loads issue back to back, so the step costs about one L2 round
-// trip instead of one per decision.
-struct MgrSnap {
-  uint32_t phases, probe_valid, local_q, local_total, local_iters, fusion_off, members, bucket_valid;
-  uint32_t iterations, heavy_pulls, far_min, far_min_next, stamp_ctr;
-  uint32_t hub[2], near[2], far[2], slot[kRing];
-  unsigned long long member_heavy, t_start;
-};
-__device__ __forceinline__ MgrSnap snapshot(const Control* c) {
-  MgrSnap m;
-  m.phases = vld(&c->phases);
-  m.probe_valid = vld(&c->probe_valid);
-  m.local_q = vld(&c->local_q);
-  m.local_total = vld(&c->local_total);
-  m.local_iters = vld(&c->local_iters);
-  m.fusion_off = vld(&c->fusion_off);
-  m.members = vld(&c->members_count);
-  m.bucket_valid = vld(&c->bucket_valid);
-  m.iterations = vld(&c->iterations);
-  m.heavy_pulls = vld(&c->heavy_pulls);
-  m.far_min = vld(&c->far_min);
-  m.far_min_next = vld(&c->far_min_next);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    m.hub[i] = vld(&c->hub_count[i]);
-    m.near[i] = vld(&c->near_count[i]);
-    m.far[i] = vld(&c->far_count[i]);
-  }
-#pragma unroll
-  for (int s = 0; s < kRing; ++s) m.slot[s] = vld(&c->slot_count[s]);
-  m.stamp_ctr = vld(&c->stamp_ctr);
-  m.member_heavy = vld64(&c->member_heavy);
-  m.t_start = vld64(&c->t_start);
-  return m;
-}
-
-__device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, PhaseRec& nx) {
+// (nx arrives as a copy of r; the step consumes counters in the snapshot too)
+__device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, MgrSnap& m, PhaseRec& nx) {
   Control* c = P.ctl;
-  MgrSnap m = snapshot(c);
   trace_phase(P, r, r.cur);
-  nx = r;
   nx.dense = kDenseOff;
   nx.fstamp = 0u;
   nx.phase = r.phase + 1;
@@ -1074,29 +1067,31 @@ __device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, P
     c->far_min_next = 0xFFFFFFFFu;
     from_slot = 0;
   } else {  // PROCESS (light or heavy) or LOCAL
-    PhaseRec rr = r;
+    uint32_t fq = r.fq, push_q = r.push_q, chunks = r.hub_in_chunks;
+    bool heavy = r.heavy != 0;
     if (r.kind == kPhaseLocal) {
       // the local loop consumed every frontier it ran; its last pushes sit in local_q
-      rr.fq = kQNone;
-      rr.hub_in_chunks = 0;
-      rr.push_q = m.local_q;
-      rr.heavy = 0;
+      fq = kQNone;
+      chunks = 0;
+      push_q = m.local_q;
+      heavy = false;
       c->local_total = m.local_total + m.local_iters;
     }
-    const PhaseRec& r = rr;
-    consume_process_counters(c, r);
-    // the same consumption in the snapshot
-    if (r.fq == kQNear0 || r.fq == kQNear1) m.near[r.fq] = 0;
-    else if (r.fq == kQMembers) m.members = 0;
-    else if (r.fq >= kQSlot0 && r.fq < kQSlot0 + kRing) m.slot[r.fq - kQSlot0] = 0;
-    if (r.hub_in_chunks) m.hub[r.hub_in & 1] = 0u;
+    consume_queue(c, fq);
+    if (fq == kQNear0 || fq == kQNear1) m.near[fq] = 0;
+    else if (fq == kQMembers) m.members = 0;
+    else if (fq >= kQSlot0 && fq < kQSlot0 + kRing) m.slot[fq - kQSlot0] = 0;
+    if (chunks) {
+      c->hub_count[r.hub_in & 1] = 0u;
+      m.hub[r.hub_in & 1] = 0u;
+    }
     const uint32_t hch = m.hub[r.hub_out & 1];
-    const uint32_t nn = m.near[r.push_q & 1];
+    const uint32_t nn = m.near[push_q & 1];
     nx.hub_in = r.hub_out;
     nx.hub_in_count = hch;
     nx.hub_in_chunks = hch;
     nx.hub_out = r.hub_out ^ 1u;
-    if (r.heavy) {
+    if (heavy) {
       if (hch > 0) {             // heavy hub chunks first; near pushes keep accumulating
         nx.fq = kQNone;
         nx.fcount = 0;
@@ -1106,9 +1101,9 @@ __device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, P
       if (nn > 0) {              // a heavy relaxation landed in this bucket: new light round
         nx.kind = kPhaseProcess;
         nx.heavy = 0;
-        nx.fq = r.push_q;
+        nx.fq = push_q;
         nx.fcount = nn;
-        nx.push_q = r.push_q ^ 1u;
+        nx.push_q = push_q ^ 1u;
         nx.hround = P.phase_base + nx.phase;
         set_dense(P, nx, kDenseNear, r.stamp);
         return;
@@ -1116,9 +1111,9 @@ __device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, P
     } else {
       if (nn > 0 || hch > 0) {
         nx.kind = kPhaseProcess;
-        nx.fq = nn ? r.push_q : kQNone;
+        nx.fq = nn ? push_q : kQNone;
         nx.fcount = nn;
-        nx.push_q = r.push_q ^ 1u;
+        nx.push_q = push_q ^ 1u;
         if (hch == 0 && nn <= P.fusion && !m.fusion_off) nx.kind = kPhaseLocal;
         // (a LOCAL phase's last pushes carry a stamp drawn inside it: no sweep after one)
         if (nn > 0 && r.kind != kPhaseLocal) set_dense(P, nx, kDenseNear, r.stamp);
@@ -1286,7 +1281,8 @@ constexpr uint32_t kDirectMax = 1024;
 // solve budget; whoever gives up sets the error word, which all waits poll.
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 template <typename Manager>
-__device__ __forceinline__ void next_phase(const Params& P, PhaseRec* s_rec, WarpPhase* slots, bool expanded,
+__device__ __forceinline__ void next_phase(const Params& P, PhaseRec* s_rec, PhaseRec* s_next, MgrSnap* s_snap,
+                                           WarpPhase* slots, bool expanded,
                                            uint32_t& barrier, Manager&& manager) {
   Control* c = P.ctl;
   __syncthreads();   // every warp is done with the phase and its record
@@ -1303,24 +1299,26 @@ __device__ __forceinline__ void next_phase(const Params& P, PhaseRec* s_rec, War
     last = __shfl_sync(0xffffffffu, last, 0);
     volatile uint32_t* rec = reinterpret_cast<volatile uint32_t*>(s_rec);
     if (last) {
+      snapshot(c, s_snap);
+      volatile uint32_t* next = reinterpret_cast<volatile uint32_t*>(s_next);
+      if (lane < (uint32_t)kRecWords) next[lane] = rec[lane];
+      __syncwarp();
       if (lane == 0) {
-        const uint32_t err = vld(&c->error);
-        const PhaseRec r = *s_rec;
-        PhaseRec nx;
-        manager(r, nx);
-        if (err != kErrNone) nx.kind = kPhaseDone;
+        PhaseRec& nx = *s_next;
+        manager(*s_rec, *s_snap, nx);
+        if (s_snap->error != kErrNone) nx.kind = kPhaseDone;
         nx.fcount = min(nx.fcount, P.qcap);
         nx.direct = nx.kind == kPhaseProcess && nx.fcount <= kDirectMax && nx.hub_in_chunks == 0 &&
                     nx.dense == kDenseOff;
-        *s_rec = nx;
       }
       __syncwarp();
       fence_acq_rel();
       if (lane < (uint32_t)kRecWords) {
-        const uint32_t w = rec[lane];
+        const uint32_t w = next[lane];
+        rec[lane] = w;
         asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(c->box + lane),
                      "l"(((unsigned long long)barrier << 32) | w) : "memory");
-        if (s_rec->kind == kPhaseDone) reinterpret_cast<uint32_t*>(&c->rec)[lane] = w;
+        if (s_next->kind == kPhaseDone) reinterpret_cast<uint32_t*>(&c->rec)[lane] = w;
       }
     } else {
       unsigned long long w = 0;
@@ -1366,7 +1364,8 @@ __device__ __forceinline__ void next_phase(const Params& P, PhaseRec* s_rec, War
 template <class W, bool PRED, int MODE>
 __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_constant__ Params P) {
   using L = Label<PRED>;
-  __shared__ PhaseRec s_rec;
+  __shared__ PhaseRec s_rec, s_next;
+  __shared__ MgrSnap s_snap;
   __shared__ WarpPhase s_phase[kWarpsPerBlock];
   extern __shared__ uint32_t s_stage[];   // kStageWords per warp
   Tally t;
@@ -1387,8 +1386,8 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
     }
   }
   uint32_t barrier = 0;
-  next_phase(P, &s_rec, s_phase, false, barrier,
-             [&](const PhaseRec&, PhaseRec& nx) { manager_init<PRED, MODE>(P, nx); });
+  next_phase(P, &s_rec, &s_next, &s_snap, s_phase, false, barrier,
+             [&](const PhaseRec&, MgrSnap&, PhaseRec& nx) { manager_init<PRED, MODE>(P, nx); });
   for (;;) {
     const PhaseRec R = s_rec;
     if (R.kind == kPhaseDone) break;
@@ -1482,10 +1481,11 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
       }
     }
     if (expands) flush_phase(s_phase + (threadIdx.x >> 5), t);
-    next_phase(P, &s_rec, s_phase, MODE == kModeDelta && expands, barrier, [&](const PhaseRec& r, PhaseRec& nx) {
-      if (MODE == kModeBF) manager_bf(P, r, nx);
-      else manager_delta(P, r, nx);
-    });
+    next_phase(P, &s_rec, &s_next, &s_snap, s_phase, MODE == kModeDelta && expands, barrier,
+               [&](const PhaseRec& r, MgrSnap& m, PhaseRec& nx) {
+                 if (MODE == kModeBF) manager_bf(P, r, m, nx);
+                 else manager_delta(P, r, m, nx);
+               });
   }
   // totals of the solve (the last phase ended with a block barrier)
   if (threadIdx.x < (uint32_t)kWarpsPerBlock) {
