@@ -300,9 +300,9 @@ b2_status b2_minplus_status(b2_stream stream);
  * that array until exit.  All calls on a device share it: calls that overlap
  * on the GPU race and must be serialized by the caller.  The first call on a
  * device resolves the array's device address (cudaGetSymbolAddress) with that
- * device current.  Every call synchronizes `stream` after each squaring (it
- * reads the change flag on the host), so no call may be made on a stream that
- * is being captured. */
+ * device current.  Every call waits for `stream` once (it reads the change
+ * flags on the host), so no call may be made on a stream that is being
+ * captured. */
 b2_status b2_apsp_f32_noalloc(float* d_D, int32_t N, b2_stream stream, int32_t* squarings_out);
 /* Sustained (min,+) pairs per second of this GPU's CUDA cores, measured by a
  * register-only kernel of the same instruction mix as the GEMM inner loop
