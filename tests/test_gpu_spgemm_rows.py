@@ -65,10 +65,12 @@ def test_rows_of_every_length(b2, orc, cuda, dtype, N):
     _check(b2, orc, cuda, rows, blen, N, dtype, N % 77)
 
 
-# long rows: one pass of 49152 columns, its edges, several passes, and the widest
-# matrix that is accumulated densely and the first that is not
+# long rows: one pass of 49152 columns, its edges, several passes (where some of the
+# rows are too short for them and are sorted), and the widest matrix that is
+# accumulated densely and the first that is not
 @pytest.mark.parametrize("dtype", [np.float32, np.int32])
-@pytest.mark.parametrize("N", [3, 513, 1000, 24576, 24577, 49151, 49152, 49153, 130000, 196608, 196609])
+@pytest.mark.parametrize("N", [3, 513, 1000, 24576, 24577, 49151, 49152, 49153, 130000, 196608, 196609, 786432,
+                               786433])
 def test_long_rows(b2, orc, cuda, dtype, N):
     rng = np.random.default_rng(N % 991)
     K = 1500
