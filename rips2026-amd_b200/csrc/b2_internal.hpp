@@ -168,8 +168,8 @@ struct alignas(128) Control {
 // after every finished round / bucket (`rounds` last, with a system-scope
 // release); the calling thread polls it while the kernel runs.
 struct ProgressBoard {
-  uint32_t rounds;
-  uint32_t changed;
+  uint32_t rounds;     // finished rounds; top bit: the last of them changed something
+  uint32_t reserved;
   unsigned long long t_ns;   // end of the round, ns after the solve's start
 };
 

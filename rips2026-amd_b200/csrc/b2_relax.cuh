@@ -13,14 +13,17 @@
 namespace b2 {
 
 // Publish a finished round / bucket to the mapped progress record (one
-// thread; `rounds` is stored last with a system-scope release).
+// thread).  The round and whether it changed anything are one word, stored last
+// with a system-scope release: with a word each, the host could read round k with
+// the flag of round k + 1, the last one among them, as soon as rounds follow each
+// other within its poll.
 __device__ __forceinline__ void publish_progress(ProgressBoard* b, uint32_t rounds, uint32_t changed,
                                                  unsigned long long t_ns) {
   if (!b) return;
-  *(volatile uint32_t*)&b->changed = changed;
   *(volatile unsigned long long*)&b->t_ns = t_ns;
   __threadfence_system();
-  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(&b->rounds), "r"(rounds) : "memory");
+  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(&b->rounds),
+               "r"((rounds & 0x7fffffffu) | (changed ? 0x80000000u : 0u)) : "memory");
 }
 
 // ---------------------------------------------------------------------------

@@ -1616,7 +1616,6 @@ b2_status progress_begin(b2_graph g, const b2_sssp_opts& o, ProgressBoard** boar
     }
   }
   *(volatile uint32_t*)&w.board_h->rounds = 0;
-  *(volatile uint32_t*)&w.board_h->changed = 0;
   *(volatile unsigned long long*)&w.board_h->t_ns = 0;
   *board_d = w.board_d;
   return B2_SUCCESS;
@@ -1642,9 +1641,9 @@ void progress_poll(b2_graph g, const b2_sssp_opts& o, cudaEvent_t done, int32_t 
   const volatile ProgressBoard* b = g->ws.board_h;
   for (;;) {
     const cudaError_t q = cudaEventQuery(done);
-    const uint32_t r = b->rounds;
+    const uint32_t w = b->rounds, r = w & 0x7fffffffu;
     std::atomic_thread_fence(std::memory_order_acquire);
-    if (r > *reported) report_upto(o, max_iters, r, b->changed, (double)b->t_ns * 1e-6, reported);
+    if (r > *reported) report_upto(o, max_iters, r, w >> 31, (double)b->t_ns * 1e-6, reported);
     if (q != cudaErrorNotReady) return;
     std::this_thread::sleep_for(std::chrono::microseconds(20));
   }
