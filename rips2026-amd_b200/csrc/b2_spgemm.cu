@@ -68,6 +68,10 @@ constexpr int kDenseCols = 49152;
 constexpr int kDensePasses = 16;
 constexpr unsigned long long kDensePerPass = 640;
 constexpr unsigned long long kHeavyRow = 32768;   // dealt first, so that none starts last
+constexpr int kDenseThreads = 1024;               // largest block of k_rows_dense
+// Candidates of a row are counted in 32 bits, and the index that walks them must
+// not wrap in its last step of up to kDenseThreads; longer rows are refused.
+constexpr unsigned long long kDenseRowMax = 0xFFFFFFFFull - kDenseThreads;
 
 enum SpStatus : uint32_t { kSpOk = 0, kSpBadIndex = 1, kSpBadRowptr = 2 };
 
@@ -113,7 +117,7 @@ struct VKey<int32_t> {
 struct SpCounters {
   unsigned long long heavy, lng, mid, wide;   // entries of the four row lists
   uint32_t status;
-  uint32_t too_long;   // a row of 2^32 candidates or more
+  uint32_t too_long;   // a row of more than kDenseRowMax candidates
 };
 
 // Candidates per row, validation, and the lists of the rows that need
@@ -162,7 +166,7 @@ __global__ void k_row_bound(int64_t M, int64_t K, int64_t annz, int64_t bnnz, co
     const bool is_dense = is_long && s >= dense_from;
     const bool is_heavy = is_dense && s >= kHeavyRow;
     const bool is_mid = lead && !is_long && s > (unsigned long long)kSmallRowMax;
-    if (is_dense && s > 0xFFFFFFFFull) cnt->too_long = 1u;
+    if (is_dense && s > kDenseRowMax) cnt->too_long = 1u;
     if (lead) ub[i] = is_dense && s > dense_slots ? dense_slots : s;
     const uint32_t below = (1u << lane) - 1u;
     const uint32_t bh = __ballot_sync(0xffffffffu, is_heavy);
@@ -538,6 +542,7 @@ __global__ void __launch_bounds__(kRowWarps * 32)
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_rows_dense(const RowArgs<T> R, const int64_t* __restrict__ rows, int64_t nheavy,
                                                    int64_t nlong, int cap, unsigned long long* next) {
+  static_assert(NT <= kDenseThreads, "kDenseRowMax leaves room for a step of the largest block");
   extern __shared__ uint32_t s_acc[];   // cap words
   __shared__ uint32_t s_excl[NT + 1];
   __shared__ long long s_base[NT];
@@ -892,7 +897,7 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   if (e != cudaSuccess) return from_cuda(e);
   if (hc.status == kSpBadIndex) return B2_INVALID_INDEX;
   if (hc.status == kSpBadRowptr) return B2_INVALID_ROWPTR;
-  if (hc.too_long) return B2_NOT_SUPPORTED;   // the row kernels count a row's candidates in 32 bits
+  if (hc.too_long) return B2_NOT_SUPPORTED;
   const int64_t nheavy = (int64_t)hc.heavy, nlong = (int64_t)hc.lng, nmid = (int64_t)hc.mid;
   const int64_t L = (int64_t)hc.wide;   // rows to expand and sort: the last L entries of mrows
   const int64_t* const wrows = mrows.p + (M - L);
@@ -917,7 +922,7 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
       // 512 threads while two blocks or more fit an SM, else 1024
       if (e == cudaSuccess)
         e = cap <= 24576 ? launch_dense<T, 512>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st)
-                         : launch_dense<T, 1024>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st);
+                         : launch_dense<T, kDenseThreads>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st);
     }
     const bool b32 = B->nnz < (1ll << 31);   // 32-bit indices into B beside the 32-bit keys
     auto blocks = [&](int64_t warps, int per_sm) {
