@@ -874,8 +874,10 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   // a densely accumulated row needs at most N result slots (kept past the ordinary
   // rows' limit, by which the row kernels tell them apart)
   const unsigned long long passes = (unsigned long long)((N + kDenseCols - 1) / kDenseCols);
-  const unsigned long long dense_from =
-      passes > (unsigned long long)kDensePasses ? ~0ull : passes > 1 ? passes * kDensePerPass : 0ull;
+  // (a matrix without columns takes no pass: the expansion checks its entries' columns)
+  const unsigned long long dense_from = passes == 0 || passes > (unsigned long long)kDensePasses ? ~0ull
+                                        : passes > 1 ? passes * kDensePerPass
+                                                     : 0ull;
   const unsigned long long dense_slots =
       std::max<unsigned long long>((unsigned long long)N, (unsigned long long)kWarpRowMax + 1);
   cudaError_t e = cudaMemsetAsync(counters.p, 0, sizeof(SpCounters), st);
