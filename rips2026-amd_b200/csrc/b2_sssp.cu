@@ -90,6 +90,7 @@ struct Params {
   const uint32_t* __restrict__ lightcnt;   // null: relax whole rows in every sub-phase
   void* dist;        // labels receiving atomicMin
   void* dist_cur;    // BF: the second label array (see bf_read / bf_write)
+  unsigned long long* ties;   // BF with predecessors and a probe: smaller predecessors at equal distances
   uint32_t* pstamp;
   uint32_t* bstamp;
   uint32_t* farflag;
@@ -444,9 +445,15 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
       old[q] = atom_min_keep_if(cand[q] < L::key(cur[q]), wr + ed[q].x, cw, t.keep, (typename L::T)0);
       if (PRED && cand[q] == L::key(cur[q]) && cw < cur[q]) {
         // a smaller predecessor at an equal distance: the vertex is not expanded
-        // again, so both arrays take it
-        atomicMin(rd + ed[q].x, cw);
-        atomicMin(wr + ed[q].x, cw);
+        // again, so both arrays take it.  A solve that may end with the probe keeps
+        // it apart: a probe's output has the predecessors of each vertex's last
+        // improvement, a converged one's the smallest of all.
+        if (P.ties) {
+          atomicMin(P.ties + ed[q].x, cw);
+        } else {
+          atomicMin(rd + ed[q].x, cw);
+          atomicMin(wr + ed[q].x, cw);
+        }
       }
     }
 #pragma unroll
@@ -464,7 +471,6 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
 #pragma unroll
   for (int q = 0; q < U; ++q) {
     cand[q] = act[q] ? W::extend(dsrc[q], ed[q].y) : kInfKey;
-    
     cur[q] = ld_keep_if(cand[q] != kInfKey && !R.direct, lab + ed[q].x, t.keep, L::kInf);
   }
 #pragma unroll
@@ -1380,6 +1386,7 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
   for (size_t v = tid; v < P.n; v += stride) {
     ((typename L::T*)P.dist)[v] = L::kInf;
     if (MODE == kModeBF) ((typename L::T*)P.dist_cur)[v] = L::kInf;
+    if (PRED && MODE == kModeBF && P.ties) P.ties[v] = ~0ull;
     if (MODE == kModeDelta) {
       P.bstamp[v] = 0xFFFFFFFFu;
       P.farflag[v] = 0u;
@@ -1463,8 +1470,12 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
       // (mostly L2-resident) instead of scattering 4-byte writes
       for (size_t o = tid; o < P.n; o += stride) {
         const size_t v = P.inv ? (size_t)__ldg(P.inv + o) : o;   // internal id of output slot o
-        const typename L::T wv = ldcg(srcl + v);
+        typename L::T wv = ldcg(srcl + v);
         const uint32_t k = L::key(wv);
+        if (PRED && MODE == kModeBF && P.ties && R.aux != 1u) {
+          const unsigned long long tie = ldcg(P.ties + v);   // (no tie has a smaller key than the label)
+          if ((uint32_t)(tie >> 32) == k) wv = min(wv, (typename L::T)tie);
+        }
         if (W::kFloat) {
           ((float*)P.out_dist)[o] = (k == kInfKey) ? __uint_as_float(0x7f800000u) : key_to_f32(k);
         } else if (!P.dist_is_out || (const void*)srcl != P.out_dist) {
@@ -1729,6 +1740,8 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
     if (mi > 0x7fffffff) mi = 0x7fffffff;
     P.max_iters = (uint32_t)mi;
     P.detect_negcycle = o.detect_negative_cycle ? 1u : 0u;
+    static_assert((kQSlot0 + 1) % 2 == 0, "64-bit words over two of the window queues, which Bellman-Ford does not use");
+    if (pred && P.detect_negcycle) P.ties = (unsigned long long*)(w.queues + (size_t)(kQSlot0 + 1) * (size_t)g->n);
     P.inv_delta = 1.0f;
     P.delta_u = 1u;
   } else {
