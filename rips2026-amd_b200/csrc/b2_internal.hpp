@@ -126,7 +126,8 @@ struct alignas(128) Control {
   uint32_t bar_gen;
   uint32_t error;
   uint32_t error_site;
-  PhaseRec rec;            // the last phase's record (read by the host)
+  PhaseRec rec;            // the record that ended the solve (read by the host; zero if every block
+                           // left through a bounded wait instead)
   // The running phase's record: word i with the number of the barrier that
   // released it in the upper half, so that a waiting block polls the record itself.
   alignas(128) unsigned long long box[32];

@@ -1877,12 +1877,9 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
     stats->local_subphases = hc.local_total;
     stats->delta_updates = hc.delta_updates;
     stats->heavy_pulls = hc.heavy_pulls;
-    if (mode == kModeDelta) {
-      float inv;
-      memcpy(&inv, &hc.rec.dinv, 4);
-      stats->delta_final = isf ? 1.0 / (double)inv : (double)hc.rec.dq;
-    } else
-      stats->delta_final = delta;
+    // (the width never changes within a solve; the control block's last record is not
+    //  there when a failed solve ends between phases)
+    stats->delta_final = mode != kModeDelta ? delta : isf ? 1.0 / (double)P.inv_delta : (double)P.delta_u;
   }
   if (ds != B2_SUCCESS) return ds;
   if (stats && o.collect_reach) {
