@@ -1303,6 +1303,7 @@ __device__ __forceinline__ void next_phase(const Params& P, PhaseRec* s_rec, Pha
       last = arrived == gridDim.x * barrier - 1u;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
+    __syncwarp();   // (a shuffle orders no memory: the warp's loads follow lane 0's acquire)
     volatile uint32_t* rec = reinterpret_cast<volatile uint32_t*>(s_rec);
     if (last) {
       snapshot(c, s_snap);
