@@ -192,7 +192,7 @@ typedef struct b2_sssp_opts {
 } b2_sssp_opts;
 
 typedef struct b2_trace_entry {
-  uint32_t kind;        /* 1 relax, 2 commit, 3 far split, 4 probe, 5 output, 7 fused (one block),
+  uint32_t kind;        /* 1 relax, 3 far split, 4 probe, 5 output, 7 fused (one block),
                            8 heavy pass by pull; | 0x100 heavy pass; | 0x200 frontier found by
                            a stamp sweep */
   uint32_t frontier;    /* frontier entries of the phase */
@@ -207,7 +207,7 @@ typedef struct b2_stats {
   int32_t has_negative_cycle;
   int32_t phases;           /* barrier-separated phases executed by the persistent kernel */
   uint64_t edges_scanned;   /* edges read during relaxation */
-  uint64_t improvements;    /* successful atomic-min updates */
+  uint64_t improvements;    /* successful atomic-min updates (a vertex lowered twice counts twice) */
   uint64_t pushes;          /* worklist insertions */
   uint64_t reached;         /* vertices with finite distance */
   uint64_t reached_edges;   /* out-edges of reached vertices (TEPS numerator) */

@@ -460,7 +460,7 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
     for (int q = 0; q < U; ++q) {
       imp[q] = cand[q] < L::key(cur[q]) && L::key(old[q]) >= L::key(cur[q]);   // first below the read label
       t.edges += act[q] ? 1 : 0;
-      t.impr += imp[q] ? 1 : 0;
+      t.impr += cand[q] < L::key(old[q]) ? 1 : 0;   // (not issued: old = 0)
       t.pushes += imp[q] ? 1 : 0;
       stage(t.q.nearb(), t.q.nn, imp[q], ed[q].x);
     }
