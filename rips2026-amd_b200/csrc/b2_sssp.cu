@@ -932,6 +932,13 @@ __device__ __forceinline__ void snapshot(const Control* c, MgrSnap* m) {
   __syncwarp();
 }
 
+// Bellman-Ford: chunks of a high-degree source, which are listed for the first
+// round (list 1) as a push would have listed them.
+__device__ __forceinline__ uint32_t source_chunks(const Params& P) {
+  const uint64_t deg = __ldg(&P.rowptr[P.source + 1]) - __ldg(&P.rowptr[P.source]);
+  return deg < P.hub_degree ? 0u : (uint32_t)min((deg + kHubChunk - 1) / kHubChunk, (uint64_t)P.hub_cap);
+}
+
 template <bool PRED, int MODE>
 __device__ void manager_init(const Params& P, PhaseRec& r) {
   using L = Label<PRED>;
@@ -959,15 +966,7 @@ __device__ void manager_init(const Params& P, PhaseRec& r) {
   r.hround = P.phase_base + 1;
   r.hub_in = 1;
   r.hub_out = 0;
-  if (MODE == kModeBF) {   // a high-degree source: its chunks, as a push would have listed them
-    const uint64_t deg = P.rowptr[P.source + 1] - P.rowptr[P.source];
-    if (deg >= P.hub_degree) {
-      const uint32_t nch = (uint32_t)min((deg + kHubChunk - 1) / kHubChunk, (uint64_t)P.hub_cap);
-      HubEntry* H = P.hubs + (size_t)(r.hub_in & 1) * P.hub_cap;
-      for (uint32_t j = 0; j < nch; ++j) *reinterpret_cast<uint2*>(H + j) = make_uint2(P.source, j);
-      r.hub_in_chunks = nch;
-    }
-  }
+  if (MODE == kModeBF) r.hub_in_chunks = source_chunks(P);   // listed while the labels were cleared
   r.iter = 1;
   r.dq = P.delta_u;
   r.dinv = __float_as_uint(P.inv_delta);
@@ -1392,6 +1391,11 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
       P.bstamp[v] = 0xFFFFFFFFu;
       P.farflag[v] = 0u;
     }
+  }
+  if (MODE == kModeBF && P.has_hubs) {
+    const uint32_t nch = source_chunks(P);
+    for (size_t j = tid; j < nch; j += stride)
+      *reinterpret_cast<uint2*>(P.hubs + P.hub_cap + j) = make_uint2(P.source, (uint32_t)j);
   }
   uint32_t barrier = 0;
   next_phase(P, &s_rec, &s_next, &s_snap, s_phase, false, barrier,
