@@ -145,8 +145,11 @@ typedef struct b2_sssp_opts {
                                exit) when the bucket's members hold more than pull_fraction x n
                                heavy out-edges (default 8); the incoming CSR is built on first
                                use, only for graphs with m >= pull_fraction x n; <= 0: push only */
-  uint32_t grid_blocks;     /* 0: the co-resident persistent grid (BF / delta: one block per SM on
-                               small graphs); k: at most k blocks */
+  uint32_t grid_blocks;     /* 0: the co-resident persistent grid (BF / delta on graphs of up to 512
+                               vertices per SM: one block per SM, a block on every fourth one
+                               while two other solves run on the device); k: at most k blocks.
+                               The blocks of a solve start together, so solves on other threads
+                               and streams overlap as far as their grids fit */
   double timeout_ms;        /* bound on the whole solve and on every device wait, in ms
                                (default 20000; fractions of a millisecond allowed): past it the
                                kernel stops at its next wait or phase boundary and the call

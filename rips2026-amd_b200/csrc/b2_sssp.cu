@@ -1671,6 +1671,20 @@ void progress_finish(b2_graph g, const b2_sssp_opts& o, int32_t max_iters, uint3
   report_upto(o, max_iters, final_rounds, (uint32_t)last_changed, (double)b->t_ns * 1e-6, reported);
 }
 
+namespace {
+// Bellman-Ford and delta-stepping solves between their launch and the end of their
+// wait, per device.
+struct InFlight {
+  static std::atomic<int> count[kMaxDevices];
+  std::atomic<int>& mine;
+  int others;
+  explicit InFlight(int dev) : mine(count[dev >= 0 && dev < kMaxDevices ? dev : 0]), others(mine.fetch_add(1)) {}
+  ~InFlight() { mine.fetch_sub(1); }
+  InFlight(const InFlight&) = delete;
+};
+std::atomic<int> InFlight::count[kMaxDevices];
+}  // namespace
+
 b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t* d_pred,
                    const b2_sssp_opts* o_in, cudaStream_t st, b2_stats* stats) {
   if (!g || !d_dist) return B2_INVALID_ARGUMENT;
@@ -1826,14 +1840,24 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, st);
-  // graphs with fewer vertices than one block per SM has threads: one block per
+  // Graphs with fewer vertices than one block per SM has threads: one block per
   // SM.  A few items then run on as many SMs, and a barrier of 148 blocks costs
   // little more than one of 8 (Bellman-Ford, RMAT-13: 0.28 ms with one thread per
   // vertex, 0.20 with 148 blocks, 0.19 with 296; ER-1000: 0.18 and 0.16).
+  // The blocks of a solve start together, so only two such grids fit the device at
+  // once: a solve that meets two others takes a quarter of the SMs.  Sixteen threads
+  // with a graph each, time per solve with one block per SM / with this rule / with
+  // one thread per vertex: ER-4096 Bellman-Ford 72 / 32 / 31 us, delta-stepping
+  // 151 / 41 / 42; ER-20000 97 / 32 / 34 and 197 / 55 / 61; ER-60000 121 / 46 / 125
+  // and 260 / 73 / 240.  A solve alone loses 4 % (Bellman-Ford, ER-4096) to 20 %
+  // (ER-60000) on a quarter, so it keeps them all.
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int small_grid = g->n <= (int64_t)sms * kThreads ? std::max(1, sms) : INT32_MAX;
+  InFlight in_flight(dev);
+  const int small_grid = g->n > (int64_t)sms * kThreads ? INT32_MAX
+                         : in_flight.others < 2         ? std::max(1, sms)
+                                                        : std::max(1, sms / 4);
 #define B2_LAUNCH(WT, PR, MD)                                              \
   do {                                                                     \
     grid = max_grid<WT, PR, MD>();                                         \
