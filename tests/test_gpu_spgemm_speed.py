@@ -1,0 +1,32 @@
+"""GPU time of the sparse product's row kernels against each other: no row class and no width of
+the result falls off a cliff.  Bounds lie well between the measured ratio and that of the fault."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROWS = 1 << 16
+
+
+def _ms(b2, torch, entries, each, columns):
+    """Median time of a product of ROWS rows of `entries` x `each` candidates."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+
+    def matrix(length, cols):
+        rp = torch.arange(ROWS + 1, dtype=torch.int64, device="cuda") * length
+        ci = torch.randint(0, cols, (ROWS * length,), device="cuda", generator=gen, dtype=torch.int32)
+        return rp, ci, torch.randint(0, 1000, (ROWS * length,), device="cuda", generator=gen, dtype=torch.int32), cols
+
+    a, b = matrix(entries, ROWS), matrix(each, columns)
+    times = []
+    for _ in range(13):
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        b2.minplus_spgemm(a, b)
+        t1.record()
+        torch.cuda.synchronize()
+        times.append(t0.elapsed_time(t1))
+    return sorted(times[3:])[5]
+
+
+def test_rows_past_384_candidates(b2, cuda):
+    """512 candidates against 384: 1.3, and 2.8 with the sorting network of 16 registers left rolled."""
+    assert _ms(b2, cuda, 16, 32, ROWS) < 2.0 * _ms(b2, cuda, 16, 24, ROWS)
