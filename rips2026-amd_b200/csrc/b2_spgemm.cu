@@ -315,13 +315,17 @@ __device__ __forceinline__ void sort_keys(K (&key)[P], uint32_t hl) {
   }
 }
 
-// Sort and leave the keys in order in skey[0 .. LANES * regs).
-template <typename K, int LANES, int PR, int P>
-__device__ __forceinline__ void sort_to_shared(K (&key)[P], uint32_t hl, K* skey) {
+// Sort and leave the keys in order in skey[0 .. LANES * regs).  True if some
+// lane's keys are all of one column, as every run of 2 PR - 1 or more has a lane's
+// (not asked for half warps, whose runs are short enough to walk).
+template <typename K, int LANES, int PR, int SB, int P>
+__device__ __forceinline__ bool sort_to_shared(K (&key)[P], uint32_t hl, K* skey) {
   sort_keys<K, LANES, PR>(key, hl);
   __syncwarp();   // staged keys have been read
 #pragma unroll
   for (int r = 0; r < PR; ++r) skey[hl * PR + r] = key[r];
+  if (LANES < 32) return false;
+  return __any_sync(0xffffffffu, key[PR - 1] != ~(K)0 && (key[0] >> SB) == (key[PR - 1] >> SB));
 }
 
 // One lane's share of a chunk of up to LANES entries of a row of A.
@@ -402,6 +406,37 @@ __device__ __forceinline__ K make_key(const RowArgs<T>& R, T a, T b, int32_t j, 
   return ok ? ((K)(uint32_t)j << SB) | (K)slot : ~(K)0;
 }
 
+// First key of a column's run among the sorted keys.
+template <typename K, int SB>
+__device__ __forceinline__ bool is_head(K me, K before) {
+  return me != ~(K)0 && ((before >> SB) != (me >> SB) || before == ~(K)0);
+}
+
+// Lower each run's first value to the run's minimum, every member for itself, in a
+// row of a whole warp.  Short runs are walked by their head, which spares rows of
+// few duplicates this pass (it cost the rows of half a warp, whose longest run is
+// 128, 7 % and gained a narrow result's 14 %); walked so, 2^16 rows of 512
+// candidates in one column took 1.44 ms a call instead of 0.70.
+template <typename K, int SB>
+__device__ __forceinline__ void lower_heads(const K* skey, uint32_t* sval, int regs, uint32_t lane) {
+  constexpr uint32_t kMask = (uint32_t)(((K)1 << SB) - 1);
+  uint32_t newest = 0;   // the last head so far
+#pragma unroll 1
+  for (int r = 0; r < regs; ++r) {
+    const uint32_t e = (uint32_t)r * 32u + lane;
+    const K me = skey[e], before = e ? skey[e - 1] : ~(K)0;
+    const bool head = is_head<K, SB>(me, before);
+    const uint32_t heads = __ballot_sync(0xffffffffu, head);
+    if (me != ~(K)0 && !head) {
+      const uint32_t at = heads & ((1u << lane) - 1u);
+      const uint32_t first = at ? (uint32_t)r * 32u + 31u - __clz(at) : newest;
+      atomicMin(&sval[(uint32_t)skey[first] & kMask], sval[(uint32_t)me & kMask]);
+    }
+    if (heads) newest = (uint32_t)r * 32u + 31u - __clz(heads);
+  }
+  __syncwarp();
+}
+
 // One row per group of LANES lanes, of at most LANES * regs candidates (regs <= P).
 template <typename T, typename K, int LANES, int P>
 __device__ __forceinline__ void do_row(const RowArgs<T>& R, int64_t i, bool mine, unsigned long long o0, int64_t a0,
@@ -469,18 +504,20 @@ __device__ __forceinline__ void do_row(const RowArgs<T>& R, int64_t i, bool mine
     }
   }
   if (__any_sync(0xffffffffu, bad) && bad) atomicCAS(R.status, kSpOk, (uint32_t)kSpBadIndex);
+  bool long_run;
   if (P == 8) {
-    if (regs <= 4) sort_to_shared<K, LANES, 4>(key, hl, skey);
-    else if (regs == 5) sort_to_shared<K, LANES, 5>(key, hl, skey);
-    else if (regs == 6) sort_to_shared<K, LANES, 6>(key, hl, skey);
-    else if (regs == 7) sort_to_shared<K, LANES, 7>(key, hl, skey);
-    else sort_to_shared<K, LANES, 8>(key, hl, skey);
+    if (regs <= 4) long_run = sort_to_shared<K, LANES, 4, SB>(key, hl, skey);
+    else if (regs == 5) long_run = sort_to_shared<K, LANES, 5, SB>(key, hl, skey);
+    else if (regs == 6) long_run = sort_to_shared<K, LANES, 6, SB>(key, hl, skey);
+    else if (regs == 7) long_run = sort_to_shared<K, LANES, 7, SB>(key, hl, skey);
+    else long_run = sort_to_shared<K, LANES, 8, SB>(key, hl, skey);
   } else {
-    if (regs <= 8) sort_to_shared<K, LANES, 8>(key, hl, skey);
-    else if (regs <= 12) sort_to_shared<K, LANES, 12 <= P ? 12 : P>(key, hl, skey);
-    else sort_to_shared<K, LANES, P>(key, hl, skey);
+    if (regs <= 8) long_run = sort_to_shared<K, LANES, 8, SB>(key, hl, skey);
+    else if (regs <= 12) long_run = sort_to_shared<K, LANES, 12 <= P ? 12 : P, SB>(key, hl, skey);
+    else long_run = sort_to_shared<K, LANES, P, SB>(key, hl, skey);
   }
   __syncwarp();   // sorted keys and all values are in shared memory
+  if (long_run) lower_heads<K, SB>(skey, sval, regs, hl);
   // heads of column runs, in order
   int32_t* tc = R.tcol + o0;
   T* tv = R.tval + o0;
@@ -489,11 +526,11 @@ __device__ __forceinline__ void do_row(const RowArgs<T>& R, int64_t i, bool mine
   for (int r = 0; r < regs; ++r) {
     const uint32_t e = (uint32_t)(r * LANES) + hl;
     const K me = skey[e], before = e ? skey[e - 1] : ~(K)0;
-    const bool head = me != ~(K)0 && ((before >> SB) != (me >> SB) || before == ~(K)0);
+    const bool head = is_head<K, SB>(me, before);
     const uint32_t bal = __ballot_sync(0xffffffffu, head);
     if (head) {
       uint32_t v = sval[(uint32_t)(me & kMask)];
-      for (uint32_t q = e + 1; q < (uint32_t)(regs * LANES); ++q) {
+      for (uint32_t q = e + 1; !long_run && q < (uint32_t)(regs * LANES); ++q) {
         const K other = skey[q];
         if ((other >> SB) != (me >> SB) || other == ~(K)0) break;
         v = min(v, sval[(uint32_t)(other & kMask)]);
