@@ -126,26 +126,27 @@ struct SpCounters {
 // end: mid_rows the rows of up to kWarpRowMax candidates (front) and the long rows
 // to expand and sort (back); long_rows the long rows to accumulate densely, those
 // of at least `dense_from` candidates, the ones of kHeavyRow or more from the front
-// and the others from the back.  Eight lanes per row (a row of A rarely
-// has more entries; one warp per row left most lanes idle: 0.14 -> 0.07 ms for
-// 2^20 rows of 8), list appends aggregated per warp.
+// and the others from the back.  LANES lanes per row (bound_lanes), list appends
+// aggregated per warp.
+template <int LANES>
 __global__ void k_row_bound(int64_t M, int64_t K, int64_t annz, int64_t bnnz, const int64_t* __restrict__ arp,
                             const int32_t* __restrict__ aci, const int64_t* __restrict__ brp,
                             unsigned long long* __restrict__ ub, SpCounters* cnt, int64_t* __restrict__ long_rows,
                             int64_t* __restrict__ mid_rows, unsigned long long dense_from,
                             unsigned long long dense_slots) {
-  const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u;
+  const uint32_t lane = threadIdx.x & 31u, sub = lane & (LANES - 1);
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = warp * 4; base < M; base += nwarps * 4) {
-    const int64_t i = base + (lane >> 3);
+  constexpr int kRpw = 32 / LANES;
+  for (int64_t base = warp * kRpw; base < M; base += nwarps * kRpw) {
+    const int64_t i = base + lane / LANES;
     unsigned long long s = 0;
     if (i < M) {
       const int64_t a0 = arp[i], a1 = arp[i + 1];
       if (a0 < 0 || a1 < a0 || a1 > annz) {
         if (sub == 0) atomicCAS(&cnt->status, kSpOk, (uint32_t)kSpBadRowptr);
       } else {
-        for (int64_t p = a0 + sub; p < a1; p += 8) {
+        for (int64_t p = a0 + sub; p < a1; p += LANES) {
           const int32_t k = aci[p];
           if (k < 0 || (int64_t)k >= K) {
             atomicCAS(&cnt->status, kSpOk, (uint32_t)kSpBadIndex);
@@ -161,7 +162,7 @@ __global__ void k_row_bound(int64_t M, int64_t K, int64_t annz, int64_t bnnz, co
       }
     }
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const bool lead = sub == 0 && i < M;
     const bool is_long = lead && s > (unsigned long long)kWarpRowMax;
     const bool is_dense = is_long && s >= dense_from;
@@ -193,6 +194,14 @@ __global__ void k_row_bound(int64_t M, int64_t K, int64_t annz, int64_t bnnz, co
     }
   }
 }
+
+// A row of A rarely has more than eight entries, and a warp for each leaves most
+// lanes idle (2^20 rows of 8: 0.14 ms with a warp, 0.07 with eight lanes; even for
+// rows of 384 the two are alike).  Where the rows are so few that a warp for each is
+// at hand anyway, the longest of them is what counts (the call for 8192 rows of 3000
+// entries, 3000 columns: 0.83 ms with eight lanes, 0.67 with a warp; for one row of
+// 10^6 entries 32.3 and 11.7).
+int bound_lanes(int64_t M) { return M <= 8192 ? 32 : 8; }
 
 template <typename T>
 struct RowArgs {
@@ -939,8 +948,10 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   cudaError_t e = cudaMemsetAsync(counters.p, 0, sizeof(SpCounters), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(ub.p + M, 0, 8, st);
   if (e == cudaSuccess) {
-    k_row_bound<<<grid_rows((M + 3) / 4), 256, 0, st>>>(M, K, A->nnz, B->nnz, arp, A->colind, brp, ub.p, counters.p,
-                                                        lrows.p, mrows.p, dense_from, dense_slots);
+    const int lanes = bound_lanes(M);
+    auto* bound = lanes == 32 ? k_row_bound<32> : k_row_bound<8>;
+    bound<<<grid_rows((M * lanes + 31) / 32), 256, 0, st>>>(M, K, A->nnz, B->nnz, arp, A->colind, brp, ub.p, counters.p,
+                                                            lrows.p, mrows.p, dense_from, dense_slots);
     e = cudaGetLastError();
   }
   size_t tb = 0;

@@ -35,3 +35,27 @@ def test_rows_past_384_candidates(b2, cuda):
 def test_rows_of_one_column(b2, cuda):
     """512 candidates in one column against distinct ones: 0.9, and 1.8 with a run walked by its head."""
     assert _ms(b2, cuda, 64, 8, 1) < 1.3 * _ms(b2, cuda, 64, 8, ROWS)
+
+
+def test_one_long_row_of_a(b2, cuda):
+    """One row of 2^20 entries against 2^13 rows of 128: 70, and 200 with eight lanes on the row."""
+    torch = cuda
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    total = 1 << 20
+    ones = torch.ones(total, dtype=torch.int32, device="cuda")
+    b = (torch.arange(4097, dtype=torch.int64, device="cuda"), torch.arange(4096, dtype=torch.int32, device="cuda"),
+         ones[:4096], 4096)
+    ci = torch.randint(0, 4096, (total,), device="cuda", generator=gen, dtype=torch.int32)
+    ms = {}
+    for rows in (1, 1 << 13):
+        a = (torch.arange(rows + 1, dtype=torch.int64, device="cuda") * (total // rows), ci, ones, 4096)
+        times = []
+        for _ in range(9):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            b2.minplus_spgemm(a, b)
+            t1.record()
+            torch.cuda.synchronize()
+            times.append(t0.elapsed_time(t1))
+        ms[rows] = sorted(times[3:])[3]
+    assert ms[1] < 120 * ms[1 << 13], ms
