@@ -58,16 +58,25 @@ constexpr int kRowWarps = 8;               // warps per block of k_rows
 
 // Long rows: k_rows_dense takes a row of a matrix of up to kDenseCols columns
 // (192 KB of shared memory), and of a wider one in passes over its columns if the
-// row has kDensePerPass candidates or more for each pass.  A pass costs its scan
-// of the columns (about 6 us) whatever the row holds, expanding and sorting about
-// 20 ns a candidate: rows of 576 candidates in 250000 columns (six passes) take
-// 60 ms densely and 19 ms sorted for 250000 rows, RMAT-18 of edge factor 2 (rows
-// up to millions of candidates) 24 ms with every row dense, 91 ms with every row
-// sorted, 19.5 with this rule at 320 candidates per pass and 15.9 at 640; rows of
-// 576 in 90000 columns 7.7 ms at 320 and 6.8 at 640.
+// row has enough candidates for them.  A pass costs its scan of the columns (about
+// 6 us) whatever the row holds; expanding and sorting costs by the candidate, more
+// so once CUB no longer sorts a segment in one block (5000 candidates, and again
+// about 20000) and where the expansion does not fit the memory that the pool keeps.
+// So rows of under kDensePerPass candidates a pass are sorted, rows of sorted_max()
+// or more accumulated densely, and those between as sort_between() says.  2^13 rows
+// of 3000 candidates in 150000 columns (four passes) 2.64 ms densely and 1.42
+// sorted, of 8000 3.93 and 3.91; of 16000 in 600000 columns (13 passes) 16.4 and
+// 7.1, of 24000 21 and 34; 100 rows of 8000 in 300000 columns 0.28 and 0.53.  90000
+// rows of 2025 in 90000 columns (3 GB of expansion) 15 ms densely and 28 to 65
+// sorted, RMAT-18 of edge factor 2 18 and 25 to 38; below kDensePerPass, 250000 rows
+// of 576 in 250000 columns 60 and 19.
 constexpr int kDenseCols = 49152;
 constexpr int kDensePasses = 16;
 constexpr unsigned long long kDensePerPass = 640;
+constexpr int64_t kSortRows = 512;   // fewer rows leave the sort's one block each waiting for the longest
+unsigned long long sorted_max(unsigned long long passes) {
+  return passes < 4 ? 5120 : std::min(20000ull, 8192 + 5800 * (passes - 4));
+}
 constexpr unsigned long long kHeavyRow = 32768;   // dealt first, so that none starts last
 constexpr int kDenseThreads = 1024;               // largest block of k_rows_dense
 // Candidates of a row are counted in 32 bits, and the index that walks them must
@@ -117,6 +126,8 @@ struct VKey<int32_t> {
 // Device counters read back in one copy after k_row_bound.
 struct SpCounters {
   unsigned long long heavy, lng, mid, wide;   // entries of the four row lists
+  unsigned long long between;                 // rows of `wide` that may as well be accumulated densely
+  unsigned long long split[2];                // cursors of k_split
   uint32_t status;
   uint32_t too_long;   // a row of more than kDenseRowMax candidates
 };
@@ -722,6 +733,10 @@ cudaError_t launch_dense(const RowArgs<T>& R, const int64_t* rows, int64_t nheav
 }
 
 // ---- long rows of wide matrices: expand-sort-compress over a row list --------
+// A warp per row, 32 entries of A at a time: a lane loads an entry, and the warp
+// walks the slots of all their B rows (entry by entry, a row of many entries of few
+// candidates was one chain of loads: 2^13 rows of 1500 entries of 2 candidates, the
+// call 3.00 ms, now 1.59).
 template <typename T>
 __global__ void k_expand(int64_t L, const int64_t* __restrict__ rows, int64_t N, const int64_t* __restrict__ arp,
                          const int32_t* __restrict__ aci, const T* __restrict__ av, const int64_t* __restrict__ brp,
@@ -734,24 +749,43 @@ __global__ void k_expand(int64_t L, const int64_t* __restrict__ rows, int64_t N,
   for (int64_t r = warp; r < L; r += nwarps) {
     const int64_t i = rows[r];
     unsigned long long pos = off[r];
-    for (int64_t p = arp[i]; p < arp[i + 1]; ++p) {
-      const int32_t k = aci[p];
-      const T a = av[p];
-      const int64_t b0 = brp[k], b1 = brp[k + 1];
-      const bool use = SpVal<T>::present(a);
-      for (int64_t q = b0 + lane; q < b1; q += 32) {
-        const int32_t j = bci[q];
-        T c = T(0);
-        bool ok = use && SpVal<T>::combine(a, bv[q], c);
-        if (j < 0 || (int64_t)j >= N) {
-          atomicCAS(status, kSpOk, (uint32_t)kSpBadIndex);
-          ok = false;
-        }
-        const unsigned long long w = pos + (unsigned long long)(q - b0);
-        ccol[w] = ok ? j : kDropCol;
-        cval[w] = c;
+    const int64_t end = arp[i + 1];
+    for (int64_t p0 = arp[i]; p0 < end; p0 += 32) {
+      const int64_t p = p0 + lane;
+      T a = T(0);
+      long long b0 = 0;
+      uint32_t len = 0;   // (all of a sort's items together are fewer than 2^31)
+      if (p < end) {
+        const int32_t k = aci[p];
+        a = av[p];
+        b0 = brp[k];
+        len = (uint32_t)(brp[k + 1] - b0);
       }
-      pos += (unsigned long long)(b1 - b0);
+      const uint32_t incl = warp_incl_scan(len), excl = incl - len;
+      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+      const long long base = b0 - (long long)excl;
+#pragma unroll 2
+      for (uint32_t s0 = 0; s0 < total; s0 += 32) {
+        const uint32_t sl = s0 + lane;
+        uint32_t t = 0;   // the last entry whose range starts at or before slot sl
+#pragma unroll
+        for (uint32_t step = 16; step >= 1; step >>= 1)
+          if (__shfl_sync(0xffffffffu, excl, t + step) <= sl) t += step;
+        const T at = __shfl_sync(0xffffffffu, a, t);
+        const long long q = __shfl_sync(0xffffffffu, base, t) + sl;
+        if (sl < total) {
+          const int32_t j = bci[q];
+          T c = T(0);
+          bool ok = SpVal<T>::present(at) && SpVal<T>::combine(at, bv[q], c);
+          if (j < 0 || (int64_t)j >= N) {
+            atomicCAS(status, kSpOk, (uint32_t)kSpBadIndex);
+            ok = false;
+          }
+          ccol[pos + sl] = ok ? j : kDropCol;
+          cval[pos + sl] = c;
+        }
+      }
+      pos += total;
     }
   }
 }
@@ -791,10 +825,25 @@ __global__ void k_compress(int64_t L, const int64_t* __restrict__ rows, const un
   }
 }
 
+// Candidates of the listed rows, and how many have between_from or more.
 __global__ void k_long_bounds(int64_t L, const int64_t* __restrict__ rows, const unsigned long long* __restrict__ off,
-                              unsigned long long* __restrict__ lub) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < L; r += (int64_t)gridDim.x * blockDim.x)
-    lub[r] = off[rows[r] + 1] - off[rows[r]];
+                              unsigned long long* __restrict__ lub, unsigned long long between_from,
+                              unsigned long long* between) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < L; r += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long s = off[rows[r] + 1] - off[rows[r]];
+    lub[r] = s;
+    if (s >= between_from) atomicAdd(between, 1ull);
+  }
+}
+
+// The listed rows of between_from candidates or more to one list, the others to another.
+__global__ void k_split(int64_t L, const int64_t* __restrict__ rows, const unsigned long long* __restrict__ off,
+                        unsigned long long between_from, unsigned long long* cursor, int64_t* __restrict__ more,
+                        int64_t* __restrict__ fewer) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < L; r += (int64_t)gridDim.x * blockDim.x) {
+    const bool m = off[rows[r] + 1] - off[rows[r]] >= between_from;
+    (m ? more : fewer)[atomicAdd(&cursor[m ? 0 : 1], 1ull)] = rows[r];
+  }
 }
 
 // scratch slots -> exact-size outputs (one warp per row)
@@ -903,8 +952,16 @@ struct SpPlan {
 
 namespace {
 
+// Whether long rows of a wide matrix that either way suits (see kDensePerPass) are
+// sorted: there are rows enough, and the expansion (two pairs of a column and a
+// value per candidate) and the result slots fit what the pool keeps, with room for
+// the sort's own scratch.
+bool sort_between(int64_t rows, unsigned long long candidates, unsigned long long slots) {
+  return rows >= kSortRows && candidates <= 0x7fffffffull && candidates * 16 + slots * 8 <= kPoolKeep / 4 * 3;
+}
+
 // Steps 1-5 up to C's row pointers; one host synchronization for the scratch
-// size (two when long rows exist) and one for nnz(C).
+// size (two or three when rows are expanded) and one for nnz(C).
 template <typename T>
 b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& plan) {
   if (!A || !B) return B2_INVALID_ARGUMENT;
@@ -940,9 +997,12 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   // rows' limit, by which the row kernels tell them apart)
   const unsigned long long passes = (unsigned long long)((N + kDenseCols - 1) / kDenseCols);
   // (a matrix without columns takes no pass: the expansion checks its entries' columns)
-  const unsigned long long dense_from = passes == 0 || passes > (unsigned long long)kDensePasses ? ~0ull
-                                        : passes > 1 ? passes * kDensePerPass
-                                                     : 0ull;
+  const bool can_pass = passes > 0 && passes <= (unsigned long long)kDensePasses;
+  const unsigned long long between_from = can_pass && passes > 1 ? passes * kDensePerPass : ~0ull;
+  const unsigned long long dense_from = !can_pass ? ~0ull
+                                        : passes == 1 ? 0ull
+                                        : M < kSortRows ? between_from
+                                                        : sorted_max(passes);
   const unsigned long long dense_slots =
       std::max<unsigned long long>((unsigned long long)N, (unsigned long long)kWarpRowMax + 1);
   cudaError_t e = cudaMemsetAsync(counters.p, 0, sizeof(SpCounters), st);
@@ -968,8 +1028,8 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   if (hc.status == kSpBadRowptr) return B2_INVALID_ROWPTR;
   if (hc.too_long) return B2_NOT_SUPPORTED;
   const int64_t nheavy = (int64_t)hc.heavy, nlong = (int64_t)hc.lng, nmid = (int64_t)hc.mid;
-  const int64_t L = (int64_t)hc.wide;   // rows to expand and sort: the last L entries of mrows
-  const int64_t* const wrows = mrows.p + (M - L);
+  int64_t L = (int64_t)hc.wide;   // rows to expand and sort: the last L entries of mrows
+  const int64_t* wrows = mrows.p + (M - L);
   uint32_t* const status = &counters.p->status;
   DBuf<int32_t> tcol;
   DBuf<T> tval;
@@ -977,21 +1037,26 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   if (tcol.alloc(U, st) != cudaSuccess || tval.alloc(U, st) != cudaSuccess ||
       cnt.alloc((size_t)M + 1, st) != cudaSuccess)
     return B2_OUT_OF_MEMORY;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const RowArgs<T> R = {M,      N,     arp,    A->colind, (const T*)A->values, brp,   B->colind, (const T*)B->values,
+                        off.p, tcol.p, tval.p, cnt.p,     status};
+  auto dense = [&](const int64_t* rows, int64_t front, int64_t back) -> b2_status {   // k_rows_dense's lists
+    DBuf<unsigned long long> next;
+    if (next.alloc(1, st) != cudaSuccess) return B2_OUT_OF_MEMORY;
+    const int cap = (int)std::min<int64_t>((N + 31) / 32 * 32, kDenseCols);
+    cudaError_t x = cudaMemsetAsync(next.p, 0, 8, st);
+    // 512 threads while two blocks or more fit an SM, else 1024
+    if (x == cudaSuccess)
+      x = cap <= 24576 ? launch_dense<T, 512>(R, rows, front, back, cap, sms, next.p, st)
+                       : launch_dense<T, kDenseThreads>(R, rows, front, back, cap, sms, next.p, st);
+    return from_cuda(x);
+  };
   if (U > 0) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const RowArgs<T> R = {M,      N,     arp,    A->colind, (const T*)A->values, brp,   B->colind, (const T*)B->values,
-                          off.p, tcol.p, tval.p, cnt.p,     status};
     if (nheavy + nlong > 0) {   // first: the longest of them take longest
-      DBuf<unsigned long long> next;
-      if (next.alloc(1, st) != cudaSuccess) return B2_OUT_OF_MEMORY;
-      e = cudaMemsetAsync(next.p, 0, 8, st);
-      const int cap = (int)std::min<int64_t>((N + 31) / 32 * 32, kDenseCols);
-      // 512 threads while two blocks or more fit an SM, else 1024
-      if (e == cudaSuccess)
-        e = cap <= 24576 ? launch_dense<T, 512>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st)
-                         : launch_dense<T, kDenseThreads>(R, lrows.p, nheavy, nlong, cap, sms, next.p, st);
+      const b2_status d = dense(lrows.p, nheavy, nlong);
+      if (d != B2_SUCCESS) return d;
     }
     const bool b32 = B->nnz < (1ll << 31);   // 32-bit indices into B beside the 32-bit keys
     auto blocks = [&](int64_t warps, int per_sm) {
@@ -1014,25 +1079,49 @@ b2_status compute(const b2_csr* A, const b2_csr* B, cudaStream_t st, SpPlan& pla
   }
   // long rows: expand, segmented sort, compress into their scratch slots
   DBuf<unsigned long long> lub, loff;
+  DBuf<int64_t> more, fewer;
   DBuf<int32_t> col0, col1;
   DBuf<T> val0, val1;
   DBuf<unsigned char> tmp2, tmp3;
+  unsigned long long LU = 0;   // candidates of the rows to sort
   if (e == cudaSuccess && L > 0) {
     if (lub.alloc((size_t)L + 1, st) != cudaSuccess || loff.alloc((size_t)L + 1, st) != cudaSuccess)
       return B2_OUT_OF_MEMORY;
-    e = cudaMemsetAsync(lub.p + L, 0, 8, st);
-    if (e == cudaSuccess) {
-      k_long_bounds<<<(int)std::min<int64_t>((L + 255) / 256, 1184), 256, 0, st>>>(L, wrows, off.p, lub.p);
-      e = cudaGetLastError();
-    }
     size_t tb1 = 0;
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb1, lub.p, loff.p, L + 1, st);
+    e = cub::DeviceScan::ExclusiveSum(nullptr, tb1, lub.p, loff.p, L + 1, st);
     if (e == cudaSuccess) e = tmp2.alloc(tb1, st);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp2.p, tb1, lub.p, loff.p, L + 1, st);
-    unsigned long long LU = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&LU, loff.p + L, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    unsigned long long between = 0;
+    auto bounds = [&]() {
+      const int g = (int)std::min<int64_t>((L + 255) / 256, 1184);
+      cudaError_t x = cudaMemsetAsync(lub.p + L, 0, 8, st);
+      if (x == cudaSuccess) {
+        k_long_bounds<<<g, 256, 0, st>>>(L, wrows, off.p, lub.p, between_from, &counters.p->between);
+        x = cudaGetLastError();
+      }
+      if (x == cudaSuccess) x = cub::DeviceScan::ExclusiveSum(tmp2.p, tb1, lub.p, loff.p, L + 1, st);
+      if (x == cudaSuccess) x = cudaMemcpyAsync(&LU, loff.p + L, 8, cudaMemcpyDeviceToHost, st);
+      if (x == cudaSuccess) x = cudaMemcpyAsync(&between, &counters.p->between, 8, cudaMemcpyDeviceToHost, st);
+      if (x == cudaSuccess) x = cudaStreamSynchronize(st);
+      return x;
+    };
+    if (e == cudaSuccess) e = bounds();
     if (e != cudaSuccess) return from_cuda(e);
+    if (between > 0 && !sort_between((int64_t)between, LU, U)) {
+      if (more.alloc((size_t)between, st) != cudaSuccess || fewer.alloc((size_t)L, st) != cudaSuccess)
+        return B2_OUT_OF_MEMORY;
+      k_split<<<(int)std::min<int64_t>((L + 255) / 256, 1184), 256, 0, st>>>(L, wrows, off.p, between_from,
+                                                                            counters.p->split, more.p, fewer.p);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return from_cuda(e);
+      const b2_status d = dense(more.p, (int64_t)between, 0);
+      if (d != B2_SUCCESS) return d;
+      L -= (int64_t)between;
+      wrows = fewer.p;
+      if (L > 0) e = bounds();   // (none of these is counted again)
+      if (e != cudaSuccess) return from_cuda(e);
+    }
+  }
+  if (e == cudaSuccess && L > 0) {
     if (LU > 0x7fffffffull) return B2_NOT_SUPPORTED;   // segmented sort item count is int
     if (col0.alloc(LU, st) != cudaSuccess || col1.alloc(LU, st) != cudaSuccess || val0.alloc(LU, st) != cudaSuccess ||
         val1.alloc(LU, st) != cudaSuccess)
