@@ -409,7 +409,9 @@ typedef struct b2_server_opts {
                                with fewer wasted relaxations pay off) */
   int32_t big_vertices;     /* graphs with at least this many vertices are solved by a cluster of
                                8 blocks (distributed shared memory, cluster barriers) on a
-                               quarter of the lanes; 0: 2^19 vertices, or 2^22 edges; < 0: never */
+                               quarter of the lanes; 0: 2^19 vertices, or 2^22 edges (where
+                               single blocks help once many such queries wait: more are
+                               answered at once that way); < 0: never */
   int32_t autotune;         /* 1: b2_server_add_graph times batches that fill the GPU under each
                                team (block / cluster) x Near-Far constant (2, 4, 8) and keeps the
                                fastest for that graph (needs an idle server); 0: the defaults */

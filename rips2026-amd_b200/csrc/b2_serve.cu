@@ -82,6 +82,21 @@ constexpr int kServeThreads = 512;
 // 2^23, 24.3 with 2^22, 24.1 with 2^21; 64 graphs (RMAT 12-20, grids 64-2048):
 // 7275 / 7260 / 7225 queries/s, p99 at 1000 queries/s 32 / 26 / 27 ms.
 constexpr int64_t kBigEdges = (int64_t)1 << 22;
+// A cluster answers such a query sooner, single blocks answer more of them at once:
+// with many waiting, blocks take them.  Where the line lies depends on the vertices
+// and on how uneven the degrees are.  Queries of one graph at once, ms by clusters /
+// blocks:
+// RMAT-15 of 4.3 M arcs, 16 queries 6.0 / 10.0, 64 12.9 / 10.8, 1024 208 / 53;
+// RMAT-17 of 7.0 M, 64 18 / 24, 128 36 / 29, 1024 274 / 142; RMAT-18 of 7.6 M, 128 44
+// / 49, 192 66 / 61, 1024 333 / 268; even degrees: 30000 vertices 64 4.7 / 6.4, 128
+// 9.7 / 7.2, 65536 vertices 128 9.8 / 9.7, 1024 76 / 52; 131072 vertices and more
+// clusters throughout (1024: 92 / 110, 400000 vertices 131 / 241).
+constexpr uint32_t kNoBurst = 0xFFFFFFFFu;
+uint32_t burst_of(b2_graph g) {
+  const double n = (double)g->n;
+  if ((double)g->max_degree >= 64.0 * g->mean_degree) return (uint32_t)(34.0 * std::pow(n / 32768.0, 0.7)) + 1;
+  return g->n < (1 << 17) ? (uint32_t)(80.0 * std::pow(n / 30000.0, 0.7)) + 1 : kNoBurst;
+}
 constexpr uint32_t kBlockHubDeg = 512;     // rows at least this long are relaxed by the whole block
 constexpr uint32_t kHubListCap = 128;
 
@@ -584,6 +599,7 @@ struct SrvGraph {
   uint32_t n;
   bool isf;
   bool big;             // solved by a block cluster instead of one block
+  uint32_t burst;       // big by its edges alone: waiting queries from which single blocks take it too
   double delta_scale;   // Near-Far constant of the bucket width
   uint32_t delta_u;
   float inv_delta;
@@ -700,17 +716,21 @@ namespace b2 {
 namespace {
 
 // One batch of queries of the lane's kind (big-graph queries on cluster lanes,
-// the others on block lanes), FIFO within the kind.  With a single lane the
-// lane takes the kind of the oldest pending query.
+// the others on block lanes, which take those on graphs big by their edges too once
+// many wait), FIFO within the kind.  With a single lane the lane takes the kind of
+// the oldest pending query.
 b2_status srv_launch(b2_server s, Lane& ln) {
   std::vector<SrvQuery> batch;
+  uint32_t waiting = 0;
+  for (const SrvQuery& q : s->pending) waiting += s->graphs[q.gid].burst != kNoBurst ? 1u : 0u;
+  auto by_block = [&](const SrvGraph& G) { return !G.big || waiting >= G.burst; };
   bool big = ln.big;
-  if (s->lanes.size() < 2 && !s->pending.empty()) big = s->graphs[s->pending.front().gid].big;
+  if (s->lanes.size() < 2 && !s->pending.empty()) big = !by_block(s->graphs[s->pending.front().gid]);
   for (auto it = s->pending.begin();
        it != s->pending.end() && (int32_t)batch.size() < s->o.max_batch && !s->free_recs.empty();) {
     SrvQuery& q = *it;
     const SrvGraph& G = s->graphs[q.gid];
-    if (G.big != big) { ++it; continue; }
+    if (big ? !G.big : !by_block(G)) { ++it; continue; }
     q.bytes = slot_bytes(G.n, q.out_pred != nullptr);
     if (!s->alloc.alloc(q.bytes, &q.off)) break;   // HBM budget: wait for running queries to finish
     q.rec = s->free_recs.back();
@@ -844,6 +864,7 @@ b2_status srv_tune_graph(b2_server s, int32_t gid) {
     for (double sc : scales) {
       SrvGraph& G = s->graphs[gid];
       G.big = team == 1;
+      G.burst = kNoBurst;
       if (set_bucket_width(G, sc) != B2_SUCCESS) continue;
       double elapsed = 0.0;
       uint64_t done_q = 0;
@@ -877,6 +898,7 @@ b2_status srv_tune_graph(b2_server s, int32_t gid) {
   cudaFree(d_out);
   SrvGraph& G = s->graphs[gid];
   G.big = best_big;
+  G.burst = kNoBurst;   // the measured team, however many wait
   b2_status st2 = set_bucket_width(G, best_scale);
   G.tuned = status == B2_SUCCESS && st2 == B2_SUCCESS;
   return status != B2_SUCCESS ? status : st2;
@@ -1022,6 +1044,7 @@ extern "C" b2_status b2_server_add_graph(b2_server s, b2_graph g, int32_t* graph
   G.n = (uint32_t)g->n;
   G.isf = g->weight_type == B2_W_F32;
   G.big = G.n >= s->big_n || (s->o.big_vertices == 0 && g->m >= kBigEdges);
+  G.burst = G.big && G.n < s->big_n ? burst_of(g) : kNoBurst;
   G.tuned = false;
   b2_status st = set_bucket_width(G, s->o.delta_scale > 0 ? s->o.delta_scale : 4.0);
   if (st != B2_SUCCESS) return st;
