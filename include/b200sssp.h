@@ -237,6 +237,11 @@ void b2_sssp_opts_default(b2_sssp_opts* opts);
  * (ctypes, cgo): frees the callee-allocated SpGEMM outputs. */
 b2_status b2_device_free(void* d_ptr);
 b2_status b2_device_copy(void* d_dst, const void* d_src, size_t bytes, b2_stream stream);
+/* Sparse products and all-pairs calls take their scratch from a pool that keeps
+ * up to 4 GiB of a device between calls (b2_apsp_*: a matrix of up to 256 MiB).
+ * This waits for the current device and gives back to it what no call (and no plan
+ * that waits to be filled) is using. */
+b2_status b2_release_scratch(void);
 
 /* ---- resident graphs -------------------------------------------------- */
 b2_status b2_graph_create(const b2_csr* csr, b2_stream stream, b2_graph* out);
@@ -285,7 +290,9 @@ b2_status b2_minplus_gemm_i32(const int32_t* dA, const int32_t* dB, int32_t* dC,
                               b2_stream stream);
 /* All-pairs shortest paths by repeated squaring of an N x N matrix in place
  * (d_D must have a zero diagonal).  Stops early when a squaring changes
- * nothing.  *squarings_out = products computed. */
+ * nothing.  *squarings_out = products computed.  The second matrix comes from
+ * the library's scratch pool up to 256 MiB (b2_release_scratch), from cudaMalloc
+ * past that. */
 b2_status b2_apsp_f32(float* d_D, int32_t N, b2_stream stream, int32_t* squarings_out);
 b2_status b2_apsp_i32(int32_t* d_D, int32_t N, b2_stream stream, int32_t* squarings_out);
 /* Waits for `stream`, then returns B2_TIMEOUT if a min-plus product launched

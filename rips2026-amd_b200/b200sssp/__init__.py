@@ -332,4 +332,4 @@ def dist_to_numpy(dist, weight: str) -> np.ndarray:
 
 
 # min-plus entry points are defined in .minplus (imported lazily by users)
-from .minplus import minplus_gemm, apsp, minplus_spgemm  # noqa: E402
+from .minplus import minplus_gemm, apsp, minplus_spgemm, release_scratch  # noqa: E402

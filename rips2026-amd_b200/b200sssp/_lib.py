@@ -100,6 +100,7 @@ _SIGS = {
     "b2_sssp_opts_default": (None, [C.POINTER(Opts)]),
     "b2_device_free": (C.c_int, [_P]),
     "b2_device_copy": (C.c_int, [_P, _P, C.c_size_t, _P]),
+    "b2_release_scratch": (C.c_int, []),
     "b2_graph_create": (C.c_int, [C.POINTER(CSR), _P, C.POINTER(_P)]),
     "b2_graph_destroy": (C.c_int, [_P]),
     "b2_graph_info_get": (C.c_int, [_P, C.POINTER(GraphInfo)]),

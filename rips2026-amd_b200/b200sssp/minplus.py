@@ -69,6 +69,12 @@ def apsp(D, stream=None) -> int:
     return n.value
 
 
+def release_scratch() -> None:
+    """Give the scratch memory that sparse products and apsp keep between calls
+    (up to 4 GiB) back to the current device."""
+    check(lib().b2_release_scratch(), "release_scratch")
+
+
 def _csr_view(rowptr, colind, values, ncols):
     torch = _torch()
     c = _lib.CSR()

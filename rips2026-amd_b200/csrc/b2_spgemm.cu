@@ -1216,6 +1216,13 @@ b2_status spgemm(const b2_csr* A, const b2_csr* B, int64_t** dC_rowptr, int32_t*
 }  // namespace
 }  // namespace b2
 
+extern "C" b2_status b2_release_scratch(void) {
+  cudaMemPool_t pool;
+  B2_CUDA_TRY(b2::scratch_pool(&pool));
+  B2_CUDA_TRY(cudaDeviceSynchronize());   // releases queued on streams are made
+  return b2::from_cuda(cudaMemPoolTrimTo(pool, 0));
+}
+
 extern "C" b2_status b2_minplus_spgemm_f32(const b2_csr* A, const b2_csr* B, int64_t** dC_rowptr,
                                            int32_t** dC_colind, float** dC_values, int64_t* hC_nnz,
                                            b2_stream stream) {
