@@ -315,9 +315,10 @@ b2_status b2_minplus_status(b2_stream stream);
  * captured. */
 b2_status b2_apsp_f32_noalloc(float* d_D, int32_t N, b2_stream stream, int32_t* squarings_out);
 /* Sustained (min,+) pairs per second of this GPU's CUDA cores, measured by a
- * register-only kernel of the same instruction mix as the GEMM inner loop
- * (int32: DPX add-min; fp32: FADD + three-input min).  The roofline
- * denominator for the min-plus GEMM.  Synchronous, current device. */
+ * register-only kernel (int32: the GEMM's DPX add-min; fp32: two additions and a
+ * three-input min per two pairs, which runs faster in registers than the packed
+ * additions of the GEMM).  The roofline denominator for the min-plus GEMM.
+ * Synchronous, current device. */
 b2_status b2_minplus_calibrate(int32_t is_float, double* pairs_per_second);
 
 /* CSR x CSR min-plus.  Outputs are cudaMalloc'd by the callee and owned by

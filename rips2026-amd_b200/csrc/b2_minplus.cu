@@ -905,14 +905,15 @@ b2_status apsp(T* D, int N, b2_stream s, int32_t* squarings) {
 }
 
 // ---- ALU peak calibration (roofline denominator for min-plus) -------------
-// The GEMMs' instruction mix on registers only: an 8 x 8 accumulator tile
-// per thread updated per k step exactly like mma_tile (int32: one
-// __viaddmin_s32 per pair; fp32: two FADD and one 3-input min per two pairs),
-// with no shared-memory or global traffic.  The A operand of row i at step k
-// is an accumulator of that row (acc[i][(i + k) & 7], a register chosen at
-// compile time), so every sum is a new value and no sum can be folded or
-// shared between pairs; B is 8 (16 for fp32) runtime constants.  The pair
-// count over the device time is the instruction-issue ceiling of the mix.
+// Updates of an 8 x 8 accumulator tile per thread on registers only (int32: the
+// GEMMs' one __viaddmin_s32 per pair; fp32: two additions and one three-input min
+// per two pairs), with no shared-memory or global traffic.  The A operand of row i
+// at step k is an accumulator of that row (acc[i][(i + k) & 7], a register chosen at
+// compile time), so every sum is a new value and no sum can be folded or shared
+// between pairs; B is 8 (16 for fp32) runtime constants.  fp32 reads 21.5 T pairs/s;
+// the packed addition and three-input min of k_minplus_cp read 18.7 in registers,
+// in the order that the compiler gives them, and loops whose additions share an
+// operand reached 26.8, so this is a measure, not a bound.
 template <typename T>
 __global__ void __launch_bounds__(256) k_calibrate(int iters, T seed, T step, T* sink) {
   T acc[8][8];
