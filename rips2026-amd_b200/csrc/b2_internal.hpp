@@ -54,7 +54,6 @@ struct PhaseRec {
   uint32_t push_q;      // near queue receiving same-bucket pushes
   uint32_t stamp;       // dedup stamp for those pushes
   uint32_t hub_in;      // hub list consumed this phase
-  uint32_t hub_in_count;
   uint32_t hub_in_chunks;
   uint32_t hub_out;     // hub list produced this phase
   uint32_t cur;         // current bucket (delta)
@@ -121,9 +120,7 @@ enum QueueId : uint32_t {
 // atomics on one line queue up in one L2 slice, and a warp that polls or reads a
 // word waits behind those on its neighbours.
 struct alignas(128) Control {
-  // grid barrier (must stay first; see b2_common.cuh GridBarrier)
-  uint32_t bar_arrive;
-  uint32_t bar_gen;
+  uint32_t bar_arrive;     // arrivals at the grid barriers so far
   uint32_t error;
   uint32_t error_site;
   PhaseRec rec;            // the record that ended the solve (read by the host; zero if every block

@@ -138,50 +138,48 @@ __device__ __forceinline__ void tile_coords(int tiles_m, int tiles_n, int& tm, i
 // Compute one k-tile held in shared memory (A swizzled, B plain).  A is read
 // as k-pairs (8-byte loads inside the swizzled 16-byte chunk), B as two
 // 16-byte vectors per k row.
-template <typename T>
-__device__ __forceinline__ void load_b8(const T* Bs, int k, int tx, T (&b)[8]) {
+__device__ __forceinline__ void load_b8(const int* Bs, int k, int tx, int (&b)[8]) {
   const int4 p0 = *reinterpret_cast<const int4*>(Bs + k * BN + tx * 4);
   const int4 p1 = *reinterpret_cast<const int4*>(Bs + k * BN + 64 + tx * 4);
   const int pp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
-  for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const T*>(&pp[j]);
+  for (int j = 0; j < 8; ++j) b[j] = pp[j];
 }
 
-template <typename T, bool FULL>
-__device__ __forceinline__ void mma_tile(const T* __restrict__ As, const T* __restrict__ Bs, int kvalid, int tx,
-                                         int ty, T (&acc)[8][8]) {
+template <bool FULL>
+__device__ __forceinline__ void mma_tile(const int* __restrict__ As, const int* __restrict__ Bs, int kvalid, int tx,
+                                         int ty, int (&acc)[8][8]) {
   const int sw = ty & 7;
 #pragma unroll
   for (int k = 0; k < BK; k += 2) {
     if (!FULL && k >= kvalid) break;
-    T a0[8], a1[8];
+    int a0[8], a1[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int r = ty + 16 * i;
       const int2 v = *reinterpret_cast<const int2*>(As + r * BK + (((k >> 2) ^ sw) << 2) + (k & 2));
-      a0[i] = *reinterpret_cast<const T*>(&v.x);
-      a1[i] = *reinterpret_cast<const T*>(&v.y);
+      a0[i] = v.x;
+      a1[i] = v.y;
     }
-    T b0[8], b1[8];
-    load_b8<T>(Bs, k, tx, b0);
+    int b0[8], b1[8];
+    load_b8(Bs, k, tx, b0);
     if (FULL || k + 1 < kvalid) {
-      load_b8<T>(Bs, k + 1, tx, b1);
+      load_b8(Bs, k + 1, tx, b1);
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = MP<T>::step2(acc[i][j], a0[i], b0[j], a1[i], b1[j]);
+        for (int j = 0; j < 8; ++j) acc[i][j] = MP<int>::step2(acc[i][j], a0[i], b0[j], a1[i], b1[j]);
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = MP<T>::step1(acc[i][j], a0[i], b0[j]);
+        for (int j = 0; j < 8; ++j) acc[i][j] = MP<int>::step1(acc[i][j], a0[i], b0[j]);
     }
   }
 }
 
-template <typename T>
-__device__ __forceinline__ void store_tile(T* C, int M, int N, int ldc, int m0, int n0, int tx, int ty,
-                                           const T (&acc)[8][8], const T* Aold, int lda, uint32_t* changed) {
+__device__ __forceinline__ void store_tile(int* C, int M, int N, int ldc, int m0, int n0, int tx, int ty,
+                                           const int (&acc)[8][8], const int* Aold, int lda, uint32_t* changed) {
   bool diff = false;
   const bool vec = ((ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
 #pragma unroll
@@ -193,10 +191,10 @@ __device__ __forceinline__ void store_tile(T* C, int M, int N, int ldc, int m0, 
       const int c0 = n0 + h * 64 + tx * 4;
       if (vec && c0 + 3 < N) {
         int4 v;
-        v.x = *reinterpret_cast<const int*>(&acc[i][h * 4 + 0]);
-        v.y = *reinterpret_cast<const int*>(&acc[i][h * 4 + 1]);
-        v.z = *reinterpret_cast<const int*>(&acc[i][h * 4 + 2]);
-        v.w = *reinterpret_cast<const int*>(&acc[i][h * 4 + 3]);
+        v.x = acc[i][h * 4 + 0];
+        v.y = acc[i][h * 4 + 1];
+        v.z = acc[i][h * 4 + 2];
+        v.w = acc[i][h * 4 + 3];
         *reinterpret_cast<int4*>(C + (size_t)r * ldc + c0) = v;
       } else {
 #pragma unroll
@@ -207,8 +205,8 @@ __device__ __forceinline__ void store_tile(T* C, int M, int N, int ldc, int m0, 
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           if (c0 + q < N) {
-            const T o = Aold[(size_t)r * lda + c0 + q];
-            diff |= (*reinterpret_cast<const int*>(&o) != *reinterpret_cast<const int*>(&acc[i][h * 4 + q]));
+            const int o = Aold[(size_t)r * lda + c0 + q];
+            diff |= (o != acc[i][h * 4 + q]);
           }
       }
     }
@@ -220,15 +218,14 @@ __device__ __forceinline__ void store_tile(T* C, int M, int N, int ldc, int m0, 
 // *changed (APSP squaring, where C <= A elementwise because diag(A) = 0).
 // `previous` (nullable): the last squaring's word; where it is 0 that squaring
 // changed nothing and there is nothing left to do.
-template <typename T>
 __global__ void __launch_bounds__(NT, 2)
-    k_minplus_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, T* C, int M,
-                  int N, int K, int ldc, const T* Aold, int lda, uint32_t* changed, const uint32_t* previous) {
+    k_minplus_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int* C, int M,
+                  int N, int K, int ldc, const int* Aold, int lda, uint32_t* changed, const uint32_t* previous) {
   if (previous && *previous == 0u) return;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  T* As = reinterpret_cast<T*>(base);
-  T* Bs = As + STAGES * A_TILE;
+  int* As = reinterpret_cast<int*>(base);
+  int* Bs = As + STAGES * A_TILE;
   uint64_t* full = reinterpret_cast<uint64_t*>(Bs + STAGES * B_TILE);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   int tm, tn;
@@ -242,31 +239,31 @@ __global__ void __launch_bounds__(NT, 2)
   __syncthreads();
   if (tid == 0) {
     for (int s = 0; s < STAGES && s < KT; ++s) {
-      mbar_expect_tx(&full[s], (A_TILE + B_TILE) * sizeof(T));
+      mbar_expect_tx(&full[s], (A_TILE + B_TILE) * sizeof(int));
       tma_load_2d(As + s * A_TILE, &mapA, s * BK, m0, &full[s]);
       tma_load_2d(Bs + s * B_TILE, &mapB, n0, s * BK, &full[s]);
     }
   }
-  T acc[8][8];
+  int acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = MP<T>::init();
+    for (int j = 0; j < 8; ++j) acc[i][j] = MP<int>::init();
   for (int kt = 0; kt < KT; ++kt) {
     const int s = kt % STAGES;
     mbar_wait(&full[s], (kt / STAGES) & 1);
     const int kvalid = min(BK, K - kt * BK);
-    if (kvalid == BK) mma_tile<T, true>(As + s * A_TILE, Bs + s * B_TILE, BK, tx, ty, acc);
-    else mma_tile<T, false>(As + s * A_TILE, Bs + s * B_TILE, kvalid, tx, ty, acc);
+    if (kvalid == BK) mma_tile<true>(As + s * A_TILE, Bs + s * B_TILE, BK, tx, ty, acc);
+    else mma_tile<false>(As + s * A_TILE, Bs + s * B_TILE, kvalid, tx, ty, acc);
     __syncthreads();   // every thread is done with stage s
     if (tid == 0 && kt + STAGES < KT) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_expect_tx(&full[s], (A_TILE + B_TILE) * sizeof(T));
+      mbar_expect_tx(&full[s], (A_TILE + B_TILE) * sizeof(int));
       tma_load_2d(As + s * A_TILE, &mapA, (kt + STAGES) * BK, m0, &full[s]);
       tma_load_2d(Bs + s * B_TILE, &mapB, n0, (kt + STAGES) * BK, &full[s]);
     }
   }
-  store_tile<T>(C, M, N, ldc, m0, n0, tx, ty, acc, Aold, lda, changed);
+  store_tile(C, M, N, ldc, m0, n0, tx, ty, acc, Aold, lda, changed);
 }
 
 // ---- cp.async kernel --------------------------------------------------------
@@ -543,20 +540,17 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-template <typename T>
-bool make_map(CUtensorMap* map, const T* ptr, int rows, int cols, int ld, int box_cols, int box_rows, bool swz) {
+bool make_map(CUtensorMap* map, const int* ptr, int rows, int cols, int ld, int box_cols, int box_rows, bool swz) {
   auto fn = encode_fn();
   if (!fn) return false;
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15) || ((size_t)ld * sizeof(T)) % 16) return false;
+  if ((reinterpret_cast<uintptr_t>(ptr) & 15) || ((size_t)ld * sizeof(int)) % 16) return false;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(T)};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(int)};
   cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  const CUtensorMapDataType dt =
-      sizeof(T) == 4 && std::is_same<T, float>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_INT32;
-  CUresult r = fn(map, dt, 2, const_cast<T*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  swz ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<int*>(ptr), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swz ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
@@ -636,7 +630,7 @@ cudaError_t ensure_kernels(const Capacity** cap) {
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess && std::is_same<T, int>::value)
-      e = cudaFuncSetAttribute(k_minplus_tma<int>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem);
+      e = cudaFuncSetAttribute(k_minplus_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem);
     if (e == cudaSuccess) e = prepare_cp<T, Big>(sms, c.big);
     if (e == cudaSuccess) e = prepare_cp<T, Small>(sms, c.small);
     if (e != cudaSuccess) return e;
@@ -771,18 +765,13 @@ bool tma_can_read(const T* p, int ld) {
 cudaError_t launch_tma(const int* A, const int* B, int* C, int M, int N, int K, int lda, int ldb, int ldc,
                        cudaStream_t st, const int* Aold, uint32_t* changed, const uint32_t* previous, bool* launched) {
   CUtensorMap ma, mb;
-  *launched = make_map<int>(&ma, A, M, K, lda, BK, BM, true) && make_map<int>(&mb, B, K, N, ldb, BN, BK, false);
+  *launched = make_map(&ma, A, M, K, lda, BK, BM, true) && make_map(&mb, B, K, N, ldb, BN, BK, false);
   if (!*launched) return cudaSuccess;
   const cudaError_t e = mark_tma_used();
   if (e != cudaSuccess) return e;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  k_minplus_tma<int><<<tiles, NT, kTmaSmem, st>>>(ma, mb, C, M, N, K, ldc, Aold, lda, changed, previous);
+  k_minplus_tma<<<tiles, NT, kTmaSmem, st>>>(ma, mb, C, M, N, K, ldc, Aold, lda, changed, previous);
   return cudaGetLastError();
-}
-cudaError_t launch_tma(const float*, const float*, float*, int, int, int, int, int, int, cudaStream_t, const float*,
-                       uint32_t*, const uint32_t*, bool* launched) {
-  *launched = false;   // pick_shape never asks for it
-  return cudaSuccess;
 }
 
 template <typename T>
@@ -794,11 +783,13 @@ cudaError_t launch_minplus(const T* A, const T* B, T* C, int M, int N, int K, in
   if (e != cudaSuccess) return e;
   const bool a_vec = tma_can_read(A, lda);
   Shape sh = pick_shape(M, N, K, *cap, a_vec && tma_can_read(B, ldb), std::is_same<T, int>::value);
-  if (sh.kernel == kTma) {
-    bool launched = false;
-    e = launch_tma(A, B, C, M, N, K, lda, ldb, ldc, st, Aold, changed, previous, &launched);
-    if (launched || e != cudaSuccess) return e;
-    sh = Shape{kBig, 1};   // no tensor map (driver entry point missing)
+  if constexpr (std::is_same<T, int>::value) {
+    if (sh.kernel == kTma) {
+      bool launched = false;
+      e = launch_tma(A, B, C, M, N, K, lda, ldb, ldc, st, Aold, changed, previous, &launched);
+      if (launched || e != cudaSuccess) return e;
+      sh = Shape{kBig, 1};   // no tensor map (driver entry point missing)
+    }
   }
   Operands<T> P;
   P.A = A;

@@ -108,7 +108,6 @@ struct SLabel<false> {
   __device__ static T inf() { return kInfKey; }
   __device__ static T make(uint32_t key, uint32_t) { return key; }
   __device__ static uint32_t key(T x) { return x; }
-  __device__ static T atomic_min(T* a, T v) { return atomicMin(a, v); }
 };
 template <>
 struct SLabel<true> {
@@ -116,7 +115,6 @@ struct SLabel<true> {
   __device__ static T inf() { return ~0ull; }
   __device__ static T make(uint32_t key, uint32_t p) { return ((T)key << 32) | p; }
   __device__ static uint32_t key(T x) { return (uint32_t)(x >> 32); }
-  __device__ static T atomic_min(T* a, T v) { return atomicMin(a, v); }
 };
 
 // Bucket of a label key; kSNone for unreached.  Buckets only order the work
@@ -140,7 +138,6 @@ struct SShared {
   uint32_t nhub[3];    // long rows of the frontier
   uint32_t fcount;     // far pile entries
   uint32_t fnext;      // kept far entries during a split
-  uint32_t cur;        // current bucket
   uint32_t minb;       // split: smallest live bucket
   uint32_t stop[3];    // budget verdict of a phase (0: go on)
   uint32_t hubs[2][kHubListCap];   // by parity of the phase

@@ -80,7 +80,7 @@ constexpr int kThreads = 512;
 #ifndef B2_HUB_UNROLL
 #define B2_HUB_UNROLL 4
 #endif
-constexpr int kUnroll = B2_UNROLL;   // edge slots per lane per step
+constexpr int kUnroll = B2_UNROLL;   // edge slots per lane per step (hub chunks: B2_HUB_UNROLL)
 
 struct Params {
   uint32_t n;
@@ -168,6 +168,8 @@ __device__ __forceinline__ void set_error(const Params& P, uint32_t code, uint32
 // happen when a buffer passes half full and at the end of every phase.
 constexpr int kWarpsPerBlock = kThreads / 32;
 constexpr uint32_t kNearBuf = 256, kFarBuf = 256, kSlotBuf = 256, kMemBuf = 128;
+static_assert(32 * kUnroll <= kNearBuf / 2 && 32 * B2_HUB_UNROLL <= kNearBuf / 2,
+              "a step's pushes fit a buffer that is flushed past its half");
 constexpr uint32_t kDenseSpan = 256;   // vertices per sweep work item (8 per lane)
 constexpr uint32_t kListBuf = kDenseSpan + 32;   // one span's vertices + fewer than 32 carried
 constexpr uint32_t kStageWords = kNearBuf + kFarBuf + 2 * kSlotBuf + kMemBuf + kListBuf + kRing;
@@ -1028,7 +1030,6 @@ __device__ __noinline__ void manager_bf(const Params& P, const PhaseRec& r, cons
   nx.fcount = nn;
   nx.push_q = r.push_q ^ 1u;
   nx.hub_in = r.hub_out;
-  nx.hub_in_count = hch;
   nx.hub_in_chunks = hch;
   nx.hub_out = r.hub_out ^ 1u;
   nx.aux = r.iter >= P.max_iters ? 1u : 0u;
@@ -1093,7 +1094,6 @@ __device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, M
     const uint32_t hch = m.hub[r.hub_out & 1];
     const uint32_t nn = m.near[push_q & 1];
     nx.hub_in = r.hub_out;
-    nx.hub_in_count = hch;
     nx.hub_in_chunks = hch;
     nx.hub_out = r.hub_out ^ 1u;
     if (heavy) {
@@ -1136,7 +1136,6 @@ __device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, M
           nx.fq = kQNone;
           nx.fcount = P.n;
           nx.hub_in_chunks = 0;
-          nx.hub_in_count = 0;
         } else {
           nx.kind = kPhaseProcess;
           nx.fq = kQMembers;
@@ -1173,7 +1172,6 @@ __device__ __noinline__ void manager_delta(const Params& P, const PhaseRec& r, M
   nx.hround = P.phase_base + nx.phase;
   nx.far_sel = far_sel;
   nx.hub_in = r.hub_out;
-  nx.hub_in_count = 0;
   nx.hub_in_chunks = 0;
   nx.hub_out = r.hub_out ^ 1u;
   if (found >= 0) {
