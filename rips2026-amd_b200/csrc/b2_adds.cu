@@ -71,14 +71,19 @@ constexpr uint32_t kNotQueued = 0xFFFFFFFFu;   // qb[v]: not waiting in any buck
 constexpr uint32_t kGrab = 32;                 // entries a warp takes from its block's pool (one per lane)
 // Entries a block claims from a bucket at once: its share of the bucket's
 // unclaimed entries, but at most kBlockClaimMax and at least about
-// kBlockClaimEdges edges' worth (64 to kBlockClaimMax entries).  Claims are
-// compare-and-swaps of one word per bucket, so many small ones cost their square
-// (of n blocks that try, one succeeds at a time), and fewer than 512 entries
-// leave some of a block's 16 warps without a grab; but large claims of long rows
-// keep the other blocks idle.  With 64 / 128 / 256 / 512 / 1024 entries: grid
-// 900 x 1000 4.25 / 2.99 / 2.42 / 2.02 / 1.59 ms, ER-300000 of degree 12 2.30 /
-// 2.08 / 1.53 / 1.11 / 1.03, RMAT-18 2.04 / 1.53 / 1.29 / 1.27 / 1.23, RMAT-20
-// (mean degree 30) 3.7 / 3.6 / 4.1 / 4.8 / 5.2.
+// kBlockClaimEdges edges' worth (kBlockClaimMin to kBlockClaimMax entries).  Claims
+// are compare-and-swaps of one word per bucket, so many small ones cost their square
+// (of n blocks that try, one succeeds at a time), and fewer than 512 entries leave
+// some of a block's 16 warps without a grab; but large claims of long rows keep the
+// other blocks idle.  At the default width, 64 entries always / this rule / twice
+// its edges (uint32, mean of 6 sources): RMAT-14 0.42 / 0.35 / 0.33 ms, RMAT-16 0.95
+// / 0.69 / 0.55, RMAT-18 1.61 / 1.45 / 1.27, RMAT-19 2.41 / 2.14 / 2.35, RMAT-20
+// 3.56 / 3.41 / 3.85, ER-300000 of degree 12 2.30 / 1.52 / 1.19, grid 900 x 1000
+// 3.66 / 1.81 / 1.74.  The mean degree is a rough guide: smaller and more even
+// graphs would take larger claims.  Large uneven graphs whose buckets are narrower
+// than the Near-Far width keep kBlockClaimMin (a quarter of it: RMAT-19 2.47 ms with
+// 64 entries, 3.07 with 128; RMAT-20 3.77 and 4.75).
+constexpr uint32_t kBlockClaimMin = 64;
 constexpr uint32_t kBlockClaimMax = 1024;
 constexpr double kBlockClaimEdges = 4096.0;
 constexpr uint32_t kChunkEdges = 256;          // edges per hub chunk
@@ -1173,8 +1178,14 @@ b2_status run_adds(b2_graph g, uint32_t source, void* d_dist, int32_t* d_pred, c
   else grid = pred ? adds_grid<WU32, true>() : adds_grid<WU32, false>();
   if (o.grid_blocks && (int)o.grid_blocks < grid) grid = (int)o.grid_blocks;
   if (grid <= 0) return B2_CUDA_ERROR;
-  P.claim_min = (uint32_t)std::min<double>(
-      kBlockClaimMax, std::max(64.0, std::floor(kBlockClaimEdges / std::max(1.0, g->mean_degree) / 32.0) * 32.0));
+  P.claim_min = kBlockClaimMin;
+  double near_far = 0.0;
+  b2_delta_heuristic(g, 16.0, &near_far);
+  const bool uneven = (double)g->max_degree >= 64.0 * g->mean_degree;
+  if (!(uneven && g->n >= (1 << 19) && delta < 0.75 * near_far))
+    P.claim_min = (uint32_t)std::min<double>(
+        kBlockClaimMax,
+        std::max((double)kBlockClaimMin, std::floor(kBlockClaimEdges / std::max(1.0, g->mean_degree) / 32.0) * 32.0));
   P.adapt_cap = (uint32_t)grid * (kAThreads / 32) * kGrab;   // one grab per warp fills the grid
   if (stats) {
     memset(stats, 0, sizeof(*stats));

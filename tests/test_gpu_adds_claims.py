@@ -1,0 +1,23 @@
+"""GPU ADDS with buckets narrower and wider than the default on large uneven graphs: right, and the
+narrow ones not held up by large claims."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("scale,delta_scale", [(18, 4.0), (19, 4.0), (19, 16.0), (19, 64.0)])
+def test_narrow_buckets(b2, orc, cuda, scale, delta_scale):
+    h = b2.gen_rmat(scale, 16, seed=1)
+    g = b2.Graph.from_host(h, "u32")
+    source = int(h.colind[12345])
+    ref = orc.dijkstra(h.rowptr, h.colind, h.weights, source)
+    d, p, _ = g.sssp(source, method="adds", pred=True, delta_scale=delta_scale)
+    assert np.array_equal(d.cpu().numpy().view(np.uint32), ref)
+    assert orc.validate_spt(h.rowptr, h.colind, h.weights, source, ref, p.cpu().numpy()) == 0
+    if scale == 19 and delta_scale == 4.0:
+        # a quarter of the default width against half of it: 1.04, and 1.27 with claims of 128 entries
+        best = {w: min(g.sssp(source, method="adds", delta_scale=w)[2]["kernel_ms"] for _ in range(15))
+                for w in (4.0, 8.0)}
+        assert best[4.0] < 1.15 * best[8.0], best
+    g.close()
