@@ -326,7 +326,8 @@ b2_status b2_minplus_calibrate(int32_t is_float, double* pairs_per_second);
  * candidates are skipped; duplicates are min-reduced.  Output columns are
  * sorted within each row.  A, B: on_device = 1, rowptr_bits = 64.  A row of A
  * with more than 2^32 - 1025 candidates (entries of B met, absent ones and
- * duplicates included) returns B2_NOT_SUPPORTED. */
+ * duplicates included) returns B2_NOT_SUPPORTED.  Where a column meets zeros of both
+ * signs, either is returned. */
 b2_status b2_minplus_spgemm_f32(const b2_csr* A, const b2_csr* B, int64_t** dC_rowptr,
                                 int32_t** dC_colind, float** dC_values, int64_t* hC_nnz,
                                 b2_stream stream);
