@@ -122,6 +122,14 @@ __device__ __forceinline__ unsigned long long atom_min_if(bool p, unsigned long 
                : "+l"(old) : "l"(a), "l"(x), "r"((uint32_t)p) : "memory");
   return old;
 }
+__device__ __forceinline__ void red_min_if(bool p, uint32_t* a, uint32_t x) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.global.min.u32 [%0], %1;\n\t}"
+               ::"l"(a), "r"(x), "r"((uint32_t)p) : "memory");
+}
+__device__ __forceinline__ void red_min_if(bool p, unsigned long long* a, unsigned long long x) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.global.min.u64 [%0], %1;\n\t}"
+               ::"l"(a), "l"(x), "r"((uint32_t)p) : "memory");
+}
 __device__ __forceinline__ uint32_t ld_cg_if(bool p, const uint32_t* a, uint32_t dflt) {
   uint32_t v = dflt;
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.cg.u32 %0, [%1];\n\t}"

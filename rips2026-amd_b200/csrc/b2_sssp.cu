@@ -69,7 +69,9 @@
 
 namespace b2 {
 
-enum Mode : int { kModeBF = 0, kModeDelta = 1 };
+// kModeBFProbe: Bellman-Ford with predecessors that may end with the negative-cycle probe
+enum Mode : int { kModeBF = 0, kModeDelta = 1, kModeBFProbe = 2 };
+__host__ __device__ constexpr bool is_bf(int mode) { return mode != kModeDelta; }
 constexpr int kThreads = 512;
 #ifndef B2_UNROLL
 #define B2_UNROLL 4
@@ -241,7 +243,7 @@ template <int MODE>
 __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, WarpQ& q, bool force) {
   const uint32_t nn = (force || q.nn > kNearBuf / 2) ? q.nn : 0u;
   uint32_t nf = 0, nm = 0, ns = 0;
-  if (MODE != kModeBF) {
+  if (!is_bf(MODE)) {
     nf = (force || q.nf > kFarBuf / 2) ? q.nf : 0u;
     nm = (force || q.nm > kMemBuf / 2) ? q.nm : 0u;
     ns = (force || q.ns > kSlotBuf / 2) ? q.ns : 0u;
@@ -256,7 +258,7 @@ __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, Wa
                     : lane == 2 ? &c->members_count
                                 : &c->slot_count[lane & (kRing - 1)];
   uint32_t* hist = q.histb();
-  if (MODE != kModeBF && ns) {
+  if (!is_bf(MODE) && ns) {
     if (lane < (uint32_t)kRing) hist[lane] = 0;
     __syncwarp();
     for (uint32_t i = lane; i < ns; i += 32) {   // slot -> (slot, rank within it)
@@ -272,7 +274,7 @@ __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, Wa
   if (__any_sync(0xffffffffu, over)) {
     if (over) set_error(P, kErrQueueOverflow, lane < 3 ? 11 + (lane ? 1 + lane : 0) : 12);
   } else {
-    if (MODE != kModeBF && ns) {
+    if (!is_bf(MODE) && ns) {
       __syncwarp();
       if (lane >= 16) hist[lane - 16] = base;
       __syncwarp();
@@ -283,7 +285,7 @@ __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, Wa
     }
     const uint32_t bn = __shfl_sync(0xffffffffu, base, 0);
     for (uint32_t i = lane; i < nn; i += 32) queue_ptr(P, R.push_q)[bn + i] = q.nearb()[i];
-    if (MODE == kModeBF && P.has_hubs) {
+    if (is_bf(MODE) && P.has_hubs) {
       for (uint32_t i0 = 0; i0 < nn; i0 += 32) {
         const bool in = i0 + lane < nn;
         const uint32_t v = in ? q.nearb()[i0 + lane] : 0u;
@@ -292,7 +294,7 @@ __device__ __forceinline__ void flush_all(const Params& P, const PhaseRec& R, Wa
         append_hubs(P, R, v, deg, deg >= P.hub_degree);
       }
     }
-    if (MODE != kModeBF) {
+    if (!is_bf(MODE)) {
       const uint32_t bf = __shfl_sync(0xffffffffu, base, 1), bm = __shfl_sync(0xffffffffu, base, 2);
       for (uint32_t i = lane; i < nf; i += 32) queue_ptr(P, kQFar0 + R.far_sel)[bf + i] = q.farb()[i];
       for (uint32_t i = lane; i < nm; i += 32) queue_ptr(P, kQMembers)[bm + i] = q.memb()[i];
@@ -397,7 +399,7 @@ __device__ __forceinline__ void route_batch(const Params& P, const PhaseRec& R, 
       stage(t.q.nearb(), t.q.nn, want, v);
       t.pushes += want ? 1 : 0;
     }
-    if (MODE != kModeBF) {
+    if (!is_bf(MODE)) {
       if (__any_sync(0xffffffffu, cls[q] == 2)) {
         const bool want = cls[q] == 2 && obuck[q] > b[q];
         const uint32_t bal = __ballot_sync(0xffffffffu, want);
@@ -433,9 +435,12 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
   uint32_t cand[U];
   typename L::T cur[U], old[U];
   bool imp[U];
-  if (MODE == kModeBF) {
+  if (is_bf(MODE)) {
     typename L::T* rd = (typename L::T*)bf_read(P, R);
     typename L::T* wr = (typename L::T*)bf_write(P, R);
+    // the written array's tie by the label atomic or beside it: which of the two is
+    // faster differs by the weight type (1 to 3 % either way)
+    constexpr bool kTieByAtomic = PRED && W::kFloat && MODE != kModeBFProbe;
 #pragma unroll
     for (int q = 0; q < U; ++q) {
       cand[q] = act[q] ? W::extend(dsrc[q], ed[q].y) : kInfKey;
@@ -444,17 +449,24 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
 #pragma unroll
     for (int q = 0; q < U; ++q) {
       const typename L::T cw = L::make(cand[q], src[q]);
-      old[q] = atom_min_keep_if(cand[q] < L::key(cur[q]), wr + ed[q].x, cw, t.keep, (typename L::T)0);
-      if (PRED && cand[q] == L::key(cur[q]) && cw < cur[q]) {
-        // a smaller predecessor at an equal distance: the vertex is not expanded
-        // again, so both arrays take it.  A solve that may end with the probe keeps
-        // it apart: a probe's output has the predecessors of each vertex's last
-        // improvement, a converged one's the smallest of all.
-        if (P.ties) {
-          atomicMin(P.ties + ed[q].x, cw);
-        } else {
-          atomicMin(rd + ed[q].x, cw);
-          atomicMin(wr + ed[q].x, cw);
+      // With predecessors a smaller one at an equal distance counts too, but the
+      // vertex is not expanded again, so both arrays take it.  A solve that may end
+      // with the probe keeps it apart: a probe's output has the predecessors of each
+      // vertex's last improvement, a converged one's the smallest of all.
+      // (Predicated: branches here cost RMAT-22 with predecessors 5 %.)
+      if constexpr (kTieByAtomic) {
+        old[q] = atom_min_keep_if(cw < cur[q], wr + ed[q].x, cw, t.keep, (typename L::T)0);
+        red_min_if(cw < cur[q] && !(cand[q] < L::key(cur[q])), rd + ed[q].x, cw);
+      } else {
+        old[q] = atom_min_keep_if(cand[q] < L::key(cur[q]), wr + ed[q].x, cw, t.keep, (typename L::T)0);
+        if (PRED) {
+          const bool tie = cand[q] == L::key(cur[q]) && cw < cur[q];
+          if (MODE == kModeBFProbe) {
+            red_min_if(tie, (typename L::T*)P.ties + ed[q].x, cw);
+          } else {
+            red_min_if(tie, rd + ed[q].x, cw);
+            red_min_if(tie, wr + ed[q].x, cw);
+          }
         }
       }
     }
@@ -462,7 +474,8 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
     for (int q = 0; q < U; ++q) {
       imp[q] = cand[q] < L::key(cur[q]) && L::key(old[q]) >= L::key(cur[q]);   // first below the read label
       t.edges += act[q] ? 1 : 0;
-      t.impr += cand[q] < L::key(old[q]) ? 1 : 0;   // (not issued: old = 0)
+      if constexpr (kTieByAtomic) t.impr += cand[q] < L::key(cur[q]) && cand[q] < L::key(old[q]) ? 1 : 0;
+      else t.impr += cand[q] < L::key(old[q]) ? 1 : 0;   // (not issued: old = 0)
       t.pushes += imp[q] ? 1 : 0;
       stage(t.q.nearb(), t.q.nn, imp[q], ed[q].x);
     }
@@ -495,7 +508,7 @@ __device__ __forceinline__ void relax_batch(const Params& P, const PhaseRec& R, 
 template <class W, bool PRED, int MODE>
 __device__ __forceinline__ uint32_t src_key(const Params& P, const PhaseRec& R, uint32_t v) {
   using L = Label<PRED>;
-  const typename L::T* lab = (const typename L::T*)(MODE == kModeBF ? bf_read(P, R) : P.dist);
+  const typename L::T* lab = (const typename L::T*)(is_bf(MODE) ? bf_read(P, R) : P.dist);
   return L::key(ldcg(lab + v));
 }
 
@@ -566,7 +579,7 @@ __device__ __forceinline__ void expand_vertices(const Params& P, const PhaseRec&
     // the row bounds do not depend on the label: both loads go out together
     // (one dependent memory round trip less per item)
     phase_range(P, R, v, lo, hi, has_heavy, &row_end);
-    if (MODE == kModeBF) {   // carry the label over
+    if (is_bf(MODE)) {   // carry the label over
       const typename Label<PRED>::T w = ldcg((const typename Label<PRED>::T*)bf_read(P, R) + v);
       atomicMin((typename Label<PRED>::T*)bf_write(P, R) + v, w);
       du = Label<PRED>::key(w);
@@ -950,7 +963,7 @@ __device__ void manager_init(const Params& P, PhaseRec& r) {
   // candidate can ever replace it; the output maps pred[source] to -1.
   const uint32_t zk = P.is_float ? f32_to_key(0.0f) : 0u;
   lab[P.source] = L::make(zk, 0u);
-  if (MODE == kModeBF) ((typename L::T*)P.dist_cur)[P.source] = L::make(zk, 0u);
+  if (is_bf(MODE)) ((typename L::T*)P.dist_cur)[P.source] = L::make(zk, 0u);
   queue_ptr(P, kQNear0)[0] = P.source;
   c->near_count[0] = 1;
   c->near_count[1] = 0;
@@ -968,7 +981,7 @@ __device__ void manager_init(const Params& P, PhaseRec& r) {
   r.hround = P.phase_base + 1;
   r.hub_in = 1;
   r.hub_out = 0;
-  if (MODE == kModeBF) r.hub_in_chunks = source_chunks(P);   // listed while the labels were cleared
+  if (is_bf(MODE)) r.hub_in_chunks = source_chunks(P);   // listed while the labels were cleared
   r.iter = 1;
   r.dq = P.delta_u;
   r.dinv = __float_as_uint(P.inv_delta);
@@ -1383,14 +1396,14 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
   // INIT: all labels unreached; delta bucket stamps / far flags cleared.
   for (size_t v = tid; v < P.n; v += stride) {
     ((typename L::T*)P.dist)[v] = L::kInf;
-    if (MODE == kModeBF) ((typename L::T*)P.dist_cur)[v] = L::kInf;
-    if (PRED && MODE == kModeBF && P.ties) P.ties[v] = ~0ull;
+    if (is_bf(MODE)) ((typename L::T*)P.dist_cur)[v] = L::kInf;
+    if (MODE == kModeBFProbe) P.ties[v] = ~0ull;
     if (MODE == kModeDelta) {
       P.bstamp[v] = 0xFFFFFFFFu;
       P.farflag[v] = 0u;
     }
   }
-  if (MODE == kModeBF && P.has_hubs) {
+  if (is_bf(MODE) && P.has_hubs) {
     const uint32_t nch = source_chunks(P);
     for (size_t j = tid; j < nch; j += stride)
       *reinterpret_cast<uint2*>(P.hubs + P.hub_cap + j) = make_uint2(P.source, (uint32_t)j);
@@ -1475,7 +1488,7 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
         const size_t v = P.inv ? (size_t)__ldg(P.inv + o) : o;   // internal id of output slot o
         typename L::T wv = ldcg(srcl + v);
         const uint32_t k = L::key(wv);
-        if (PRED && MODE == kModeBF && P.ties && R.aux != 1u) {
+        if (MODE == kModeBFProbe && R.aux != 1u) {
           const unsigned long long tie = ldcg(P.ties + v);   // (no tie has a smaller key than the label)
           if ((uint32_t)(tie >> 32) == k) wv = min(wv, (typename L::T)tie);
         }
@@ -1497,7 +1510,7 @@ __global__ void __launch_bounds__(kThreads, B2_SSSP_MINB) k_sssp(const __grid_co
     if (expands) flush_phase(s_phase + (threadIdx.x >> 5), t);
     next_phase(P, &s_rec, &s_next, &s_snap, s_phase, MODE == kModeDelta && expands, barrier,
                [&](const PhaseRec& r, MgrSnap& m, PhaseRec& nx) {
-                 if (MODE == kModeBF) manager_bf(P, r, m, nx);
+                 if (is_bf(MODE)) manager_bf(P, r, m, nx);
                  else manager_delta(P, r, m, nx);
                });
   }
@@ -1864,7 +1877,8 @@ b2_status run_sssp(b2_graph g, int mode, uint32_t source, void* d_dist, int32_t*
     e = grid > 0 ? launch<WT, PR, MD>(P, grid, st) : cudaErrorInvalidConfiguration; \
   } while (0)
   if (mode == kModeBF) {
-    if (isf) { if (pred) B2_LAUNCH(WF32, true, kModeBF); else B2_LAUNCH(WF32, false, kModeBF); }
+    if (P.ties) { if (isf) B2_LAUNCH(WF32, true, kModeBFProbe); else B2_LAUNCH(WU32, true, kModeBFProbe); }
+    else if (isf) { if (pred) B2_LAUNCH(WF32, true, kModeBF); else B2_LAUNCH(WF32, false, kModeBF); }
     else { if (pred) B2_LAUNCH(WU32, true, kModeBF); else B2_LAUNCH(WU32, false, kModeBF); }
   } else {
     if (isf) { if (pred) B2_LAUNCH(WF32, true, kModeDelta); else B2_LAUNCH(WF32, false, kModeDelta); }
