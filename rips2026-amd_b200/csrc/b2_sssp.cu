@@ -32,8 +32,8 @@
 // chunks of high-degree vertices are listed when those are pushed and run beside
 // the frontier of their round.  With a commit phase, and hub chunks in a phase of
 // their own, a round took three grid barriers: RMAT-17 with predecessors 0.58 ->
-// 0.36 ms, ER-4096 0.28 -> 0.19 ms. (Slower only past what L2 holds of two arrays: RMAT-24
-// with predecessors 25.1 -> 26.2 ms.)
+// 0.36 ms, ER-4096 0.28 -> 0.19 ms.  (Slower only past what L2 holds of two arrays:
+// RMAT-24 with predecessors 25.1 -> 26.2 ms.)
 //
 // Times in this file compare two builds on one graph and source; solves of a family
 // and size differ by up to 20 % between graphs and sources.
